@@ -355,8 +355,18 @@ static void upload_and_factor(plasma_context_t *plasma, const upload_t *up,
     }
     plasma_cuda_lansy_inf(cp, plasma->dquiet, PlasmaLower, A, d_anorm, symv_work);
     cudaEventRecord(plasma->ev[5], cp);
+    /* the walk scales panel rows by the diagonal before its columns are in */
+    float *diag = (float *)malloc((size_t)As.gm * sizeof(float));
+    if (diag == NULL) {
+        plasma_request_fail(sequence, request, PlasmaErrorOutOfMemory);
+        return;
+    }
+    #pragma omp parallel for schedule(static)
+    for (int i = 0; i < As.gm; i++)
+        diag[i] = i < n ? (float)up->pA[(size_t)i * up->lda + i] : 1.0f;
     plasma_pXpotrf_arrivals(plasma, PlasmaLower, As, sequence, request, call, mode, ng,
-                            gstart, plasma->ev_group);
+                            gstart, plasma->ev_group, diag);
+    free(diag);
     cudaStreamWaitEvent(S, plasma->ev[5], 0);
 }
 

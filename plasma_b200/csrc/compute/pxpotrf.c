@@ -42,13 +42,14 @@ typedef struct {
     char *panel[3];    /* rounded copies of panel k (buffer k % 3, or all) */
     char *wimg;        /* operand image of the diagonal tile for the
                           tensor-core panel solve (plasma_cuda_trsm_tc)    */
+    float *scale;      /* row scales of the split half-precision copies    */
 } walk_t;
 
 /* FP32 factors: every mode runs its update on the tensor cores when the
  * tiles allow it.  FP32 accuracy comes from a split of the panel: three
- * TF32 products of a two-part split, or with PLASMA_FP32_SPLIT=bf16x6
- * (256-wide tiles) six BF16 products of a three-part split, which moves
- * 6 instead of 8 operand bytes per element at the same tensor time. */
+ * half-precision products of a two-part split with row scales, or with
+ * PLASMA_FP32_SPLIT=bf16x6 (256-wide tiles) six BF16 products of a
+ * three-part split. */
 static int tc_mode(plasma_desc_t A, int mode)
 {
     static int split_env = -1;
@@ -58,11 +59,11 @@ static int tc_mode(plasma_desc_t A, int mode)
     }
     return mode == PlasmaFactorTF32 ? PLASMA_TC_TF32
          : mode == PlasmaFactorBF16 ? PLASMA_TC_BF16
-         : (A.mb == 256 && split_env) ? PLASMA_TC_BF16X6 : PLASMA_TC_TF32X3;
+         : (A.mb == 256 && split_env) ? PLASMA_TC_BF16X6 : PLASMA_TC_FP16X3;
 }
 
 /* the panel copies: three buffers, or one holding every panel; then the
- * operand image of the panel solve.  Panel k's copy is written by the
+ * operand image of the panel solve and the row scales.  Panel k's copy is written by the
  * solve of step k (or by plasma_cuda_panel_round right after it); with
  * three buffers the one it reuses was last read by the step k-3 update,
  * which the critical stream has waited for (N(k-2)) before step k. */
@@ -70,7 +71,7 @@ static size_t panel_scratch_bytes(plasma_desc_t A, int tc, int full)
 {
     const size_t one = (plasma_cuda_panel_bytes(tc, A, full) + 1023) & ~(size_t)1023;
     const size_t wimg = (plasma_cuda_trsm_tc_bytes(A.nb) + 1023) & ~(size_t)1023;
-    return (full ? 1 : 3) * one + wimg + 1024;
+    return (full ? 1 : 3) * one + wimg + 2 * (size_t)A.gm * sizeof(float) + 1024;
 }
 
 void plasma_pXpotrf_reserve(plasma_context_t *plasma, plasma_enum_t uplo, plasma_desc_t A,
@@ -89,7 +90,7 @@ static void update(walk_t *w, cudaStream_t s, int k, int nlo, int nhi)
 {
     if (w->mode) {
         if (plasma_cuda_update_tc(s, w->st, w->mode, w->A, k, nlo, nhi,
-                                  panel_buf(w, k), w->full, w->sms))
+                                  panel_buf(w, k), w->full, w->scale, w->sms))
             return;
     }
     plasma_cuda_update(s, w->st, w->uplo, w->A, k, nlo, nhi, w->sms);
@@ -98,7 +99,8 @@ static void update(walk_t *w, cudaStream_t s, int k, int nlo, int nhi)
 static void round_panel(walk_t *w, cudaStream_t s, int k)
 {
     if (w->mode)
-        plasma_cuda_panel_round(s, w->st, w->mode, w->A, k, panel_buf(w, k), w->full);
+        plasma_cuda_panel_round(s, w->st, w->mode, w->A, k, panel_buf(w, k), w->full,
+                                w->scale);
 }
 
 /* The panel solve of step k: on the tensor cores next to a tensor-core
@@ -109,7 +111,7 @@ static int trsm(walk_t *w, cudaStream_t s, int k)
 {
     if (w->mode && w->wimg != NULL) {
         const int r = plasma_cuda_trsm_tc(s, w->st, w->mode, w->A, k, k + 1, w->A.mt,
-                                          w->wimg, panel_buf(w, k), w->full);
+                                          w->wimg, panel_buf(w, k), w->full, w->scale);
         if (r)
             return r == 2;
     }
@@ -128,7 +130,7 @@ void plasma_pXpotrf_mode(plasma_context_t *plasma, plasma_enum_t uplo,
                          plasma_desc_t A, plasma_sequence_t *sequence,
                          plasma_request_t *request, int call, int mode)
 {
-    plasma_pXpotrf_arrivals(plasma, uplo, A, sequence, request, call, mode, 0, NULL, NULL);
+    plasma_pXpotrf_arrivals(plasma, uplo, A, sequence, request, call, mode, 0, NULL, NULL, NULL);
 }
 
 /* The arriving-columns DAG: one update stream per column group.  At step k
@@ -226,7 +228,8 @@ static void walk_groups(plasma_context_t *plasma, walk_t *w, int call, int ngrou
 void plasma_pXpotrf_arrivals(plasma_context_t *plasma, plasma_enum_t uplo,
                              plasma_desc_t A, plasma_sequence_t *sequence,
                              plasma_request_t *request, int call, int mode,
-                             int ngroups, const int *gstart, const cudaEvent_t *arrive)
+                             int ngroups, const int *gstart, const cudaEvent_t *arrive,
+                             const float *diag)
 {
     if (sequence->status != PlasmaSuccess)
         return;
@@ -255,6 +258,7 @@ void plasma_pXpotrf_arrivals(plasma_context_t *plasma, plasma_enum_t uplo,
     w.full = grouped;
     w.panel[0] = w.panel[1] = w.panel[2] = NULL;
     w.wimg = NULL;
+    w.scale = NULL;
     int tc = tc_mode(A, mode);
     if (plasma_cuda_update_tc_ok(A, uplo)) {
         char *buf = (char *)plasma_scratch(plasma, PLASMA_SLOT_MIXED,
@@ -267,6 +271,20 @@ void plasma_pXpotrf_arrivals(plasma_context_t *plasma, plasma_enum_t uplo,
             w.panel[1] = buf + one;
             w.panel[2] = buf + 2 * one;
             w.wimg = buf + (w.full ? 1 : 3) * one;
+            const size_t wb = (plasma_cuda_trsm_tc_bytes(A.nb) + 1023) & ~(size_t)1023;
+            w.scale = (float *)(w.wimg + wb);
+            if (tc == PLASMA_TC_FP16X3) {
+                /* the diagonal of a matrix still arriving comes from the
+                 * host, into the reciprocals' place until they are formed
+                 * (every thread reads its own entry first) */
+                float *d = NULL;
+                if (grouped) {
+                    d = w.scale + A.gm;
+                    cudaMemcpyAsync(d, diag, (size_t)A.gm * sizeof(float),
+                                    cudaMemcpyHostToDevice, S);
+                }
+                plasma_cuda_row_scale(S, A, d, w.scale);
+            }
         }
     }
     /* FP32 panels: TF32 products next to a TF32/BF16 update, else the

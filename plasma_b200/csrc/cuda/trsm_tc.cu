@@ -30,8 +30,8 @@
 //             operand of the update of every block to its right (one MMA
 //             chain of N up to 192 into their adjacent accumulators);
 //   warps 6-9: the same rows (tensor lanes 32 (w mod 4) ..) -- read X_j,
-//             stage it, and its rounded copies when the trailing update takes
-//             TF32 operands, in shared memory for TMA stores to A(m,k) and to
+//             stage it, and its copies in the operand format of the trailing
+//             update (scaled half-precision hi and lo parts, or TF32), in shared memory for TMA stores to A(m,k) and to
 //             the panel buffer the update reads; the stores stay off the
 //             chain of dependent steps above (the X product of block j+1
 //             only waits until these warps have read X_j).
@@ -65,6 +65,7 @@ struct TsArgs {
     int panel;          // write the rounded copies of the solved tiles
     int poff;           // panel tile of row tile m: poff + m (hi), + pstride (lo)
     int pstride;
+    const float *scale; // row scales of half-precision copies, or null: TF32
 };
 
 __device__ __forceinline__ uint32_t tf32_round(float x)
@@ -316,6 +317,8 @@ k_trsm_tc(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUte
                                 ((size_t)nb * nb * 4));
         float *stg = (float *)(sm + TS_STG + q * TS_STG_WARP);
         bool staged = false;    // a store group of this warp may still read stg
+        const int row = r0 + 32 * q + lane;
+        const float sc = g.scale != nullptr && row < rows ? g.scale[m * nb + row] : 1.f;
         for (int j = 0; j < nblk; j++) {
             const bool okx = __all_sync(0xffffffffu, mbar_wait(&x_bar, j & 1, &abort_s));
             if (!okx) break;
@@ -334,11 +337,12 @@ k_trsm_tc(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUte
 #pragma unroll
                 for (int i = 0; i < 32; i++) {
                     const float v = x[32 * h + i];
-                    const uint32_t hi = tf32_round(v);
                     stg[i * 32 + lane] = v;
-                    stg[1024 + i * 32 + lane] = __uint_as_float(hi);
-                    stg[2048 + i * 32 + lane] =
-                        __uint_as_float(tf32_round(v - __uint_as_float(hi)));
+                    if (g.scale != nullptr)
+                        split_half(v * sc, ((__half *)(stg + 1024))[i * 32 + lane],
+                                   ((__half *)(stg + 2048))[i * 32 + lane]);
+                    else
+                        stg[1024 + i * 32 + lane] = __uint_as_float(tf32_round(v));
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
@@ -475,16 +479,19 @@ bool encode_w_map(CUtensorMap *map, void *base, int nb, int parts)
     return r == CUDA_SUCCESS;
 }
 
-// 3-D map over column-major nb x nb tiles {rows, columns, tile}, box 32 x 32
-bool encode_tiles_32(CUtensorMap *map, void *base, int nb, long long ntiles)
+// 3-D map over column-major nb x nb tiles {rows, columns, tile} of FP32 or
+// (half) FP16 elements, box 32 x 32
+bool encode_tiles_32(CUtensorMap *map, void *base, int nb, long long ntiles, bool half)
 {
     PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
     if (encode == nullptr || ntiles <= 0) return false;
     cuuint64_t dims[3] = {(cuuint64_t)nb, (cuuint64_t)nb, (cuuint64_t)ntiles};
-    cuuint64_t strides[2] = {(cuuint64_t)nb * 4, (cuuint64_t)nb * nb * 4};
+    const cuuint64_t esz = half ? 2 : 4;
+    cuuint64_t strides[2] = {nb * esz, (cuuint64_t)nb * nb * esz};
     cuuint32_t box[3] = {32, 32, 1};
     cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, estr,
+    CUresult r = encode(map, half ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                  : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS;
@@ -505,11 +512,11 @@ extern "C" size_t plasma_cuda_trsm_tc_bytes(int nb)
 // scratch of plasma_cuda_trsm_tc_bytes(nb).  `panel` (may be null): the
 // rounded operand copies of the trailing update for `mode` in the layout
 // `full` (plasma_cuda_panel_round's); written here when the update takes
-// TF32 operands.  Returns 0 when not eligible (nothing launched), 1 when the
+// TF32 or split half-precision operands (the latter need the row scales).  Returns 0 when not eligible (nothing launched), 1 when the
 // solve ran, 2 when it also wrote the panel copies.
 extern "C" int plasma_cuda_trsm_tc(cudaStream_t s, plasma_devstat_t *st, int mode,
                                    plasma_desc_t A, int k, int mlo, int mhi, void *wimg,
-                                   void *panel, int full)
+                                   void *panel, int full, const float *scale)
 {
     if (!plasma_cuda_update_tc_ok(A, PlasmaLower) || wimg == nullptr ||
         ((uintptr_t)wimg & 1023) != 0 || plasma_tile_mview(A, k) != A.nb)
@@ -526,15 +533,17 @@ extern "C" int plasma_cuda_trsm_tc(cudaStream_t s, plasma_devstat_t *st, int mod
     const int split = mode == PLASMA_TC_TF32 || mode == PLASMA_TC_BF16 ? 1 : 3;
     const int parts = split == 3 ? 2 : 1;
     int poff = 0, pstride = 0;
+    const bool half = mode == PLASMA_TC_FP16X3;
     const bool write_panel = panel != nullptr &&
-                             (mode == PLASMA_TC_TF32X3 || mode == PLASMA_TC_TF32);
+                             ((half && scale != nullptr) || mode == PLASMA_TC_TF32);
     if (write_panel) plasma_cuda_panel_layout(A, k, full, &poff, &pstride);
     const long long atiles = (long long)(plasma_desc_storage_bytes(A) / ((size_t)nb * nb * 4));
     CUtensorMap wmap, amap, pmap;
     if (!encode_w_map(&wmap, wimg, nb, parts) ||
-        !encode_tiles_32(&amap, A.matrix, nb, atiles) ||
+        !encode_tiles_32(&amap, A.matrix, nb, atiles, false) ||
         !encode_tiles_32(&pmap, write_panel ? panel : A.matrix, nb,
-                         write_panel ? (long long)parts * pstride : atiles))
+                         write_panel ? (long long)parts * pstride : atiles,
+                         write_panel && half))
         return 0;
 
     TsArgs g;
@@ -545,6 +554,7 @@ extern "C" int plasma_cuda_trsm_tc(cudaStream_t s, plasma_devstat_t *st, int mod
     g.panel = write_panel ? 1 : 0;
     g.poff = poff;
     g.pstride = pstride;
+    g.scale = write_panel && half ? scale : nullptr;
 
     static unsigned long long attr = 0;
     if (plasma_first_on_device(&attr)) {

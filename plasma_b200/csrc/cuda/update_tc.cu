@@ -9,16 +9,25 @@
 // FP32 in tensor memory:
 //   TF32   : one kind::tf32 MMA per k-step on the TF32-rounded panel;
 //   BF16   : one kind::f16 MMA per k-step on the BF16-rounded panel;
-//   TF32X3 : the panel split as a = hi + lo (hi = tf32(a), lo = tf32(a - hi))
-//            and a*b formed as lo*hi + hi*lo + hi*hi, three kind::tf32 MMAs,
-//            which keeps about 22 bits of every product (the FP32 factor);
+//   FP16X3 : the panel split as a*s = hi + lo (hi = half(a*s),
+//            lo = half(a*s - hi), s a power of two of the row) and a*b formed as
+//            lo*hi + hi*lo + hi*hi, three kind::f16 MMAs, unscaled on the way
+//            out (the FP32 factor).  The split and the dropped lo*lo term are
+//            those of Markidis et al. (2018) / Ootomo & Yokota (2022).  Half
+//            precision has TF32's 11 significant bits at half its operand
+//            bytes and twice its MMA rate; what it lacks is exponent range,
+//            which the row scale supplies: |L(i,k)| <= sqrt(A(i,i)), so with
+//            s_i = 2^14 / 2^ceil(log2 sqrt(A(i,i))) nothing overflows, products
+//            keep 22 bits down to 2^-16 of the row's bound and an absolute
+//            2^-39 of it below that, against the 2^-24 rounding of the sums.
+//            (n = 32768: all trailing updates of a factor 77 ms with three
+//            TF32 products of the same split.)
 //   BF16X6 : the panel split in three BF16 parts, a = h + m + l (h = bf16(a),
 //            m = bf16(a - h), l = bf16(a - h - m)), and a*b formed from the six
 //            products whose order is at most 2^-16 (l*h, h*l, m*m, m*h, h*m,
-//            h*h), six kind::f16 MMAs: about 23 bits of every product, the
-//            same tensor time as TF32X3 (a BF16 MMA covers twice the K) and
-//            6 instead of 8 operand bytes per element (the FP32 factor on
-//            256-wide tiles, CTA-pair kernel only).
+//            h*h), six kind::f16 MMAs: about 23 bits of every product at
+//            twice the tensor time of FP16X3, with FP32's whole exponent range
+//            (256-wide tiles, CTA-pair kernel only).
 //
 // One CTA owns a run of `ipc` consecutive work items (a 128 x nb block of one
 // output tile each; items of one tile column are adjacent, so they share the
@@ -26,7 +35,7 @@
 //   warp 0     : TMA producer -- 4-D tensor maps over the column-major panel
 //                tiles (128-byte swizzle; 32-byte swizzle atoms for TF32, the
 //                only MN-major TF32 layout), a ring of 48 KB stages (4 for
-//                TF32X3, 3 otherwise);
+//                FP16X3, 3 otherwise);
 //   warp 1     : MMA issuer -- one thread issues tcgen05.mma (M = 128, N = nb,
 //                MN-major A and B), tcgen05.commit frees a stage and, after
 //                the last k-step of an item, publishes its accumulator;
@@ -47,6 +56,7 @@
 #include "tc.cuh"
 
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <stdlib.h>
 
 namespace {
@@ -59,32 +69,32 @@ constexpr int TC_STAGE_BYTES = 48 * 1024;
 constexpr int TC_EPI_BUF_BYTES = 32 * 32 * 4;
 
 enum { MODE_TF32 = PLASMA_TC_TF32, MODE_BF16 = PLASMA_TC_BF16,
-       MODE_TF32X3 = PLASMA_TC_TF32X3, MODE_BF16X6 = PLASMA_TC_BF16X6 };
+       MODE_FP16X3 = PLASMA_TC_FP16X3, MODE_BF16X6 = PLASMA_TC_BF16X6 };
 
 template <int MODE>
 struct Geo {
-    static constexpr bool HALF16 = MODE == MODE_BF16 || MODE == MODE_BF16X6;
+    static constexpr bool HALF16 = MODE != MODE_TF32;
     static constexpr int ESZ = HALF16 ? 2 : 4;
     static constexpr int MNBOX = 128 / ESZ;           // elements per 128-byte row
-    static constexpr int BK = MODE == MODE_BF16 ? 64
-                            : (MODE == MODE_TF32 || MODE == MODE_BF16X6) ? 32 : 16;
+    static constexpr int BK = MODE == MODE_BF16 ? 64 : 32;
     static constexpr int KI = HALF16 ? 16 : 8;        // K per instruction
-    static constexpr int PARTS = MODE == MODE_TF32X3 ? 2 : MODE == MODE_BF16X6 ? 3 : 1;
+    static constexpr int PARTS = MODE == MODE_FP16X3 ? 2 : MODE == MODE_BF16X6 ? 3 : 1;
     static constexpr uint32_t LAYOUT = HALF16 ? 2u : 1u;
     static constexpr uint32_t SBO = HALF16 ? 1024u : 512u;
     static constexpr int CHUNK = BK * 128;            // one MN chunk of a stage
     static constexpr int A_BYTES = (TC_M / MNBOX) * CHUNK;
-    // TF32X3 moves twice the operand bytes per product: a deeper ring (more
-    // bytes in flight against the L2 latency), one epilogue buffer per warp
-    static constexpr int STAGES = MODE == MODE_TF32X3 ? 4 : 3;
-    static constexpr int EPI_BUFS = MODE == MODE_TF32X3 ? 1 : 2;
+    // the split modes: a deeper ring (more bytes in flight against the L2
+    // latency), one epilogue buffer per warp
+    static constexpr int STAGES = MODE == MODE_FP16X3 ? 4 : 3;
+    static constexpr int EPI_BUFS = MODE == MODE_FP16X3 ? 1 : 2;
     static constexpr int SMEM = STAGES * TC_STAGE_BYTES +
                                 TC_EPI_WARPS * EPI_BUFS * TC_EPI_BUF_BYTES + 1024;
 };
 
 __device__ __forceinline__ uint32_t instr_desc(int mode, int n)
 {
-    uint32_t fmt = mode == MODE_BF16 ? 1u : 2u;   // BF16 : TF32
+    // A and B format: F16, BF16 (kind::f16) or TF32 (kind::tf32)
+    uint32_t fmt = mode == MODE_FP16X3 ? 0u : mode == MODE_BF16 ? 1u : 2u;
     return (1u << 4)                 // D format F32
          | (fmt << 7) | (fmt << 10)  // A, B format
          | (1u << 15) | (1u << 16)   // A, B MN-major
@@ -97,7 +107,7 @@ __device__ __forceinline__ void mma(uint32_t tmem, uint64_t a, uint64_t b,
                                     uint32_t idesc, uint32_t acc)
 {
     const uint32_t z = 0;      // no output lane disabled
-    if (MODE != MODE_BF16)
+    if (!Geo<MODE>::HALF16)
         asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
             "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
@@ -122,7 +132,24 @@ struct TcArgs {
     int mt;             // tiles per part in the operand map (part p at +p*mt)
     long long nitems;
     int ipc;            // items per CTA
+    const float *unscale;   // FP16X3: 1/s of every matrix row
 };
+
+// The accumulator of rows i, columns j holds s_i s_j times the product: the
+// 32 columns from `uj` (16-byte aligned) of one row, negated and unscaled.
+// The two factors are applied one after the other, so that neither their
+// product nor a partial one leaves the FP32 range when the result is in it.
+__device__ __forceinline__ void unscale32(float (&v)[32], float ui, const float *uj)
+{
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const float4 u = __ldg((const float4 *)uj + q);
+        v[4 * q] = v[4 * q] * ui * u.x;
+        v[4 * q + 1] = v[4 * q + 1] * ui * u.y;
+        v[4 * q + 2] = v[4 * q + 2] * ui * u.z;
+        v[4 * q + 3] = v[4 * q + 3] * ui * u.w;
+    }
+}
 
 // work item -> (m, n, si); items run over si fastest, then m, then n
 __device__ __forceinline__ void tc_item(const TcArgs &g, long long w, int &m, int &n,
@@ -245,7 +272,7 @@ k_update_tc(const __grid_constant__ CUtensorMap opmap,
                                             G::LAYOUT);
                     uint64_t db = smem_desc(sb_hi + kk * G::KI * 128, G::CHUNK, G::SBO,
                                             G::LAYOUT);
-                    if (MODE == MODE_TF32X3) {
+                    if (MODE == MODE_FP16X3) {
                         unsigned char *sa_lo = sp + G::A_BYTES;
                         unsigned char *sb_lo = sb_hi + b_bytes;
                         uint64_t dal = smem_desc(sa_lo + kk * G::KI * 128, G::CHUNK, G::SBO,
@@ -286,9 +313,11 @@ k_update_tc(const __grid_constant__ CUtensorMap opmap,
             const int row = r0 + lane;
             const bool diag = m == n;
             const int c0 = half * (nb / 2);
+            const float ui = MODE == MODE_FP16X3 ? __ldg(g.unscale + m * nb + row) : 1.f;
             for (int cc = c0; cc < c0 + nb / 2; cc += 32, nchunk++) {
                 float v[32];
                 tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(a * nb + cc), v);
+                if (MODE == MODE_FP16X3) unscale32(v, ui, g.unscale + n * nb + cc);
                 float *buf = stage_epi + (nchunk % TC_EPI_BUFS) * (TC_EPI_BUF_BYTES / 4);
                 // the reduction that last read this buffer must be done with it
                 if (nchunk >= TC_EPI_BUFS && lane == 0) bulk_wait_read<TC_EPI_BUFS - 1>();
@@ -337,7 +366,7 @@ k_update_tc(const __grid_constant__ CUtensorMap opmap,
 // whole 256 x 256 output tile per item.  The MMA runs with cta_group::2,
 // M = 256 and N = 256: each CTA stages its own 128 rows of A(m,k) and its
 // own 128 rows of A(n,k) (half of the B operand), so a CTA moves 32 KB of
-// operands per k-step instead of 48 KB (TF32X3) -- a third less L2 traffic
+// operands per k-step instead of 48 KB (FP16X3) -- a third less L2 traffic
 // per product, and a 6-deep ring in the same shared memory.  Tensor memory
 // of each CTA holds its 128 output rows (two accumulators of 256 columns).
 //   rank 0 (leader) : producer, MMA issuer, epilogue of rows 0..127;
@@ -355,8 +384,8 @@ struct PairGeo {
     using G = Geo<MODE>;
     // per part: 128 rows of A(m,k) and 128 rows of A(n,k), BK columns each
     static constexpr int STAGE = G::PARTS * 2 * G::A_BYTES;   // 32 KB, BF16X6 48 KB
-    static constexpr int EPI_BUFS = MODE == MODE_TF32X3 || MODE == MODE_BF16X6 ? 1 : 2;
-    static constexpr int STAGES = MODE == MODE_TF32X3 ? 6 : MODE == MODE_BF16X6 ? 4 : 5;
+    static constexpr int EPI_BUFS = MODE == MODE_FP16X3 || MODE == MODE_BF16X6 ? 1 : 2;
+    static constexpr int STAGES = MODE == MODE_FP16X3 ? 6 : MODE == MODE_BF16X6 ? 4 : 5;
     static constexpr int SMEM = STAGES * STAGE +
                                 TC_EPI_WARPS * EPI_BUFS * TC_EPI_BUF_BYTES + 1024;
     static_assert(SMEM <= 227 * 1024, "shared memory");
@@ -459,7 +488,7 @@ __device__ __forceinline__ void mma_commit_pair(uint64_t *bar)
 
 __device__ __forceinline__ uint32_t instr_desc_pair(int mode)
 {
-    uint32_t fmt = mode == MODE_BF16 || mode == MODE_BF16X6 ? 1u : 2u;
+    uint32_t fmt = mode == MODE_FP16X3 ? 0u : mode == MODE_TF32 ? 2u : 1u;
     return (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 15) | (1u << 16) |
            ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
 }
@@ -590,7 +619,7 @@ k_update_pair(const __grid_constant__ CUtensorMap opmap,
                                             G::LAYOUT);
                     uint64_t db = smem_desc(sb_hi + kk * G::KI * 128, G::CHUNK, G::SBO,
                                             G::LAYOUT);
-                    if (MODE == MODE_TF32X3) {
+                    if (MODE == MODE_FP16X3) {
                         uint64_t dal = smem_desc(sa_hi + HALF + kk * G::KI * 128, G::CHUNK,
                                                  G::SBO, G::LAYOUT);
                         uint64_t dbl = smem_desc(sb_hi + HALF + kk * G::KI * 128, G::CHUNK,
@@ -644,9 +673,11 @@ k_update_pair(const __grid_constant__ CUtensorMap opmap,
             const int row = r0 + lane;
             const bool diag = m == n;
             const int c0 = half * (NB / 2);
+            const float ui = MODE == MODE_FP16X3 ? __ldg(g.unscale + m * NB + row) : 1.f;
             for (int cc = c0; cc < c0 + NB / 2; cc += 32, nchunk++) {
                 float v[32];
                 tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(a * NB + cc), v);
+                if (MODE == MODE_FP16X3) unscale32(v, ui, g.unscale + n * NB + cc);
                 float *buf = stage_epi + (nchunk % EPI_BUFS) * (TC_EPI_BUF_BYTES / 4);
                 if (nchunk >= EPI_BUFS && lane == 0) bulk_wait_read<EPI_BUFS - 1>();
                 __syncwarp();
@@ -800,7 +831,7 @@ void panel_layout(const plasma_desc_t &A, int k, int full, int *poff, int *pstri
 
 int mode_parts(int mode)
 {
-    return mode == PLASMA_TC_TF32X3 ? 2 : mode == PLASMA_TC_BF16X6 ? 3 : 1;
+    return mode == PLASMA_TC_FP16X3 ? 2 : mode == PLASMA_TC_BF16X6 ? 3 : 1;
 }
 }  // namespace
 
@@ -824,10 +855,10 @@ extern "C" int plasma_cuda_update_tc_ok(plasma_desc_t A, plasma_enum_t uplo)
 // (full = 0) or all panels of the factor (full = 1).
 extern "C" size_t plasma_cuda_panel_bytes(int mode, plasma_desc_t A, int full)
 {
-    if (mode < PLASMA_TC_TF32 || mode > PLASMA_TC_BF16X6) return 0;
+    if (mode < PLASMA_TC_TF32 || mode > PLASMA_TC_FP16X3) return 0;
     int poff, pstride;
     panel_layout(A, 0, full, &poff, &pstride);
-    const size_t esz = mode == PLASMA_TC_BF16 || mode == PLASMA_TC_BF16X6 ? 2 : 4;
+    const size_t esz = mode == PLASMA_TC_TF32 ? 4 : 2;
     return (size_t)mode_parts(mode) * pstride * A.mb * A.mb * esz;
 }
 
@@ -836,7 +867,8 @@ extern "C" size_t plasma_cuda_panel_bytes(int mode, plasma_desc_t A, int full)
 // aligned.  Returns 0 (nothing launched) when the update is not eligible.
 extern "C" int plasma_cuda_update_tc(cudaStream_t s, plasma_devstat_t *st,
                                      int mode, plasma_desc_t A, int k, int nlo,
-                                     int nhi, const void *panel, int full, int num_sms)
+                                     int nhi, const void *panel, int full, const float *scale,
+                                     int num_sms)
 {
     if (nhi <= nlo) return 1;
     const int nb = A.mb;
@@ -845,7 +877,8 @@ extern "C" int plasma_cuda_update_tc(cudaStream_t s, plasma_devstat_t *st,
     const long long nitems = tiles * (nb / TC_M);
     if (nitems <= 0) return 1;
     if (panel == nullptr || ((uintptr_t)panel & 1023) != 0 ||
-        ((uintptr_t)A.matrix & 15) != 0)
+        ((uintptr_t)A.matrix & 15) != 0 ||
+        (mode == PLASMA_TC_FP16X3 && (scale == nullptr || ((uintptr_t)scale & 15) != 0)))
         return 0;
 
     int poff, pstride;
@@ -858,10 +891,9 @@ extern "C" int plasma_cuda_update_tc(cudaStream_t s, plasma_devstat_t *st,
         enc = encode_tile_map(&map, (void *)panel, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, nb,
                               ntiles, Geo<MODE_TF32>::BK, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
         break;
-    case PLASMA_TC_TF32X3:
-        enc = encode_tile_map(&map, (void *)panel, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, nb,
-                              ntiles, Geo<MODE_TF32X3>::BK,
-                              CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
+    case PLASMA_TC_FP16X3:
+        enc = encode_tile_map(&map, (void *)panel, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, nb,
+                              ntiles, Geo<MODE_FP16X3>::BK, CU_TENSOR_MAP_SWIZZLE_128B);
         break;
     case PLASMA_TC_BF16:
         enc = encode_tile_map(&map, (void *)panel, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, nb,
@@ -885,6 +917,7 @@ extern "C" int plasma_cuda_update_tc(cudaStream_t s, plasma_devstat_t *st,
     g.nhi = nhi;
     g.poff = poff;
     g.mt = pstride;
+    g.unscale = mode == PLASMA_TC_FP16X3 ? scale + A.gm : nullptr;
     // PLASMA_UPDATE_MAX_ITEMS caps the items per CTA (default 8): shorter
     // CTAs hand SMs back to the panel stream sooner.  PLASMA_UPDATE_PAIR
     // selects the CTA-pair kernel for 256-wide tiles (default on; 0 = off).
@@ -923,14 +956,14 @@ extern "C" int plasma_cuda_update_tc(cudaStream_t s, plasma_devstat_t *st,
     if (use_pair) {
         switch (mode) {
         case PLASMA_TC_TF32: launch_pair<MODE_TF32>(s, map, cmap, g, grid, st); break;
-        case PLASMA_TC_TF32X3: launch_pair<MODE_TF32X3>(s, map, cmap, g, grid, st); break;
+        case PLASMA_TC_FP16X3: launch_pair<MODE_FP16X3>(s, map, cmap, g, grid, st); break;
         case PLASMA_TC_BF16X6: launch_pair<MODE_BF16X6>(s, map, cmap, g, grid, st); break;
         default: launch_pair<MODE_BF16>(s, map, cmap, g, grid, st); break;
         }
     } else {
         switch (mode) {
         case PLASMA_TC_TF32: launch_update<MODE_TF32>(s, map, cmap, g, grid, st); break;
-        case PLASMA_TC_TF32X3: launch_update<MODE_TF32X3>(s, map, cmap, g, grid, st); break;
+        case PLASMA_TC_FP16X3: launch_update<MODE_FP16X3>(s, map, cmap, g, grid, st); break;
         default: launch_update<MODE_BF16>(s, map, cmap, g, grid, st); break;
         }
     }
@@ -941,12 +974,12 @@ extern "C" int plasma_cuda_update_tc(cudaStream_t s, plasma_devstat_t *st,
 // Operand copy of panel k: panel tile m (m = k+1 .. mt-1) <- A(m,k) rounded
 // to the product precision, same column-major layout.  TF32: round to
 // nearest, ties away, kept in an FP32 container; BF16: round to nearest
-// even; TF32X3: hi = tf32(a) at tile m and lo = tf32(a - hi) at tile m + mt
-// (a - hi is exact in FP32).
+// even; FP16X3: hi = half(a*s) at tile m and lo = half(a*s - hi) at tile
+// m + mt (a*s and a*s - hi are exact in FP32).
 namespace {
 template <int MODE>
 __global__ void k_panel_round(plasma_desc_t A, int k, void *panel, int poff, int pstride,
-                              const plasma_devstat_t *st)
+                              const float *scale, const plasma_devstat_t *st)
 {
     if (plasma_failed(st)) return;
     const int m = k + 1 + blockIdx.y;
@@ -962,6 +995,13 @@ __global__ void k_panel_round(plasma_desc_t A, int k, void *panel, int poff, int
             __nv_bfloat16 *o = (__nv_bfloat16 *)panel + t * tot + 4 * e;
 #pragma unroll
             for (int i = 0; i < 4; i++) o[i] = __float2bfloat16_rn(xs[i]);
+        } else if (MODE == MODE_FP16X3) {
+            __half *o = (__half *)panel + t * tot + 4 * e;
+            const size_t plane = (size_t)pstride * tot;
+            const float4 s4 = *(const float4 *)(scale + m * nb + (int)(4 * e % nb));
+            const float ss[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) split_half(xs[i] * ss[i], o[i], o[plane + i]);
         } else if (MODE == MODE_BF16X6) {
             // h, m, l planes at tiles m, m + mt, m + 2 mt; both differences
             // are exact in FP32 (each drops the leading 8 significant bits)
@@ -978,29 +1018,52 @@ __global__ void k_panel_round(plasma_desc_t A, int k, void *panel, int poff, int
                 o[2 * plane + i] = __float2bfloat16_rn(r2);
             }
         } else {
-            uint32_t hi[4], lo[4];
+            uint32_t r[4];
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi[i]) : "f"(xs[i]));
-                if (MODE == MODE_TF32X3) {
-                    float r = xs[i] - __uint_as_float(hi[i]);
-                    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo[i]) : "f"(r));
-                }
-            }
-            uint4 *o = (uint4 *)panel + (t * tot) / 4 + e;
-            *o = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            if (MODE == MODE_TF32X3) {
-                uint4 *ol = (uint4 *)panel + ((t + pstride) * tot) / 4 + e;
-                *ol = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-            }
+            for (int i = 0; i < 4; i++)
+                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r[i]) : "f"(xs[i]));
+            *((uint4 *)panel + (t * tot) / 4 + e) = make_uint4(r[0], r[1], r[2], r[3]);
         }
     }
 }
+
+// Row scales of the FP16X3 split for a factorization of A (lower): scale[i]
+// = 2^(14 - e), 2^e the power of two at or above sqrt(A(i,i)), and
+// scale[rows + i] its reciprocal; both exact.  A diagonal entry that is not
+// positive and finite takes 1: such a row meets the failing pivot (info)
+// before anything reads it further.  diag: the diagonal as a vector, for a
+// matrix whose columns are still arriving.
+__global__ void k_row_scale(plasma_desc_t A, const float *diag, float *scale, int rows)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= rows) return;
+    float d;
+    if (diag != nullptr) {
+        d = diag[i];
+    } else {
+        const int t = i / A.mb, r = i - t * A.mb;
+        d = ((const float *)plasma_tile_addr(A, t, t))[(size_t)r * plasma_tile_mmain(A, t) + r];
+    }
+    int e = 14;
+    if (d > 0.f && d <= 3.402823466e38f) {
+        frexpf(d, &e);                   // d < 2^e, so sqrt(d) < 2^ceil(e/2)
+        e = (e + 1) >> 1;
+    }
+    scale[i] = ldexpf(1.f, 14 - e);
+    scale[rows + i] = ldexpf(1.f, e - 14);
+}
 }  // namespace
+
+extern "C" void plasma_cuda_row_scale(cudaStream_t s, plasma_desc_t A, const float *diag,
+                                      float *scale)
+{
+    PLASMA_COUNT_LAUNCH();
+    k_row_scale<<<ceil_div(A.gm, 256), 256, 0, s>>>(A, diag, scale, A.gm);
+}
 
 extern "C" void plasma_cuda_panel_round(cudaStream_t s, plasma_devstat_t *st,
                                         int mode, plasma_desc_t A, int k,
-                                        void *panel, int full)
+                                        void *panel, int full, const float *scale)
 {
     int rows = A.mt - k - 1;
     if (rows <= 0) return;
@@ -1010,16 +1073,16 @@ extern "C" void plasma_cuda_panel_round(cudaStream_t s, plasma_devstat_t *st,
     dim3 grid(16, rows);
     switch (mode) {
     case PLASMA_TC_BF16:
-        k_panel_round<MODE_BF16><<<grid, 256, 0, s>>>(A, k, panel, poff, pstride, st);
+        k_panel_round<MODE_BF16><<<grid, 256, 0, s>>>(A, k, panel, poff, pstride, scale, st);
         break;
-    case PLASMA_TC_TF32X3:
-        k_panel_round<MODE_TF32X3><<<grid, 256, 0, s>>>(A, k, panel, poff, pstride, st);
+    case PLASMA_TC_FP16X3:
+        k_panel_round<MODE_FP16X3><<<grid, 256, 0, s>>>(A, k, panel, poff, pstride, scale, st);
         break;
     case PLASMA_TC_BF16X6:
-        k_panel_round<MODE_BF16X6><<<grid, 256, 0, s>>>(A, k, panel, poff, pstride, st);
+        k_panel_round<MODE_BF16X6><<<grid, 256, 0, s>>>(A, k, panel, poff, pstride, scale, st);
         break;
     default:
-        k_panel_round<MODE_TF32><<<grid, 256, 0, s>>>(A, k, panel, poff, pstride, st);
+        k_panel_round<MODE_TF32><<<grid, 256, 0, s>>>(A, k, panel, poff, pstride, scale, st);
         break;
     }
 }

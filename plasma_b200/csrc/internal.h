@@ -212,10 +212,11 @@ void plasma_cuda_potrf_tile(cudaStream_t s, plasma_devstat_t *st, int call,
  * (upper: A(k,m) <- U_kk^{-T} A(k,m)), given W = inv(L_kk). mlo..mhi-1 is the
  * tile range processed. */
 /* Panel solve of step k on the tensor cores (FP32, lower, tiles of 128 or
- * 256); writes the update's rounded panel copies when the mode's operands
- * are TF32.  0: not eligible, 1: solved, 2: solved and copies written. */
+ * 256); writes the update's panel copies when the mode's operands are TF32
+ * or split half precision.  0: not eligible, 1: solved, 2: solved and copies written. */
 int plasma_cuda_trsm_tc(cudaStream_t s, plasma_devstat_t *st, int mode, plasma_desc_t A,
-                        int k, int mlo, int mhi, void *wimg, void *panel, int full);
+                        int k, int mlo, int mhi, void *wimg, void *panel, int full,
+                        const float *scale);
 size_t plasma_cuda_trsm_tc_bytes(int nb);
 /* Block inverses for the one-launch sweeps with an LU factor (unit-lower L
  * forward, U backward); 0 when the sweep block is not 64 rows. */
@@ -280,9 +281,10 @@ void plasma_cuda_lacpy(cudaStream_t s, plasma_devstat_t *st,
  * Product precisions: */
 #define PLASMA_TC_TF32   1   /* one TF32 product                         */
 #define PLASMA_TC_BF16   2   /* one BF16 product                         */
-#define PLASMA_TC_TF32X3 3   /* lo*hi + hi*lo + hi*hi TF32 split (FP32)   */
-#define PLASMA_TC_BF16X6 4   /* six products of a three-part BF16 split
+#define PLASMA_TC_BF16X6 3   /* six products of a three-part BF16 split
                                 (FP32; 256-wide tiles)                     */
+#define PLASMA_TC_FP16X3 4   /* lo*hi + hi*lo + hi*hi of a half-precision
+                                split with row scales (FP32)               */
 int plasma_cuda_update_tc_ok(plasma_desc_t A, plasma_enum_t uplo);
 /* Operand copies of the panels: full = 0 holds one panel (the caller
  * alternates two buffers), full = 1 every panel of the factor, so that an
@@ -290,12 +292,16 @@ int plasma_cuda_update_tc_ok(plasma_desc_t A, plasma_enum_t uplo);
 size_t plasma_cuda_panel_bytes(int tc_mode, plasma_desc_t A, int full);
 int plasma_cuda_update_tc(cudaStream_t s, plasma_devstat_t *st, int tc_mode,
                           plasma_desc_t A, int k, int nlo, int nhi,
-                          const void *panel, int full, int num_sms);
+                          const void *panel, int full, const float *scale, int num_sms);
+/* Row scales of the FP16X3 split: 2 A.gm floats (scales, then reciprocals),
+ * from A's diagonal, or from `diag` (A.gm floats) when given. */
+void plasma_cuda_row_scale(cudaStream_t s, plasma_desc_t A, const float *diag, float *scale);
 /* Copy of panel k in the operand format of tc_mode, in the layout `full`
  * (row tile m of the panel at tile m, or at k*mt - k(k-1)/2 + m - k; the
  * further parts of a split at one plane further each). */
 void plasma_cuda_panel_round(cudaStream_t s, plasma_devstat_t *st, int tc_mode,
-                             plasma_desc_t A, int k, void *panel, int full);
+                             plasma_desc_t A, int k, void *panel, int full,
+                             const float *scale);
 /* FP32 diagonal tile held in shared memory (order a multiple of 32, at most
  * 256); 0 when not applicable. */
 int plasma_cuda_potrf_diag_smem(cudaStream_t s, plasma_devstat_t *st, int call,
@@ -393,7 +399,9 @@ void plasma_pXpotrf_mode(plasma_context_t *plasma, plasma_enum_t uplo,
 /* The same factorization of a matrix whose tile columns are still arriving:
  * group g = tile columns [gstart[g], gstart[g+1]) is in place once event
  * arrive[g] has completed (gstart[0] = 0, gstart[ngroups] = A.nt,
- * 1 <= ngroups <= PLASMA_MAX_GROUPS). */
+ * 1 <= ngroups <= PLASMA_MAX_GROUPS).  diag: A's diagonal on the host
+ * (A.gm floats, 1 on the padding), read before the call returns; NULL when A
+ * is in place (ngroups = 0). */
 /* Grows the panel-copy scratch of plasma_pXpotrf_arrivals beforehand (a
  * slot that grows waits for every stream). */
 void plasma_pXpotrf_reserve(plasma_context_t *plasma, plasma_enum_t uplo, plasma_desc_t A,
@@ -401,7 +409,8 @@ void plasma_pXpotrf_reserve(plasma_context_t *plasma, plasma_enum_t uplo, plasma
 void plasma_pXpotrf_arrivals(plasma_context_t *plasma, plasma_enum_t uplo,
                              plasma_desc_t A, plasma_sequence_t *sequence,
                              plasma_request_t *request, int call, int mode,
-                             int ngroups, const int *gstart, const cudaEvent_t *arrive);
+                             int ngroups, const int *gstart, const cudaEvent_t *arrive,
+                             const float *diag);
 void plasma_pXpotrs(plasma_context_t *plasma, plasma_enum_t uplo,
                     plasma_desc_t A, plasma_desc_t B,
                     plasma_sequence_t *sequence, plasma_request_t *request);
