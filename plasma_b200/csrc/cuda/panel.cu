@@ -1,19 +1,22 @@
-// panel.cu -- FP64 critical path of a Cholesky step on the tensor cores:
+// panel.cu -- FP32 critical path of a Cholesky step on the tensor cores:
 // the diagonal-tile factorisation and the panel triangular solve
-// (compute/pzpotrf.c:41-56: plasma_core_dpotrf on A(k,k), then
-// plasma_core_dtrsm(Right, Lower, Trans, NonUnit) on every A(m,k), m > k).
+// (compute/pzpotrf.c:41-56: plasma_core_spotrf on A(k,k), then
+// plasma_core_strsm(Right, Lower, Trans, NonUnit) on every A(m,k), m > k)
+// for tiles that the shared-memory factor (potrf_smem.cu) and the tcgen05
+// solve (trsm_tc.cu) do not take, with TF32 products (SPLIT = 1 or 3).  FP64
+// tiles go to potrf_diag.cu and trsm_f64.cu.
 //
-// k_potrf_diag_dmma -- one CTA factors the diagonal tile left-looking in
+// k_potrf_diag_mma -- one CTA factors the diagonal tile left-looking in
 //   64-column panels.  The update of a panel by the columns to its left,
-//   P -= L(j0:n, 0:j0) L(j0:j0+64, 0:j0)^T, runs on DMMA (mma.sync f64); the
+//   P -= L(j0:n, 0:j0) L(j0:j0+64, 0:j0)^T, runs on mma.sync; the
 //   64-wide panel is then factored in shared memory as four 16-column
-//   sub-panels: DMMA update by the sub-panels to its left, one warp factors
+//   sub-panels: mma.sync update by the sub-panels to its left, one warp factors
 //   the 16x16 diagonal block through shuffles, and every thread solves one
 //   row below it (three barriers per 16 columns).
 //   Pivot test and info as LAPACK dpotrf (first pivot not > 0, or NaN).
-// k_trsm_panel_dmma -- X L^T = A(m,k) for all m > k.  A CTA keeps 64 rows of
+// k_trsm_panel_mma -- X L^T = A(m,k) for all m > k.  A CTA keeps 64 rows of
 //   one tile (all nb columns) in shared memory and walks the 64-column blocks
-//   left to right:  Y_j = X_j - X_{<j} L_{j,<j}^T  (DMMA, L streamed from L2
+//   left to right:  Y_j = X_j - X_{<j} L_{j,<j}^T  (mma.sync, L streamed from L2
 //   through a cp.async double buffer), then X_j L_jj^T = Y_j by right-looking
 //   substitution, four lanes per row exchanging the solved entry by shuffle.
 #include "common.cuh"
@@ -65,7 +68,7 @@ k_potrf_diag_mma(plasma_desc_t A, int k, int iinfo, plasma_devstat_t *st,
             cp_async_el(P + c * P_LD + r, v ? L + (size_t)(j0 + c) * ld + j0 + r : L, v);
         }
         cp_async_commit();
-        // ---- left-looking update on DMMA: warp w owns rows 32w..32w+31,
+        // ---- left-looking update on mma.sync: warp w owns rows 32w..32w+31,
         //      operand chunks double-buffered through cp.async
         if (j0 > 0) {
             T acc[2][8][4];
@@ -155,7 +158,7 @@ k_potrf_diag_mma(plasma_desc_t A, int k, int iinfo, plasma_devstat_t *st,
         T *rdiag_s = Sa + 4;               // reciprocals of the block diagonal
         for (int cs = 0; cs < jb; cs += SP) {
             const int sw = min(SP, jb - cs);
-            // (a) sub-panel -= previous sub-panels of this panel (DMMA, K = cs)
+            // (a) sub-panel -= previous sub-panels of this panel (K = cs)
             if (cs > 0) {
                 T acc[2][2][4];
 #pragma unroll
@@ -477,7 +480,7 @@ extern "C" int plasma_cuda_potrf_diag_fast(cudaStream_t s, plasma_devstat_t *st,
     double nk = plasma_tile_mview(A, k);
     int prof = plasma_prof_begin(s);
     if (A.precision == PlasmaRealDouble)
-        launch_diag<double, 1>(s, st, call, A, k, iinfo);
+        plasma_cuda_potrf_diag_f64(s, st, call, A, k, iinfo);   // potrf_diag.cu
     else if (plasma_cuda_potrf_diag_smem(s, st, call, uplo, A, k, iinfo, g_fp32_split))
         ;   // FP32 tile held in shared memory (potrf_smem.cu)
     else if (g_fp32_split == 1)
@@ -497,8 +500,8 @@ extern "C" int plasma_cuda_trsm_panel_fast(cudaStream_t s, plasma_devstat_t *st,
         (A.precision != PlasmaRealDouble && A.precision != PlasmaRealFloat))
         return 0;
     int nk = plasma_tile_mview(A, k);
-    int align = A.precision == PlasmaRealDouble ? 2 : 4;
-    if (nk % PB != 0 || plasma_tile_mmain(A, k) % align != 0)
+    if (A.precision == PlasmaRealDouble ? nk % 32 != 0
+                                        : nk % PB != 0 || plasma_tile_mmain(A, k) % 4 != 0)
         return 0;
     if (mhi <= mlo)
         return 1;
@@ -507,7 +510,7 @@ extern "C" int plasma_cuda_trsm_panel_fast(cudaStream_t s, plasma_devstat_t *st,
     for (int m = mlo; m < mhi; m++) rows += plasma_tile_mview(A, m);
     int prof = plasma_prof_begin(s);
     if (A.precision == PlasmaRealDouble)
-        launch_trsm<double, 1>(s, st, A, k, mlo, mhi);
+        plasma_cuda_trsm_f64(s, st, A, k, mlo, mhi);            // trsm_f64.cu
     else if (g_fp32_split == 1)
         launch_trsm<float, 1>(s, st, A, k, mlo, mhi);
     else

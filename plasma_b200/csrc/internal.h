@@ -307,6 +307,12 @@ void plasma_cuda_panel_round(cudaStream_t s, plasma_devstat_t *st, int tc_mode,
 int plasma_cuda_potrf_diag_smem(cudaStream_t s, plasma_devstat_t *st, int call,
                                 plasma_enum_t uplo, plasma_desc_t A, int k,
                                 int iinfo, int split);
+/* FP64 diagonal tile of order <= 256 (cuda/potrf_diag.cu); 0 for others. */
+int plasma_cuda_potrf_diag_f64(cudaStream_t s, plasma_devstat_t *st, int call,
+                               plasma_desc_t A, int k, int iinfo);
+/* FP64 panel solve, tile columns a multiple of 32 (cuda/trsm_f64.cu). */
+int plasma_cuda_trsm_f64(cudaStream_t s, plasma_devstat_t *st, plasma_desc_t A, int k,
+                         int mlo, int mhi);
 /* FP32 panel kernels: 3 = FP32-accurate split TF32 products, 1 = TF32. */
 void plasma_cuda_panel_set_split(int split);
 /* A(i,i) = value for i in [i0, i1) (identity padding of FP32 factors). */
