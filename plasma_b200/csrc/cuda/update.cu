@@ -66,15 +66,17 @@ __host__ __device__ __forceinline__ long long count_items(int nlo, int nhi,
 // SM: one CTA's epilogue (a read-modify-write of C from HBM) overlaps the
 // other's tensor-core main loop.  The C block is prefetched into L2 when the
 // item starts, so the epilogue reads hit L2.
+//
+// A 128 x 64 block with K = 128 takes 8.6 us of one SM's FP64 pipe whatever
+// else runs, so a launch with fewer blocks than SMs (the next panel's column,
+// a band's step, a small matrix: the critical path) is cut into 64 x 32
+// blocks, four times as many.
 // ---------------------------------------------------------------------------
 constexpr int DBM = 128;
 constexpr int DBN = 64;
 constexpr int DBK = 16;
 constexpr int DSTAGES = 4;
 constexpr int DPAD = 4;                 // row strides 132 / 68 doubles
-constexpr int DLDS_A = DBM + DPAD;
-constexpr int DLDS_B = DBN + DPAD;
-constexpr int DSMEM = DSTAGES * DBK * (DLDS_A + DLDS_B) * (int)sizeof(double);
 
 struct DmmaOperands {
     const double *a; int lda; int arows;   // A(m,k) logical rows
@@ -83,6 +85,14 @@ struct DmmaOperands {
     bool vec;                              // 16-byte copies are legal
 };
 
+template <int TM, int TN>
+struct UpdGeo {
+    static constexpr int LDA = TM + DPAD, LDB = TN + DPAD;
+    static constexpr int MI = TM / 64, NI = TN / 16;     // m16 x n8 pieces per warp
+    static constexpr int SMEM = DSTAGES * DBK * (LDA + LDB) * (int)sizeof(double);
+};
+
+template <int TM, int TN>
 __device__ __forceinline__ void dmma_load_stage(double *As, double *Bs,
                                                 const DmmaOperands &op,
                                                 int kc, int tid)
@@ -90,45 +100,46 @@ __device__ __forceinline__ void dmma_load_stage(double *As, double *Bs,
     if (op.vec) {
         // pairs of rows: A chunk 64 pairs x 16 cols, B chunk 32 pairs x 16
 #pragma unroll
-        for (int q = 0; q < (DBM * DBK / 2) / THREADS; q++) {
+        for (int q = 0; q < (TM * DBK / 2) / THREADS; q++) {
             int e = tid + q * THREADS;
-            int r = 2 * (e % (DBM / 2)), c = e / (DBM / 2);
+            int r = 2 * (e % (TM / 2)), c = e / (TM / 2);
             int gi = op.i0 + r, gk = kc + c;
             bool v = gi < op.arows && gk < op.K;
             const double *src = v ? op.a + (size_t)gk * op.lda + gi : op.a;
-            cp_async_16(As + c * DLDS_A + r, src, v);
+            cp_async_16(As + c * (TM + DPAD) + r, src, v);
         }
 #pragma unroll
-        for (int q = 0; q < (DBN * DBK / 2) / THREADS; q++) {
+        for (int q = 0; q < (TN * DBK / 2) / THREADS; q++) {
             int e = tid + q * THREADS;
-            int r = 2 * (e % (DBN / 2)), c = e / (DBN / 2);
+            int r = 2 * (e % (TN / 2)), c = e / (TN / 2);
             int gj = op.j0 + r, gk = kc + c;
             bool v = gj < op.brows && gk < op.K;
             const double *src = v ? op.b + (size_t)gk * op.ldb + gj : op.b;
-            cp_async_16(Bs + c * DLDS_B + r, src, v);
+            cp_async_16(Bs + c * (TN + DPAD) + r, src, v);
         }
         return;
     }
 #pragma unroll
-    for (int q = 0; q < (DBM * DBK) / THREADS; q++) {
+    for (int q = 0; q < (TM * DBK) / THREADS; q++) {
         int e = tid + q * THREADS;
-        int r = e % DBM, c = e / DBM;
+        int r = e % TM, c = e / TM;
         int gi = op.i0 + r, gk = kc + c;
         bool v = gi < op.arows && gk < op.K;
         const double *src = v ? op.a + (size_t)gk * op.lda + gi : op.a;
-        cp_async_8(As + c * DLDS_A + r, src, v);
+        cp_async_8(As + c * (TM + DPAD) + r, src, v);
     }
 #pragma unroll
-    for (int q = 0; q < (DBN * DBK) / THREADS; q++) {
+    for (int q = 0; q < (TN * DBK) / THREADS; q++) {
         int e = tid + q * THREADS;
-        int r = e % DBN, c = e / DBN;
+        int r = e % TN, c = e / TN;
         int gj = op.j0 + r, gk = kc + c;
         bool v = gj < op.brows && gk < op.K;
         const double *src = v ? op.b + (size_t)gk * op.ldb + gj : op.b;
-        cp_async_8(Bs + c * DLDS_B + r, src, v);
+        cp_async_8(Bs + c * (TN + DPAD) + r, src, v);
     }
 }
 
+template <int TM, int TN>
 __global__ void __launch_bounds__(THREADS, 2)
 k_update_dmma(plasma_desc_t A, int k, int nlo, int nhi, int nitems,
               const plasma_devstat_t *st)
@@ -136,16 +147,17 @@ k_update_dmma(plasma_desc_t A, int k, int nlo, int nhi, int nitems,
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if (plasma_failed(st)) return;
     double *As = reinterpret_cast<double *>(smem_raw);
-    double *Bs = As + DSTAGES * DBK * DLDS_A;
+    double *Bs = As + DSTAGES * DBK * (TM + DPAD);
 
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const int wm = warp >> 1;          // 0..3 -> 32 rows each
-    const int wn = warp & 1;           // 0..1 -> 32 cols each
+    constexpr int MI = UpdGeo<TM, TN>::MI, NI = UpdGeo<TM, TN>::NI;
+    const int wm = warp >> 1;          // 0..3 -> 16 MI rows each
+    const int wn = warp & 1;           // 0..1 -> 8 NI cols each
     const int mt = A.mt;
-    const int sbm = (A.mb + DBM - 1) / DBM;
-    const int sbn = (A.mb + DBN - 1) / DBN;
+    const int sbm = (A.mb + TM - 1) / TM;
+    const int sbn = (A.mb + TN - 1) / TN;
 
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         Item it;
@@ -161,10 +173,10 @@ k_update_dmma(plasma_desc_t A, int k, int nlo, int nhi, int nitems,
             it.m = n + p;
         }
         DmmaOperands op;
-        op.i0 = it.si * DBM;
-        op.j0 = it.sj * DBN;
+        op.i0 = it.si * TM;
+        op.j0 = it.sj * TN;
         // a block of a diagonal tile that lies strictly above the diagonal
-        if (it.m == it.n && op.j0 > op.i0 + DBM - 1) continue;
+        if (it.m == it.n && op.j0 > op.i0 + TM - 1) continue;
         op.a = (const double *)plasma_tile_addr(A, it.m, k);
         op.lda = plasma_tile_mmain(A, it.m);
         op.arows = plasma_tile_mview(A, it.m);
@@ -177,19 +189,19 @@ k_update_dmma(plasma_desc_t A, int k, int nlo, int nhi, int nitems,
 
         double *C = (double *)plasma_tile_addr(A, it.m, it.n);
         const int ldc = plasma_tile_mmain(A, it.m);
-        // warm L2 with the C block: 64 columns x 128 rows = 512 lines
-        for (int e = tid; e < DBN * (DBM / 16); e += THREADS) {
-            int j = op.j0 + e / (DBM / 16);
-            int i = op.i0 + (e % (DBM / 16)) * 16;
+        // warm L2 with the C block
+        for (int e = tid; e < TN * (TM / 16); e += THREADS) {
+            int j = op.j0 + e / (TM / 16);
+            int i = op.i0 + (e % (TM / 16)) * 16;
             if (j < op.brows && i < op.arows)
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(C + (size_t)j * ldc + i));
         }
 
-        double acc[2][4][4];
+        double acc[MI][NI][4];
 #pragma unroll
-        for (int a = 0; a < 2; a++)
+        for (int a = 0; a < MI; a++)
 #pragma unroll
-            for (int b = 0; b < 4; b++)
+            for (int b = 0; b < NI; b++)
 #pragma unroll
                 for (int c = 0; c < 4; c++) acc[a][b][c] = 0.0;
 
@@ -198,7 +210,7 @@ k_update_dmma(plasma_desc_t A, int k, int nlo, int nhi, int nitems,
 #pragma unroll
         for (int s = 0; s < DSTAGES - 1; s++) {
             if (s < nk)
-                dmma_load_stage(As + s * DBK * DLDS_A, Bs + s * DBK * DLDS_B,
+                dmma_load_stage<TM, TN>(As + s * DBK * (TM + DPAD), Bs + s * DBK * (TN + DPAD),
                                 op, s * DBK, tid);
             cp_async_commit();
         }
@@ -208,30 +220,30 @@ k_update_dmma(plasma_desc_t A, int k, int nlo, int nhi, int nitems,
             int pf = kt + DSTAGES - 1;
             if (pf < nk) {
                 int sl = pf % DSTAGES;
-                dmma_load_stage(As + sl * DBK * DLDS_A, Bs + sl * DBK * DLDS_B,
+                dmma_load_stage<TM, TN>(As + sl * DBK * (TM + DPAD), Bs + sl * DBK * (TN + DPAD),
                                 op, pf * DBK, tid);
             }
             cp_async_commit();
 
-            const double *as = As + (kt % DSTAGES) * DBK * DLDS_A + wm * 32;
-            const double *bs = Bs + (kt % DSTAGES) * DBK * DLDS_B + wn * 32;
+            const double *as = As + (kt % DSTAGES) * DBK * (TM + DPAD) + wm * 16 * MI;
+            const double *bs = Bs + (kt % DSTAGES) * DBK * (TN + DPAD) + wn * 8 * NI;
 #pragma unroll
             for (int k8 = 0; k8 < DBK; k8 += 8) {
-                double bf[4][2];
+                double bf[NI][2];
 #pragma unroll
-                for (int ni = 0; ni < 4; ni++) {
-                    bf[ni][0] = bs[(k8 + t) * DLDS_B + ni * 8 + g];
-                    bf[ni][1] = bs[(k8 + t + 4) * DLDS_B + ni * 8 + g];
+                for (int ni = 0; ni < NI; ni++) {
+                    bf[ni][0] = bs[(k8 + t) * (TN + DPAD) + ni * 8 + g];
+                    bf[ni][1] = bs[(k8 + t + 4) * (TN + DPAD) + ni * 8 + g];
                 }
 #pragma unroll
-                for (int mi = 0; mi < 2; mi++) {
+                for (int mi = 0; mi < MI; mi++) {
                     double af[4];
-                    af[0] = as[(k8 + t) * DLDS_A + mi * 16 + g];
-                    af[1] = as[(k8 + t) * DLDS_A + mi * 16 + g + 8];
-                    af[2] = as[(k8 + t + 4) * DLDS_A + mi * 16 + g];
-                    af[3] = as[(k8 + t + 4) * DLDS_A + mi * 16 + g + 8];
+                    af[0] = as[(k8 + t) * (TM + DPAD) + mi * 16 + g];
+                    af[1] = as[(k8 + t) * (TM + DPAD) + mi * 16 + g + 8];
+                    af[2] = as[(k8 + t + 4) * (TM + DPAD) + mi * 16 + g];
+                    af[3] = as[(k8 + t + 4) * (TM + DPAD) + mi * 16 + g + 8];
 #pragma unroll
-                    for (int ni = 0; ni < 4; ni++)
+                    for (int ni = 0; ni < NI; ni++)
                         dmma_16x8x8(acc[mi][ni], af, bf[ni]);
                 }
             }
@@ -242,28 +254,28 @@ k_update_dmma(plasma_desc_t A, int k, int nlo, int nhi, int nitems,
         // before any store so that their latencies overlap.
         const bool diag = it.m == it.n;
 #pragma unroll
-        for (int mi = 0; mi < 2; mi++) {
-            double cv[2][4][2];
+        for (int mi = 0; mi < MI; mi++) {
+            double cv[2][NI][2];
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                int i = op.i0 + wm * 32 + mi * 16 + g + h * 8;
+                int i = op.i0 + wm * 16 * MI + mi * 16 + g + h * 8;
 #pragma unroll
-                for (int ni = 0; ni < 4; ni++)
+                for (int ni = 0; ni < NI; ni++)
 #pragma unroll
                     for (int e = 0; e < 2; e++) {
-                        int j = op.j0 + wn * 32 + ni * 8 + 2 * t + e;
+                        int j = op.j0 + wn * 8 * NI + ni * 8 + 2 * t + e;
                         bool ok = i < op.arows && j < op.brows && (!diag || i >= j);
                         cv[h][ni][e] = ok ? C[(size_t)j * ldc + i] : 0.0;
                     }
             }
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                int i = op.i0 + wm * 32 + mi * 16 + g + h * 8;
+                int i = op.i0 + wm * 16 * MI + mi * 16 + g + h * 8;
 #pragma unroll
-                for (int ni = 0; ni < 4; ni++)
+                for (int ni = 0; ni < NI; ni++)
 #pragma unroll
                     for (int e = 0; e < 2; e++) {
-                        int j = op.j0 + wn * 32 + ni * 8 + 2 * t + e;
+                        int j = op.j0 + wn * 8 * NI + ni * 8 + 2 * t + e;
                         bool ok = i < op.arows && j < op.brows && (!diag || i >= j);
                         if (ok)
                             C[(size_t)j * ldc + i] = cv[h][ni][e] - acc[mi][ni][h * 2 + e];
@@ -547,6 +559,18 @@ k_update_simt(plasma_desc_t A, int uplo, int k, int nlo, int nhi, int nitems,
     }
 }
 
+template <int TM, int TN>
+void launch_dmma(cudaStream_t s, const plasma_devstat_t *st, const plasma_desc_t &A, int k,
+                 int nlo, int nhi, long long nitems)
+{
+    constexpr int SMEM = UpdGeo<TM, TN>::SMEM;
+    static unsigned long long attr = 0;
+    if (plasma_first_on_device(&attr))
+        cudaFuncSetAttribute(k_update_dmma<TM, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             SMEM);
+    k_update_dmma<TM, TN><<<(unsigned)nitems, THREADS, SMEM, s>>>(A, k, nlo, nhi, (int)nitems, st);
+}
+
 }  // namespace
 
 extern "C" void plasma_cuda_update(cudaStream_t s, plasma_devstat_t *st,
@@ -557,9 +581,12 @@ extern "C" void plasma_cuda_update(cudaStream_t s, plasma_devstat_t *st,
     const bool dmma = A.precision == PlasmaRealDouble && uplo == PlasmaLower;
     int sb = (A.mb + BM - 1) / BM;
     long long nitems = count_items(nlo, nhi, A.mt, sb);
+    bool small = false;
     if (dmma) {
-        long long pairs = count_items(nlo, nhi, A.mt, 1);
-        nitems = pairs * ((A.mb + DBM - 1) / DBM) * ((A.mb + DBN - 1) / DBN);
+        const long long pairs = count_items(nlo, nhi, A.mt, 1);
+        nitems = pairs * ceil_div(A.mb, DBM) * ceil_div(A.mb, DBN);
+        small = nitems <= num_sms;
+        if (small) nitems = pairs * ceil_div(A.mb, DBM / 2) * ceil_div(A.mb, DBN / 2);
     }
     if (nitems <= 0) return;
     PLASMA_COUNT_LAUNCH();
@@ -579,18 +606,12 @@ extern "C" void plasma_cuda_update(cudaStream_t s, plasma_devstat_t *st,
     }
     int prof = plasma_prof_begin(s);
     if (dmma) {
-        static unsigned long long attr_set = 0;
-        if (plasma_first_on_device(&attr_set)) {
-            cudaFuncSetAttribute(k_update_dmma,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 DSMEM);
-        }
         // one CTA per work item: SMs free up often, so the high-priority
         // critical-path kernels of the next step are scheduled in between
-        long long grid = nitems;
-        (void)num_sms;
-        k_update_dmma<<<(unsigned)grid, THREADS, DSMEM, s>>>(
-            A, k, nlo, nhi, (int)nitems, st);
+        if (small)
+            launch_dmma<DBM / 2, DBN / 2>(s, st, A, k, nlo, nhi, nitems);
+        else
+            launch_dmma<DBM, DBN>(s, st, A, k, nlo, nhi, nitems);
     } else {
         long long grid = nitems;     // one CTA per item (see above)
         if (A.precision == PlasmaRealDouble)
