@@ -22,42 +22,12 @@
 // Lower storage: L(i,j) is element (i,j) of tile (i/nb, j/nb).  Upper storage
 // (A = U^T U): L(i,j) = U(j,i).
 #include "common.cuh"
+#include "inv64.cuh"
+#include "sweep.cuh"
 
 namespace {
 
 constexpr int TS_THREADS = 256;
-
-struct SweepSync {
-    int ticket;
-    int abort;
-    int flags[1];          // [nblk]
-};
-
-__device__ __forceinline__ int ld_acquire(const int *p)
-{
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release(int *p, int v)
-{
-    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-__device__ bool wait_block(SweepSync *sy, int k, int epoch)
-{
-    long long t0 = clock64();
-    while (ld_acquire(&sy->flags[k]) != epoch) {
-        if (ld_acquire(&sy->abort)) return false;
-        if (clock64() - t0 > 4000000000LL) {
-            atomicExch(&sy->abort, 1);
-            return false;
-        }
-        __nanosleep(32);
-    }
-    return true;
-}
 
 template <typename T>
 __device__ __forceinline__ void cp_async_el_any(T *dst, const T *src)
@@ -73,37 +43,6 @@ __device__ __forceinline__ void cp_async_el_any_z(T *dst, const T *src, bool val
 {
     if (sizeof(T) == 8) cp_async_8(dst, src, valid);
     else cp_async_4(dst, src, valid);
-}
-
-// Logical block (bi, bj) of L, SB x SB: element (i,j) at p[i*si + j*sj].
-template <typename T>
-struct LBlock {
-    const T *p;
-    int si, sj;
-};
-
-template <typename T, int SB>
-__device__ __forceinline__ LBlock<T> lblock(const plasma_desc_t &A, bool lower,
-                                            int bi, int bj)
-{
-    const int gi = bi * SB, gj = bj * SB;
-    const int ti = gi / A.mb, tj = gj / A.mb;
-    const int oi = gi % A.mb, oj = gj % A.mb;
-    LBlock<T> b;
-    if (lower) {
-        const T *t = (const T *)plasma_tile_addr(A, ti, tj);
-        int ld = plasma_tile_mmain(A, ti);
-        b.p = t + (size_t)oj * ld + oi;
-        b.si = 1;
-        b.sj = ld;
-    } else {
-        const T *t = (const T *)plasma_tile_addr(A, tj, ti);
-        int ld = plasma_tile_mmain(A, tj);
-        b.p = t + (size_t)oi * ld + oj;
-        b.si = ld;
-        b.sj = 1;
-    }
-    return b;
 }
 
 // ys[i] -= sum_c M(i,c) xs[c] for i < rows, c < cols, M(i,c) = m[i*si + c*sj].
@@ -216,13 +155,14 @@ k_trsv(plasma_desc_t A, int uplo, int backward, const T *W, T *vec,
         if (t >= nblk) break;
         const int u = backward ? nblk - 1 - t : t;
         const int rows = min(SB, n - u * SB);
+        const int s0 = sweep_first(A, lower, t, SB, backward != 0, nblk);
 
         // stage W_u and the critical block (the coupling with the block of
         // ticket t-1) in shared memory; both are read-only factor data
         const T *wu = W + (size_t)u * SB * SB;
         for (int e = tid; e < SB * SB; e += TS_THREADS)
             cp_async_el_any(Wc + e, wu + e);
-        const int kc = t > 0 ? (backward ? u + 1 : u - 1) : -1;
+        const int kc = s0 < t ? (backward ? u + 1 : u - 1) : -1;
         const int kcr = kc >= 0 ? min(SB, n - kc * SB) : 0;
         if (kc >= 0) {
             // logical block stored as Lc[c*SB + i]:
@@ -243,7 +183,7 @@ k_trsv(plasma_desc_t A, int uplo, int backward, const T *W, T *vec,
         for (int i = tid; i < SB; i += TS_THREADS)
             ys[i] = i < rows ? vec[(size_t)u * SB + i] : T(0);
 
-        for (int s = 0; s < t; s++) {
+        for (int s = s0; s < t; s++) {
             const int k = backward ? nblk - 1 - s : s;
             const int kr = min(SB, n - k * SB);
             if (tid == 0) {
@@ -276,7 +216,7 @@ k_trsv(plasma_desc_t A, int uplo, int backward, const T *W, T *vec,
                 }
             }
         }
-        if (t == 0) cp_async_wait<0>();
+        if (s0 >= t) cp_async_wait<0>();
         __syncthreads();
         // diagonal block: ys <- W_u ys (forward) or W_u^T ys (backward)
         for (int i = tid; i < SB; i += TS_THREADS) {
@@ -291,6 +231,36 @@ k_trsv(plasma_desc_t A, int uplo, int backward, const T *W, T *vec,
         __syncthreads();
         if (tid == 0) st_release(&sy->flags[u], epoch);
     }
+}
+
+// W_u = inv(logical L diagonal block u, 64 x 64), formed in FP64 by
+// inv_lower64 (8 x 8 blocks, then products): 9 us where the column-by-column
+// elimination of k_trtri_blocks below takes 40.  Layout, padding and `unit`
+// as there.
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_trtri_64(plasma_desc_t A, int uplo, int unit, T *W, const plasma_devstat_t *st)
+{
+    extern __shared__ double t64_smem[];
+    double (*Ls)[65] = reinterpret_cast<double (*)[65]>(t64_smem);
+    double (*Iv)[65] = Ls + 64;
+    double (*Tm)[33] = reinterpret_cast<double (*)[33]>(Iv + 64);
+    if (plasma_failed(st)) return;
+    const int u = blockIdx.x, n = A.m;
+    const int rows = min(64, n - u * 64);
+    LBlock<T> b = lblock<T, 64>(A, uplo == PlasmaLower, u, u);
+    const int tid = threadIdx.x;
+    for (int e = tid; e < 64 * 64; e += 256) {
+        // lanes along the contiguous index of the storage
+        const int x = e % 64, y = e / 64, i = b.si == 1 ? x : y, c = b.si == 1 ? y : x;
+        Ls[i][c] = (i < rows && c < rows && i >= c && !(unit && i == c))
+            ? (double)b.p[(size_t)i * b.si + (size_t)c * b.sj] : (i == c ? 1.0 : 0.0);
+        Iv[i][c] = 0.0;
+    }
+    __syncthreads();
+    inv_lower64(Ls, Iv, Tm, false);
+    T *w = W + (size_t)u * 64 * 64;
+    for (int e = tid; e < 64 * 64; e += 256) w[e] = (T)Iv[e % 64][e / 64];
 }
 
 // W_u = inv(logical L diagonal block u, SB x SB), written densely
@@ -341,9 +311,9 @@ k_trtri_blocks(plasma_desc_t A, int uplo, int unit, T *W, const plasma_devstat_t
 }
 
 // ---------------------------------------------------------------------------
-// One-launch sweeps for a few right-hand sides (potrs / posv with
-// 2 <= nrhs <= 32; the reference runs them as the tile tasks of pztrsm.c):
-// the ticketed row blocks of k_trsv, each applied to NR columns of B at
+// One-launch sweeps for a few right-hand sides of FP32 factors (potrs / posv
+// with 2 <= nrhs <= 32; the reference runs them as the tile tasks of
+// pztrsm.c; FP64 factors take trsm_rows.cu): the ticketed row blocks of k_trsv, each applied to NR columns of B at
 // once, so the factor is read once per NR columns instead of once per
 // column, and B stays in its tile layout.
 //   forward : X_u = W_u   (B_u - sum_{k<u} L(u,k) X_k)
@@ -363,14 +333,6 @@ template <typename T, int SB, int NR>
 constexpr int trsm_rows_smem()
 {
     return (2 * SB * (SB + 1) + SB * NR + (TR_THREADS / SB) * SB * NR) * (int)sizeof(T);
-}
-
-template <typename T>
-__device__ __forceinline__ T *b_elem(const plasma_desc_t &B, int row, int col)
-{
-    const int m = row / B.mb, r = row - m * B.mb;
-    const int t = col / B.nb, c = col - t * B.nb;
-    return (T *)plasma_tile_addr(B, m, t) + (size_t)c * plasma_tile_mmain(B, m) + r;
 }
 
 // Ms[c*(SB+1) + i] <- q[i*mi + c*mc] for i < ri, c < rc, zero elsewhere
@@ -423,6 +385,7 @@ k_trsm_rows(plasma_desc_t A, int uplo, int backward, const T *W, plasma_desc_t B
         if (t >= nblk) break;
         const int u = backward ? nblk - 1 - t : t;
         const int rows = min(SB, n - u * SB);
+        const int s0 = sweep_first(A, lower, t, SB, backward != 0, nblk);
 
         // operator of ticket s: forward L(u,k), backward L(k,u)^T
         auto stage = [&](int s, T *buf) {
@@ -439,9 +402,9 @@ k_trsm_rows(plasma_desc_t A, int uplo, int backward, const T *W, plasma_desc_t B
         T acc[NR];
 #pragma unroll
         for (int j = 0; j < NR; j++) acc[j] = T(0);
-        if (t > 0) stage(0, Ms[0]);
+        if (s0 < t) stage(s0, Ms[s0 & 1]);
         cp_async_commit();
-        for (int s = 0; s < t; s++) {
+        for (int s = s0; s < t; s++) {
             const int k = backward ? nblk - 1 - s : s;
             const int kr = min(SB, n - k * SB);
             if (s + 1 < t) stage(s + 1, Ms[(s + 1) & 1]);
@@ -774,11 +737,12 @@ k_trsv_ll(plasma_desc_t A, int uplo, int backward, Couple C, float *vec,
         float bu = 0.f;
         if (tid < rows) bu = vec[(size_t)u * LL_SB + tid];
 
-        // off the chain: blocks j = 0 .. nnc-1 in sweep order (block
-        // k(j) = j forward, nblk-1-j backward), three in flight: the
+        // off the chain: blocks j = 0 .. nnc-1 in sweep order (block k(j) =
+        // s0+j forward, nblk-1-s0-j backward), three in flight: the
         // factor elements of block j+3 are requested as soon as block j
         // is consumed
-        const int nnc = t > 0 ? t - 1 : 0;
+        const int s0 = sweep_first(A, lower, t, LL_SB, backward != 0, nblk);
+        const int nnc = t > s0 ? t - 1 - s0 : 0;
         float acc[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) acc[j] = 0.f;
@@ -786,7 +750,7 @@ k_trsv_ll(plasma_desc_t A, int uplo, int backward, Couple C, float *vec,
         if (nnc > 0) {
             float4 b0[8], b1[8], b2[8];
             unsigned long long w0 = 0ull, w1 = 0ull, w2 = 0ull;
-            auto blk_of = [&](int j) { return backward ? nblk - 1 - j : j; };
+            auto blk_of = [&](int j) { return backward ? nblk - 1 - s0 - j : s0 + j; };
             auto issue = [&](int j, float4 (&b)[8], unsigned long long &w) {
                 if (j < nnc) {
                     const int k = blk_of(j);
@@ -963,6 +927,14 @@ template <typename T, int SB>
 void launch_trtri(cudaStream_t s, plasma_devstat_t *st, int uplo,
                   const plasma_desc_t &A, void *W, int nblk, int unit = 0)
 {
+    if constexpr (SB == 64) {
+        constexpr int SMEM = (2 * 64 * 65 + 64 * 33) * (int)sizeof(double);
+        static unsigned long long attr64 = 0;
+        if (plasma_first_on_device(&attr64))
+            cudaFuncSetAttribute(k_trtri_64<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        k_trtri_64<T><<<nblk, 256, SMEM, s>>>(A, uplo, unit, (T *)W, st);
+        return;
+    } else {
     static unsigned long long attr = 0;
     if (plasma_first_on_device(&attr)) {
         cudaFuncSetAttribute(k_trtri_blocks<T, SB>,
@@ -970,6 +942,7 @@ void launch_trtri(cudaStream_t s, plasma_devstat_t *st, int uplo,
                              trtri_smem<T, SB>());
     }
     k_trtri_blocks<T, SB><<<nblk, 256, trtri_smem<T, SB>(), s>>>(A, uplo, unit, (T *)W, st);
+    }
 }
 
 template <typename T, int SB>
@@ -1030,7 +1003,10 @@ size_t flags_bytes(int nblk)
 extern "C" int plasma_cuda_trsv_block(plasma_desc_t A)
 {
     if (A.mb != A.nb || A.mb % 64 != 0) return 0;
-    if (A.precision == PlasmaRealFloat && A.mb % 128 == 0) return 128;
+    // (a diagonal band holds no tile that the coupled sweep could read)
+    if (A.precision == PlasmaRealFloat && A.mb % 128 == 0 &&
+        !(A.type == PlasmaGeneralBand && A.kl + A.ku == 0))
+        return 128;
     if (A.precision == PlasmaRealFloat || A.precision == PlasmaRealDouble) return 64;
     return 0;
 }
@@ -1178,12 +1154,7 @@ extern "C" int plasma_cuda_trsm_rows(cudaStream_t s, plasma_devstat_t *st,
     PLASMA_COUNT_LAUNCH();
     int prof = plasma_prof_begin(s);
     if (A.precision == PlasmaRealDouble) {
-        if (ncols <= 4)
-            launch_trsm_rows<double, 64, 4>(s, st, uplo, backward, A, W, B, c0, ncols, sy,
-                                            epoch, grid);
-        else
-            launch_trsm_rows<double, 64, 16>(s, st, uplo, backward, A, W, B, c0, ncols, sy,
-                                             epoch, grid);
+        plasma_cuda_trsm_rows_f64(s, st, uplo, backward, A, W, B, c0, ncols, sy, epoch, grid);
     } else if (sb == 128) {
         if (ncols <= 4)
             launch_trsm_rows<float, 128, 4>(s, st, uplo, backward, A, W, B, c0, ncols, sy,

@@ -361,6 +361,9 @@ int plasma_cuda_trsv(cudaStream_t s, plasma_devstat_t *st, plasma_enum_t uplo,
 int plasma_cuda_trsm_rows(cudaStream_t s, plasma_devstat_t *st, plasma_enum_t uplo,
                           int backward, plasma_desc_t A, const void *W, plasma_desc_t B,
                           int c0, int ncols, void *sync, int epoch, int num_sms);
+void plasma_cuda_trsm_rows_f64(cudaStream_t s, plasma_devstat_t *st, plasma_enum_t uplo,
+                               int backward, plasma_desc_t A, const void *W, plasma_desc_t B,
+                               int c0, int ncols, void *sync, int epoch, int grid);
 size_t plasma_cuda_dots_work(int nv);
 void plasma_cuda_dots(cudaStream_t s, const double *V, size_t ldv, int nv,
                       const double *w, size_t n, double *out, double *work);
