@@ -218,12 +218,16 @@ static int Xposv(plasma_enum_t prec, plasma_enum_t uplo, int n, int nrhs,
      * diagonal blocks for the way back, so B is converted before it and
      * after it */
     const int via_lower = uplo == PlasmaUpper;
-    plasma_desc_t A, B;
+    plasma_desc_t F, A, B;         /* F: A with its padding (plasma_potrf_order) */
     /* the tile copy of A lives in a slot the context keeps between calls */
+    const int np = plasma_potrf_order(plasma, prec, nb, n);
     int retval = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_A, prec,
-                                  via_lower ? PlasmaLower : uplo, nb, n, n, &A);
+                                  via_lower ? PlasmaLower : uplo, nb, np, np, &F);
     if (retval != PlasmaSuccess)
         return retval;
+    A = plasma_desc_view(F, 0, 0, n, n);
+    if (np > n)
+        plasma_cuda_set_diag(plasma->stream, F, n, np, 1.0);
     retval = plasma_desc_general_create(prec, nb, nb, n, nrhs, 0, 0, n, nrhs, &B);
     if (retval != PlasmaSuccess)
         return retval;
@@ -239,7 +243,13 @@ static int Xposv(plasma_enum_t prec, plasma_enum_t uplo, int n, int nrhs,
         plasma_omp_Xlapack2desc(pA, lda, A, uplo, &sequence, &request);
         plasma_omp_Xlapack2desc(pB, ldb, B, PlasmaGeneral, &sequence, &request);
     }
-    plasma_omp_Xposv(via_lower ? PlasmaLower : uplo, A, B, &sequence, &request);
+    /* plasma_omp_Xposv with the padded factor */
+    const plasma_enum_t tri = via_lower ? PlasmaLower : uplo;
+    if (check_async(plasma, tri, F, B, &sequence, &request)) {
+        int call = plasma_call_begin(plasma, &sequence, &request);
+        plasma_pXpotrf(plasma, tri, F, &sequence, &request, call);
+        plasma_pXpotrs(plasma, tri, A, B, &sequence, &request);
+    }
     plasma_sequence_wait(&sequence);
     if (via_lower)
         plasma_omp_Xdesc2lapack_t(A, pA, lda, &sequence, &request);

@@ -391,6 +391,7 @@ void plasma_cuda_column(cudaStream_t s, plasma_desc_t D, int j, void *v,
 int plasma_sweep_reserve(plasma_context_t *plasma, plasma_desc_t A);
 int plasma_sweep_rows(plasma_context_t *plasma, plasma_enum_t uplo, int backward,
                       plasma_desc_t A, const void *W, plasma_desc_t B, int c0, int ncols);
+int plasma_potrf_order(plasma_context_t *plasma, plasma_enum_t prec, int nb, int n);
 int plasma_desc_kept(plasma_context_t *c, int slot, plasma_enum_t precision,
                      plasma_enum_t type, int nb, int m, int n, plasma_desc_t *A);
 int plasma_sweep(plasma_context_t *plasma, plasma_enum_t uplo, int backward,

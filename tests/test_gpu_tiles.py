@@ -109,3 +109,53 @@ def test_fp32_indefinite_info(L):
     for nb in (128, 256):
         info, _ = potrf(L, a, nb, np.float32)
         assert info == 701
+
+
+# several right-hand sides through the one-launch sweeps: both column widths
+# of the kernel, two launches, ragged orders (odd leading dimensions), both
+# triangles; a backward-stable solve has a residual of order n eps
+@pytest.mark.parametrize("nrhs", [2, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("n,nb", [(64, 64), (129, 64), (515, 128), (1000, 256)])
+def test_sweeps_many_rhs(L, n, nb, nrhs):
+    assert L.plasma_set(pb.PlasmaNb, nb) == 0
+    a, b = gen.likelihood(n, nrhs, seed=n + nrhs)
+    for dtype, fn, eps in ((np.float64, L.plasma_dposv, EPS), (np.float32, L.plasma_sposv, SEPS)):
+        for uplo in (LO, UP):
+            f, x = np.asfortranarray(a.astype(dtype)), np.asfortranarray(b.astype(dtype))
+            assert fn(uplo, n, nrhs, f.ctypes.data, n, x.ctypes.data, n) == 0
+            r = np.abs(b - a @ x).sum(axis=1).max()
+            scale = n * np.abs(a).sum(axis=1).max() * np.abs(x).sum(axis=1).max()
+            assert r / scale < TOL * eps
+
+
+# the same sweeps cut to a band, down to a diagonal matrix and up to a band
+# wider than a block
+@pytest.mark.parametrize("kd", [0, 1, 63, 64, 65, 200])
+@pytest.mark.parametrize("nrhs", [1, 3, 20])
+def test_band_sweeps(L, kd, nrhs):
+    n, nb = 700, 128
+    assert L.plasma_set(pb.PlasmaNb, nb) == 0
+    a, lo, up, b = gen.band(n, kd, nrhs, seed=kd)
+    for dtype, fn, eps in ((np.float64, L.plasma_dpbsv, EPS), (np.float32, L.plasma_spbsv, SEPS)):
+        for uplo, ab in ((LO, lo), (UP, up)):
+            f, x = np.asfortranarray(ab.astype(dtype)), np.asfortranarray(b.astype(dtype))
+            assert fn(uplo, n, kd, nrhs, f.ctypes.data, kd + 1, x.ctypes.data, n) == 0
+            r = np.abs(b - a @ x).sum(axis=1).max()
+            scale = n * np.abs(a).sum(axis=1).max() * np.abs(x).sum(axis=1).max()
+            assert r / scale < TOL * eps
+
+
+# FP32 orders that are no multiple of the tile go through padded tiles; the
+# other triangle and the columns past n stay as they were
+@pytest.mark.parametrize("n,nb", [(1, 128), (127, 128), (300, 128), (257, 256), (700, 256)])
+def test_fp32_ragged(L, n, nb):
+    a = gen.likelihood(n, 1, seed=n)[0]
+    for uplo in (LO, UP):
+        info, f = potrf(L, a, nb, np.float32, uplo)
+        assert info == 0
+        tri, other = (np.tril, np.triu) if uplo == LO else (np.triu, np.tril)
+        k = 1 if uplo == LO else -1
+        low = tri(f).astype(np.float64)
+        low = low if uplo == LO else low.T
+        assert np.linalg.norm(low @ low.T - a) <= TOL * n * SEPS * np.linalg.norm(a)
+        np.testing.assert_array_equal(other(f, k), other(a.astype(np.float32), k))
