@@ -40,6 +40,8 @@ typedef struct {
                           update, or 0 for the DMMA/SIMT update            */
     int full;          /* panel copies: every panel (1) or two buffers (0) */
     char *panel[3];    /* rounded copies of panel k (buffer k % 3, or all) */
+    int i8_steps;      /* FP64: steps k < i8_steps update from the panel's
+                          digits on the integer tensor cores               */
     char *wimg;        /* operand image of the diagonal tile for the
                           tensor-core panel solve (plasma_cuda_trsm_tc)    */
     float *scale;      /* row scales of the split half-precision copies    */
@@ -81,6 +83,23 @@ void plasma_pXpotrf_reserve(plasma_context_t *plasma, plasma_enum_t uplo, plasma
         plasma_scratch(plasma, PLASMA_SLOT_MIXED, panel_scratch_bytes(A, tc_mode(A, mode), full));
 }
 
+/* FP64: steps whose trailing matrix has at least 3072 rows update on the
+ * integer tensor cores (cuda/update_i8.cu); below, the digits' own launch on
+ * the critical path and the longer fill of a block cost more than the DMMA
+ * update's arithmetic.  Measured with 256-wide tiles, threshold in tile rows:
+ * n = 8192 7.5 ms (4 to 16 rows), 8.6 (24), 10.9 (never); n = 16384 33.3 (4),
+ * 31.3 (8), 31.2 (16), 32.3 (24), 64 (never). */
+static int i8_steps(plasma_desc_t A, plasma_enum_t uplo)
+{
+    const int rows = 3072 / imax(A.mb, 1);
+    return plasma_cuda_update_i8_ok(A, uplo) && A.mt > rows ? A.mt - rows : 0;
+}
+
+static size_t i8_scratch_bytes(plasma_desc_t A)
+{
+    return 3 * plasma_cuda_panel_i8_bytes(A) + 1024;
+}
+
 static void *panel_buf(walk_t *w, int k)
 {
     return w->full ? w->panel[0] : w->panel[k % 3];
@@ -93,11 +112,16 @@ static void update(walk_t *w, cudaStream_t s, int k, int nlo, int nhi)
                                   panel_buf(w, k), w->full, w->scale, w->sms))
             return;
     }
-    plasma_cuda_update(s, w->st, w->uplo, w->A, k, nlo, nhi, w->sms);
+    if (k < w->i8_steps)
+        plasma_cuda_update_i8(s, w->st, w->A, k, nlo, nhi, panel_buf(w, k), w->sms);
+    else
+        plasma_cuda_update(s, w->st, w->uplo, w->A, k, nlo, nhi, w->sms);
 }
 
 static void round_panel(walk_t *w, cudaStream_t s, int k)
 {
+    if (k < w->i8_steps)
+        plasma_cuda_panel_i8(s, w->st, w->A, k, panel_buf(w, k));
     if (w->mode)
         plasma_cuda_panel_round(s, w->st, w->mode, w->A, k, panel_buf(w, k), w->full,
                                 w->scale);
@@ -259,6 +283,17 @@ void plasma_pXpotrf_arrivals(plasma_context_t *plasma, plasma_enum_t uplo,
     w.panel[0] = w.panel[1] = w.panel[2] = NULL;
     w.wimg = NULL;
     w.scale = NULL;
+    w.i8_steps = i8_steps(A, uplo);
+    if (w.i8_steps > 0) {
+        char *buf = (char *)plasma_scratch(plasma, PLASMA_SLOT_MIXED, i8_scratch_bytes(A));
+        if (buf != NULL) {
+            buf = (char *)(((uintptr_t)buf + 1023) & ~(uintptr_t)1023);
+            for (int i = 0; i < 3; i++)
+                w.panel[i] = buf + (size_t)i * plasma_cuda_panel_i8_bytes(A);
+        } else {
+            w.i8_steps = 0;              /* no memory: the DMMA update */
+        }
+    }
     int tc = tc_mode(A, mode);
     if (plasma_cuda_update_tc_ok(A, uplo)) {
         char *buf = (char *)plasma_scratch(plasma, PLASMA_SLOT_MIXED,

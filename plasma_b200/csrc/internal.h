@@ -41,7 +41,7 @@ typedef struct {
 #define PLASMA_GROUP_STREAMS (PLASMA_NUM_STREAMS - 3)
 #define PLASMA_MAX_GROUPS 32     /* column groups of an arriving matrix */
 #define PLASMA_STAGE_STREAMS 4   /* copies of pageable host blocks       */
-#define PLASMA_SCRATCH_SLOTS 9
+#define PLASMA_SCRATCH_SLOTS 13
 
 /* scratch slots */
 enum {
@@ -52,8 +52,15 @@ enum {
     PLASMA_SLOT_REFINE  = 4,   /* refinement vectors and Krylov basis         */
     PLASMA_SLOT_SYMV    = 5,   /* per-tile partial products of the residual   */
     PLASMA_SLOT_ADJOINT = 6,   /* n x n work matrices of the adjoints         */
-    PLASMA_SLOT_DESC_A  = 7,   /* dsposv's FP64 tile copy of A (kept)         */
-    PLASMA_SLOT_DESC_AS = 8    /* dsposv's FP32 tile copy of A (kept)         */
+    /* the tile copies of the LAPACK-layout drivers' operands, kept between
+     * calls: a cudaMalloc and cudaFree per call cost 0.5 to 2 ms from 2 MB on,
+     * synchronise the device, and now and then took 0.1 to 1 s */
+    PLASMA_SLOT_DESC_A  = 7,   /* A (or L)                                    */
+    PLASMA_SLOT_DESC_AS = 8,   /* the FP32 copy of A (or Lbar)                */
+    PLASMA_SLOT_DESC_B  = 9,   /* right-hand sides                            */
+    PLASMA_SLOT_DESC_X  = 10,  /* solutions (or Xbar)                         */
+    PLASMA_SLOT_DESC_R  = 11,  /* residuals                                   */
+    PLASMA_SLOT_DESC_XS = 12   /* FP32 right-hand sides                       */
 };
 
 typedef struct {
@@ -293,6 +300,14 @@ size_t plasma_cuda_panel_bytes(int tc_mode, plasma_desc_t A, int full);
 int plasma_cuda_update_tc(cudaStream_t s, plasma_devstat_t *st, int tc_mode,
                           plasma_desc_t A, int k, int nlo, int nhi,
                           const void *panel, int full, const float *scale, int num_sms);
+/* FP64 trailing update on the integer tensor cores from the digits of a
+ * panel (cuda/update_i8.cu). */
+int plasma_cuda_update_i8_ok(plasma_desc_t A, plasma_enum_t uplo);
+size_t plasma_cuda_panel_i8_bytes(plasma_desc_t A);
+void plasma_cuda_panel_i8(cudaStream_t s, plasma_devstat_t *st, plasma_desc_t A, int k,
+                          void *panel);
+void plasma_cuda_update_i8(cudaStream_t s, plasma_devstat_t *st, plasma_desc_t A, int k, int nlo,
+                           int nhi, const void *panel, int num_sms);
 /* Row scales of the FP16X3 split: 2 A.gm floats (scales, then reciprocals),
  * from A's diagonal, or from `diag` (A.gm floats) when given. */
 void plasma_cuda_row_scale(cudaStream_t s, plasma_desc_t A, const float *diag, float *scale);
