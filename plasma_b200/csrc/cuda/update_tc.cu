@@ -163,6 +163,23 @@ __device__ __forceinline__ void tc_item(const TcArgs &g, long long w, int &m, in
     m = n + (int)p;
 }
 
+// The whole tiles (the pair kernel's items) one after the other: the search of
+// tc_item once, then a step each.
+struct TileCursor {
+    int m, n, mt;
+    __device__ __forceinline__ void start(const TcArgs &g, long long w)
+    {
+        int si;
+        mt = g.A.mt;
+        tc_item(g, w * (g.A.mb / TC_M), m, n, si);
+    }
+    __device__ __forceinline__ void next()
+    {
+        if (++m == mt) m = ++n;
+    }
+    __device__ __forceinline__ bool last_of_column() const { return m == mt - 1; }
+};
+
 template <int MODE>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 k_update_tc(const __grid_constant__ CUtensorMap opmap,
@@ -382,13 +399,18 @@ k_update_tc(const __grid_constant__ CUtensorMap opmap,
 template <int MODE>
 struct PairGeo {
     using G = Geo<MODE>;
-    // per part: 128 rows of A(m,k) and 128 rows of A(n,k), BK columns each
-    static constexpr int STAGE = G::PARTS * 2 * G::A_BYTES;   // 32 KB, BF16X6 48 KB
+    // RESB: the B operand of a tile column (this CTA's 128 rows of A(n,k), all
+    // 256 columns and parts, 128 KB) stays in shared memory over the items of
+    // that column, and the ring carries A only
+    static constexpr bool RESB = MODE == MODE_FP16X3;
+    // per part: 128 rows of A(m,k) and (in the ring) of A(n,k), BK columns each
+    static constexpr int STAGE = G::PARTS * (RESB ? 1 : 2) * G::A_BYTES;
+    static constexpr int RES = RESB ? (256 / G::BK) * G::PARTS * G::A_BYTES : 0;
     static constexpr int EPI_BUFS = MODE == MODE_FP16X3 || MODE == MODE_BF16X6 ? 1 : 2;
-    static constexpr int STAGES = MODE == MODE_FP16X3 ? 6 : MODE == MODE_BF16X6 ? 4 : 5;
-    static constexpr int SMEM = STAGES * STAGE +
+    static constexpr int STAGES = MODE == MODE_FP16X3 || MODE == MODE_BF16X6 ? 4 : 5;
+    static constexpr int SMEM = STAGES * STAGE + RES +
                                 TC_EPI_WARPS * EPI_BUFS * TC_EPI_BUF_BYTES + 1024;
-    static_assert(SMEM <= 227 * 1024, "shared memory");
+    static_assert(SMEM <= 227 * 1024 - 512, "shared memory");
 };
 
 __device__ __forceinline__ uint32_t cluster_rank()
@@ -505,7 +527,9 @@ k_update_pair(const __grid_constant__ CUtensorMap opmap,
     constexpr int STAGES = P::STAGES;
     constexpr int EPI_BUFS = P::EPI_BUFS;
     constexpr int NB = 256;
+    constexpr bool RESB = P::RESB;
     __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES];
+    __shared__ uint64_t bfull_bar[RESB ? NB / G::BK : 1], bempty_bar;
     __shared__ uint64_t tfull_bar[2], tempty_bar[2];
     __shared__ uint32_t tmem_base_s;
     __shared__ int go_s;
@@ -522,7 +546,9 @@ k_update_pair(const __grid_constant__ CUtensorMap opmap,
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     unsigned char *stage_base =
         (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    // stage: the PARTS parts of 128 rows of A(m,k), then those of A(n,k)
+    // stage: the PARTS parts of 128 rows of A(m,k), then those of A(n,k) unless
+    // these stay in `resb`, one block of the PARTS parts per k-block
+    unsigned char *resb = stage_base + STAGES * P::STAGE;
     constexpr int HALF = G::A_BYTES;
     constexpr int STAGE_BYTES = P::STAGE;
     constexpr int nkb = NB / G::BK;
@@ -537,6 +563,8 @@ k_update_pair(const __grid_constant__ CUtensorMap opmap,
             mbar_init(&tfull_bar[a], 1);
             mbar_init(&tempty_bar[a], 2 * TC_EPI_WARPS);
         }
+        for (int kb = 0; RESB && kb < nkb; kb++) mbar_init(&bfull_bar[kb], 1);
+        mbar_init(&bempty_bar, 1);
         abort_s = 0;
         go_s = !plasma_failed(st);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -560,17 +588,25 @@ k_update_pair(const __grid_constant__ CUtensorMap opmap,
     const uint32_t tmem = tmem_base_s;
     const uint32_t full_lead0 = peer_addr(&full_bar[0], 0);   // leader's full_bar[0]
     const uint32_t tempty_lead0 = peer_addr(&tempty_bar[0], 0);
+    const uint32_t bfull_lead0 = peer_addr(&bfull_bar[0], 0);
 
     if (!go) {
         // status already failed: no work, both CTAs go to the teardown
     } else if (warp == 0 && lane == 0) {
         // ---------------- producer (both CTAs)
-        int it = 0;
-        bool ok = true;
-        for (int j = 0; j < nit && ok; j++) {
-            int m, n, si;
-            tc_item(g, 2 * (first + j) + rank, m, n, si);
+        int it = 0, nb_loads = 0;
+        bool ok = true, load_b = true;
+        TileCursor cur;
+        cur.start(g, first);
+        for (int j = 0; j < nit && ok; j++, load_b = !RESB || cur.last_of_column(), cur.next()) {
+            const int m = cur.m, n = cur.n;
             const int row0 = (int)rank * TC_M;   // this CTA's rows of both operands
+            if (RESB && load_b) {
+                // the products with the column held so far are complete
+                if (nb_loads > 0 &&
+                    !mbar_wait_cluster(&bempty_bar, (nb_loads - 1) & 1, &abort_s)) break;
+                nb_loads++;
+            }
             for (int kb = 0; kb < nkb; kb++, it++) {
                 const int s = it % STAGES;
                 if (it >= STAGES &&
@@ -580,38 +616,52 @@ k_update_pair(const __grid_constant__ CUtensorMap opmap,
                 }
                 unsigned char *sp = stage_base + s * STAGE_BYTES;
                 const uint32_t fb = full_lead0 + (uint32_t)(s * sizeof(uint64_t));
-                if (leader) mbar_expect_tx(&full_bar[s], 2u * (uint32_t)STAGE_BYTES);
+                const uint32_t fbb = RESB ? bfull_lead0 + (uint32_t)(kb * sizeof(uint64_t)) : fb;
+                if (leader) {
+                    mbar_expect_tx(&full_bar[s], 2u * (uint32_t)STAGE_BYTES);
+                    if (RESB && load_b)
+                        mbar_expect_tx(&bfull_bar[kb], 2u * (uint32_t)(G::PARTS * HALF));
+                }
 #pragma unroll
                 for (int p = 0; p < G::PARTS; p++) {
                     const int toff = g.poff + p * g.mt;
+                    unsigned char *sb = RESB ? resb + (kb * G::PARTS + p) * HALF
+                                             : sp + (G::PARTS + p) * HALF;
                     tma_load_4d_pair(sp + p * HALF, &opmap, fb, 0, kb * G::BK,
                                      row0 / G::MNBOX, m + toff);
-                    tma_load_4d_pair(sp + (G::PARTS + p) * HALF, &opmap, fb, 0, kb * G::BK,
-                                     row0 / G::MNBOX, n + toff);
+                    if (load_b)
+                        tma_load_4d_pair(sb, &opmap, fbb, 0, kb * G::BK,
+                                         row0 / G::MNBOX, n + toff);
                 }
             }
         }
     } else if (warp == 1 && lane == 0 && leader) {
         // ---------------- MMA issuer (leader only)
         const uint32_t idesc = instr_desc_pair(MODE);
-        int it = 0;
-        bool ok = true;
-        for (int j = 0; j < nit && ok; j++) {
+        int it = 0, nb_loads = 0;
+        bool ok = true, new_b = RESB;
+        TileCursor cur;
+        cur.start(g, first);
+        for (int j = 0; j < nit && ok; j++, new_b = RESB && cur.last_of_column(), cur.next()) {
             const int a = j & 1;
+            const bool last_b = RESB && cur.last_of_column() && j + 1 < nit;
+            if (new_b) nb_loads++;
             if (j >= 2 && !mbar_wait_cluster(&tempty_bar[a], ((j >> 1) - 1) & 1, &abort_s))
                 break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t acc_t = tmem + (uint32_t)(a * NB);
             for (int kb = 0; kb < nkb; kb++, it++) {
                 const int s = it % STAGES;
-                if (!mbar_wait_cluster(&full_bar[s], (it / STAGES) & 1, &abort_s)) {
+                if (!mbar_wait_cluster(&full_bar[s], (it / STAGES) & 1, &abort_s) ||
+                    (new_b && !mbar_wait_cluster(&bfull_bar[RESB ? kb : 0], (nb_loads - 1) & 1,
+                                                 &abort_s))) {
                     ok = false;
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 unsigned char *sp = stage_base + s * STAGE_BYTES;
                 unsigned char *sa_hi = sp;
-                unsigned char *sb_hi = sp + G::PARTS * HALF;
+                unsigned char *sb_hi = RESB ? resb + kb * G::PARTS * HALF : sp + G::PARTS * HALF;
 #pragma unroll
                 for (int kk = 0; kk < G::BK / G::KI; kk++) {
                     const uint32_t acc_on = (kb | kk) != 0;
@@ -650,23 +700,26 @@ k_update_pair(const __grid_constant__ CUtensorMap opmap,
                 mma_commit_pair(&empty_bar[s]);
             }
             if (ok) mma_commit_pair(&tfull_bar[a]);
+            if (ok && last_b) mma_commit_pair(&bempty_bar);
         }
     } else if (warp >= TC_EPI_WARP0) {
         // ---------------- epilogue (both CTAs): this CTA's 128 rows
         const int e = warp - TC_EPI_WARP0;
         const int q = warp & 3;
         const int half = e / 4;
-        float *stage_epi = (float *)(stage_base + STAGES * STAGE_BYTES) +
+        float *stage_epi = (float *)(stage_base + STAGES * STAGE_BYTES + P::RES) +
                            (size_t)e * EPI_BUFS * (TC_EPI_BUF_BYTES / 4);
         int nchunk = 0;
-        for (int j = 0; j < nit; j++) {
+        TileCursor cur;
+        cur.start(g, first);
+        const int si = (int)rank;
+        for (int j = 0; j < nit; j++, cur.next()) {
             const int a = j & 1;
             const bool ok = __all_sync(0xffffffffu,
                                        mbar_wait_cluster(&tfull_bar[a], (j >> 1) & 1, &abort_s));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            int m, n, si;
-            tc_item(g, 2 * (first + j) + rank, m, n, si);
+            const int m = cur.m, n = cur.n;
             const int tile = (int)(((const char *)plasma_tile_addr(g.A, m, n) -
                                     (const char *)g.A.matrix) / ((size_t)NB * NB * 4));
             const int r0 = si * TC_M + 32 * q;
