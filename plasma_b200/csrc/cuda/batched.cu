@@ -9,25 +9,29 @@
 // the matrices by decreasing size (longest processing time first) and picks
 // the block width NB of each size bucket from a measured table.
 //
-// One CTA per SM, 256 threads, takes the next matrix from an atomic counter
-// until the list is exhausted, so large and small matrices balance across
-// SMs.  Per matrix, for each block column j0:
-//   (a) one warp factors the NB x NB diagonal block, lane r holding row r,
-//       pivots broadcast by shuffles (LAPACK's info on a non-positive or NaN
-//       pivot, and the matrix is abandoned);
-//   (b) every thread solves one row of the panel below, x D^T = a, with D
-//       in shared memory; the panel is kept in shared memory;
-//   (c) the trailing lower triangle is updated, A22 -= P P^T, by warps on
-//       16 x 32 blocks with DMMA (FP64) or the three-product TF32 split
-//       (FP32, FP32-accurate), C read (before the products, so the read
-//       overlaps them) and written in global memory (L2); the first 32
-//       columns first, then warp 0 factors the next diagonal block while
-//       the other warps update the rest.
+// Persistent CTAs of 256 threads (one per SM in FP64, two in FP32, whose
+// panels are half the size) take the next matrix from an atomic counter until
+// the list is exhausted, so large and small matrices balance across SMs.  Per
+// matrix, for each block column j0:
+//   (a) one warp factors the NB x NB diagonal block (blk_factor: eight
+//       columns at a time in registers; LAPACK's info on a non-positive or
+//       NaN pivot, and the matrix is abandoned);
+//   (b) the rows below solve x D^T = a in strips of 16 on the tensor cores
+//       (strip16_solve); the panel is kept in shared memory;
+//   (c) the trailing lower triangle is updated, A22 -= P P^T, with DMMA
+//       (FP64) or the three-product TF32 split (FP32, FP32-accurate), C read
+//       and written in global memory (L2): the next diagonal block first, an
+//       8-column piece per warp, then warp 0 factors it while the other warps
+//       update the rest in tasks of 16 x 32 from a counter.  The other warp
+//       of warp 0's scheduler waits for the factor before it joins: FP64
+//       tensor work on the same scheduler doubles the time of a pivot.
+// 4096 systems, n in [16, 512]: see plasma_dposv_batched below for times.
 // The solve follows in the same CTA while the factor is in L2: forward by
 // block (diagonal block by one warp, the rows below by all threads),
 // backward by block (column dot products by warps, then the diagonal block).
 #include "common.cuh"
 #include "mma.cuh"
+#include "f64_blocks.cuh"
 
 #include <stdlib.h>
 #include <string.h>
@@ -39,13 +43,18 @@ constexpr int NMAX = 512;             // largest matrix of the batched path
 constexpr int NBMAXB = 32;            // largest block width
 
 template <typename T> constexpr int ps_ld() { return NBMAXB + Pad<T>::v; }
-// shared memory: panel [NMAX][ps_ld], two 32 x 33 blocks, a vector of NMAX,
-// 32 reciprocal pivots, the inverse of the diagonal block [32][ps_ld]
+// shared memory: panel [NMAX][ps_ld], three blocks of 32 x 33 (two diagonal
+// blocks in turn and the copy of the one being factored; the adjoints use
+// them with a stride of 33), two sets of 8 x 8 inverses, a vector of NMAX, 32
+// reciprocal pivots
+constexpr int BLK_ELEMS = NBMAXB * (NBMAXB + 1);
 template <typename T> constexpr int batched_smem()
 {
-    return (NMAX * ps_ld<T>() + 2 * NBMAXB * (NBMAXB + 1) + NMAX + NBMAXB +
-            NBMAXB * ps_ld<T>()) * (int)sizeof(T);
+    return (NMAX * ps_ld<T>() + 3 * BLK_ELEMS + 2 * 8 * NBMAXB + NMAX + NBMAXB) * (int)sizeof(T);
 }
+template <typename T> constexpr int batched_ctas() { return sizeof(T) == 4 ? 2 : 1; }
+
+template <int V> struct IntC { static constexpr int value = V; };
 
 enum { OP_POSV = 0, OP_POTRF = 1, OP_POTRS = 2, OP_POTRF_ADJ = 3, OP_POTRS_ADJ = 4 };
 
@@ -66,260 +75,182 @@ struct BatchArgs {
 };
 
 // ------------------------------------------------------------------ factor
-// The diagonal block at j0 (jb x jb, lower), factored by one warp,
-// right-looking: lane r holds row r in registers (every loop unrolled, so the
-// row stays in registers), the block padded to NB x NB with the identity so
-// that no step depends on jb.  Per column c: the pivot comes from lane c by
-// one shuffle, every lane scales its entry and publishes it in Ds (column c
-// at Ds[c * (NBMAXB + 1)]), and the rank-1 update reads the column back as
-// broadcast loads, independent of one another.  (Entries above the diagonal
-// are updated too, from entries above the diagonal only, and never written
-// out.)  The block is read from A, or from Dn (column c at Dn[c * (NBMAXB
-// + 1)], its lower triangle) where the update that produced it left a copy.
-// Writes L to A and Ds, the reciprocal pivots to rdiag and the first bad
-// pivot (LAPACK's info within the block, 0 if none) to *flag.
+// y <- D^-1 y for the right-hand side entries ys[0 .. jb-1] by one warp, with
+// the inverses of D's 8 x 8 diagonal blocks: lane i holds y_i.
 template <typename T, int NB>
-__device__ __forceinline__ void diag_block(T *A, int n, int j0, int jb, T *Ds, T *rdiag,
-                                           int *flag, int lane, const T *Dn = nullptr)
+__device__ __forceinline__ void forward_block(T *ys, int jb, const T *D, const T *W8)
 {
-    constexpr int DL = NBMAXB + 1;
-    T v[NB];
+    const int lane = threadIdx.x & 31;
+    T y = lane < jb ? ys[lane] : T(0);
 #pragma unroll
-    for (int c = 0; c < NB; c++)
-        v[c] = (lane < jb && c < jb)
-                   ? (lane >= c ? (Dn != nullptr ? Dn[c * DL + lane]
-                                                 : A[(size_t)(j0 + c) * n + j0 + lane])
-                                : T(0))
-                   : (lane == c ? T(1) : T(0));
-    int bad = 0;
-    T myrd = T(1);
+    for (int q = 0; q < NB / 8; q++) {
+        const int i = lane - 8 * q;
+        T x[8], nv = T(0);
 #pragma unroll
-    for (int c = 0; c < NB; c++) {
-        const T d = __shfl_sync(0xffffffffu, v[c], c);
-        const bool ok = d > T(0);
-        if (!ok && bad == 0 && c < jb) bad = c + 1;
-        // one reciprocal square root per pivot: 1/sqrt(d), sqrt(d) = d/sqrt(d)
-        const T rd = ok ? rsqrt(d) : T(1);
-        if (lane == c) {
-            myrd = rd;
-            v[c] = ok ? d * rd : T(1);
-        } else {
-            v[c] *= rd;
+        for (int k = 0; k < 8; k++) x[k] = __shfl_sync(0xffffffffu, y, 8 * q + k);
+#pragma unroll
+        for (int k = 0; k < 8; k++) nv = fma(W8[(8 * q + k) * 8 + (i & 7)], x[k], nv);
+        if (i >= 0 && i < 8) y = nv;
+#pragma unroll
+        for (int k = 0; k < 8; k++) x[k] = __shfl_sync(0xffffffffu, y, 8 * q + k);
+        if (i >= 8) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) y = fma(-D[pd_at(8 * q + k, lane)], x[k], y);
         }
-        Ds[c * DL + lane] = v[c];
-        __syncwarp();
-#pragma unroll
-        for (int c2 = c + 1; c2 < NB; c2++) v[c2] -= v[c] * Ds[c * DL + c2];
     }
-    if (lane < jb) {
-#pragma unroll
-        for (int c = 0; c < NB; c++)
-            if (c < jb && lane >= c) A[(size_t)(j0 + c) * n + j0 + lane] = v[c];
-        rdiag[lane] = myrd;
-    }
-    if (lane == 0) *flag = bad;
+    if (lane < jb) ys[lane] = y;
 }
 
-// The inverse of the factored diagonal block, Li = L^-1 (row i at
-// Li[i * ps_ld]), by one warp: lane j solves L y = e_j column by column
-// (y_k scaled by its reciprocal pivot, then y_i -= L_ik y_k below it, the
-// column of L read from Ds as broadcast loads); every loop unrolled, y kept
-// in registers until the end.  Lanes at or beyond NB form zero columns,
-// never read.
-template <typename T, int NB>
-__device__ __forceinline__ void diag_inverse(const T *Ds, const T *rdiag, T *Li, int lane)
-{
-    constexpr int DL = NBMAXB + 1, LLD = ps_ld<T>();
-    T y[NB];
-#pragma unroll
-    for (int i = 0; i < NB; i++) y[i] = (i == lane) ? T(1) : T(0);
-#pragma unroll
-    for (int k = 0; k < NB; k++) {
-        y[k] *= rdiag[k];
-#pragma unroll
-        for (int i = k + 1; i < NB; i++) y[i] -= Ds[k * DL + i] * y[k];
-    }
-#pragma unroll
-    for (int i = 0; i < NB; i++) Li[i * LLD + lane] = y[i];
-}
-
-// Per block column j0: (b) the panel below the diagonal block, X D^T = A21,
-// as the tensor-core product X = A21 D^-T with the inverse formed right
-// after the diagonal block was factored (kept in shared memory); (c1) the
-// trailing update of the first 32 columns of A22 (they hold the next
-// diagonal block and the next panel); then warp 0 factors the next diagonal
-// block and inverts it (a) while the other warps finish the trailing update
-// (c2), so the single-warp chains of (a) overlap the tensor work.  The trailing update runs on 16 x 32 blocks of
-// the lower triangle with DMMA (FP64) or the three-product TF32 split
-// (FP32); a warp's block of C is read into registers before its products,
-// so the L2 latency of the read overlaps them.  With ys (posv: the
-// right-hand side in shared memory) the forward sweep L y = b runs along:
-// y_j by warp 0 from the diagonal block while it is in shared memory, the
-// rows below from the panel, so the solve afterwards is the backward sweep
-// alone.
+// See the header.  With ys (posv: the right-hand side in shared memory) the
+// forward sweep L y = b runs along, y_j from the diagonal block by the last
+// warp and the rows below from the panel, so the solve afterwards is the
+// backward sweep alone.  task: a counter in shared memory.
 template <typename T, int SPLIT, int NB>
-__device__ int factor_one(T *A, int n, T *Ps, T *Ds, T *rdiag, int *flag, T *ys, T *Li,
-                          T *Dn)
+__device__ int factor_one(T *A, int n, T *Ps, T *D0, T *D1, T *Dn, T *W8, T *rdiag, int *flag,
+                          int *task, T *ys)
 {
     constexpr int PLD = ps_ld<T>();
+    constexpr int WARPS = BT / 32;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
-    if (warp == 0) {
-        diag_block<T, NB>(A, n, 0, min(NB, n), Ds, rdiag, flag, lane);
-        __syncwarp();
-        diag_inverse<T, NB>(Ds, rdiag, Li, lane);
+    // warp 0: the block at D, of which Dn holds a copy
+    auto factor = [&](T *D, T *W) {
+        int bad = 0;
+        if (!__all_sync(0xffffffffu, blk_factor<T, SPLIT, NB>(D, W)))
+            bad = blk_factor_any<T, NB>(D, W, Dn, rdiag);
+        if (lane == 0) *flag = bad;
+    };
+    // the first diagonal block, padded with the identity
+    for (int e = tid; e < NB * 32; e += BT) {
+        const int r = e % 32, c = e / 32;
+        const T v = r < min(NB, n) && c < n ? (r >= c ? A[(size_t)c * n + r] : T(0))
+                                            : (r == c ? T(1) : T(0));
+        D0[pd_at(c, r)] = v;
+        Dn[pd_at(c, r)] = v;
     }
     __syncthreads();
-    for (int j0 = 0; j0 < n; j0 += NB) {
+    if (warp == 0) factor(D0, W8);
+    __syncthreads();
+    for (int j0 = 0, cur = 0; j0 < n; j0 += NB, cur ^= 1) {
         const int jb = min(NB, n - j0);
         const int m2 = n - j0 - jb;
         const int bad = *flag;
         if (bad) return j0 + bad;
-        // (b) the panel below, X = A21 L_jj^-T: a tensor-core product with
-        // the inverse, 16-row blocks taken by the warps in turn (a panel
-        // exists only below a full diagonal block, jb = NB), X written to A
-        // and to Ps
+        const T *D = cur ? D1 : D0;
+        const T *W = W8 + cur * 8 * NBMAXB;
+        T *Dnext = cur ? D0 : D1, *Wnext = W8 + (cur ^ 1) * 8 * NBMAXB;
+        if (tid == 0) *task = 0;
+        if (ys != nullptr && warp == WARPS - 1) forward_block<T, NB>(ys + j0, jb, D, W);
+        for (int e = tid; e < jb * 32; e += BT) {
+            const int r = e % 32, c = e / 32;
+            if (r >= c && r < jb) A[(size_t)(j0 + c) * n + j0 + r] = D[pd_at(c, r)];
+        }
+        // (b) the panel below (there is one only below a full diagonal
+        // block), to A and to Ps
         {
             T *A21 = A + (size_t)j0 * n + (j0 + jb);
-            for (int r0 = warp * 16; r0 < m2; r0 += BT / 2) {
-                const int ra = r0 + g;
-                T af[NB / 8][4];
+            for (int r0 = warp * 16; r0 < m2; r0 += 16 * WARPS) {
+                T y[NB / 8][4];
 #pragma unroll
-                for (int k8 = 0; k8 < NB; k8 += 8) {
-                    const T *c0 = A21 + (size_t)(k8 + t) * n, *c4 = c0 + (size_t)4 * n;
-                    af[k8 / 8][0] = ra < m2 ? c0[ra] : T(0);
-                    af[k8 / 8][1] = ra + 8 < m2 ? c0[ra + 8] : T(0);
-                    af[k8 / 8][2] = ra < m2 ? c4[ra] : T(0);
-                    af[k8 / 8][3] = ra + 8 < m2 ? c4[ra + 8] : T(0);
-                }
-                T acc[NB / 8][4];
+                for (int q = 0; q < NB / 8; q++)
 #pragma unroll
-                for (int ni = 0; ni < NB / 8; ni++)
-#pragma unroll
-                    for (int e = 0; e < 4; e++) acc[ni][e] = T(0);
-#pragma unroll
-                for (int k8 = 0; k8 < NB; k8 += 8)
-#pragma unroll
-                    for (int ni = 0; ni < NB / 8; ni++) {
-                        T bf[2];
-                        bf[0] = Li[(ni * 8 + g) * PLD + k8 + t];
-                        bf[1] = Li[(ni * 8 + g) * PLD + k8 + t + 4];
-                        mma8<SPLIT>(acc[ni], af[k8 / 8], bf);
+                    for (int e = 0; e < 4; e++) {
+                        const int r = r0 + g + 8 * (e >> 1), c = 8 * q + 2 * t + (e & 1);
+                        y[q][e] = r < m2 ? A21[(size_t)c * n + r] : T(0);
                     }
+                strip16_solve<T, SPLIT, NB>(y, D, W);
 #pragma unroll
-                for (int ni = 0; ni < NB / 8; ni++)
+                for (int q = 0; q < NB / 8; q++)
 #pragma unroll
-                    for (int h = 0; h < 2; h++)
-#pragma unroll
-                        for (int e = 0; e < 2; e++) {
-                            const int r = ra + 8 * h, c = ni * 8 + 2 * t + e;
-                            if (r < m2) {
-                                A21[(size_t)c * n + r] = acc[ni][2 * h + e];
-                                Ps[r * PLD + c] = acc[ni][2 * h + e];
-                            }
+                    for (int e = 0; e < 4; e++) {
+                        const int r = r0 + g + 8 * (e >> 1), c = 8 * q + 2 * t + (e & 1);
+                        if (r < m2) {
+                            A21[(size_t)c * n + r] = y[q][e];
+                            Ps[r * PLD + c] = y[q][e];
                         }
+                    }
             }
         }
         __syncthreads();
-        // forward sweep, diagonal block: y_j = L_jj^-1 y_j (warp 0)
-        if (ys != nullptr && warp == 0) {
-            T y = lane < jb ? ys[j0 + lane] : T(0);
-            for (int c = 0; c < jb; c++) {
-                if (lane == c) y = y * rdiag[c];
-                const T yc = __shfl_sync(0xffffffffu, y, c);
-                if (lane > c && lane < jb) y -= Ds[c * (NBMAXB + 1) + lane] * yc;
-            }
-            if (lane < jb) ys[j0 + lane] = y;
-        }
-        if (m2 == 0) {
-            __syncthreads();
-            break;
-        }
-        const int nrb = (m2 + 15) / 16, ncb = (m2 + 31) / 32;
+        if (m2 == 0) break;
         T *C = A + (size_t)(j0 + jb) * n + (j0 + jb);   // A22(0,0)
-        // blocks (bi, bj) of the lower triangle, bi >= 2 bj, numbered column
-        // by column; the warps in [w0, w0 + nw) take the blocks of the block
-        // columns [bj0, bj1)
-        auto trail = [&](int bj0, int bj1, int w0, int nw) {
-            if (warp < w0 || warp >= w0 + nw) return;
-            int first = 0, count = 0;
-            for (int bj = 0; bj < bj1 && bj < ncb; bj++) {
-                const int nb_j = max(0, nrb - 2 * bj);
-                if (bj < bj0) first += nb_j;
-                else count += nb_j;
-            }
-            for (int pp = warp - w0; pp < count; pp += nw) {
-                int bj = 0, q = first + pp;
-                while (q >= nrb - 2 * bj) { q -= nrb - 2 * bj; bj++; }
-                const int r0 = (2 * bj + q) * 16, c0 = bj * 32;
-                T cv[4][4], acc[4][4];
+        // C(r0 .. r0+15, c0 .. c0+8 NF-1) - P P^T, handed to put(r, c, value)
+        auto block = [&](int r0, int c0, auto nf, auto put) {
+            constexpr int NF = decltype(nf)::value;
+            T cv[NF][4], acc[NF][4];
+            const int ra = r0 + g;
 #pragma unroll
-                for (int ni = 0; ni < 4; ni++)
+            for (int f = 0; f < NF; f++)
 #pragma unroll
-                    for (int h = 0; h < 2; h++)
-#pragma unroll
-                        for (int e = 0; e < 2; e++) {
-                            const int r = r0 + g + 8 * h, c = c0 + ni * 8 + 2 * t + e;
-                            cv[ni][2 * h + e] = (r < m2 && c < m2 && r >= c)
-                                                    ? C[(size_t)c * n + r] : T(0);
-                            acc[ni][2 * h + e] = T(0);
-                        }
-#pragma unroll
-                for (int k8 = 0; k8 < NB; k8 += 8) {
-                    T bf[4][2];
-#pragma unroll
-                    for (int ni = 0; ni < 4; ni++) {
-                        const int cr = c0 + ni * 8 + g;
-                        bf[ni][0] = cr < m2 ? Ps[cr * PLD + k8 + t] : T(0);
-                        bf[ni][1] = cr < m2 ? Ps[cr * PLD + k8 + t + 4] : T(0);
-                    }
-                    const int ra = r0 + g;
-                    T af[4];
-                    af[0] = ra < m2 ? Ps[ra * PLD + k8 + t] : T(0);
-                    af[1] = ra + 8 < m2 ? Ps[(ra + 8) * PLD + k8 + t] : T(0);
-                    af[2] = ra < m2 ? Ps[ra * PLD + k8 + t + 4] : T(0);
-                    af[3] = ra + 8 < m2 ? Ps[(ra + 8) * PLD + k8 + t + 4] : T(0);
-#pragma unroll
-                    for (int ni = 0; ni < 4; ni++) mma8<SPLIT>(acc[ni], af, bf[ni]);
+                for (int e = 0; e < 4; e++) {
+                    const int r = ra + 8 * (e >> 1), c = c0 + 8 * f + 2 * t + (e & 1);
+                    cv[f][e] = r < m2 && c < m2 && r >= c ? C[(size_t)c * n + r] : T(0);
+                    acc[f][e] = T(0);
                 }
 #pragma unroll
-                for (int ni = 0; ni < 4; ni++)
+            for (int k8 = 0; k8 < NB; k8 += 8) {
+                T bf[NF][2], af[4];
 #pragma unroll
-                    for (int h = 0; h < 2; h++)
+                for (int f = 0; f < NF; f++) {
+                    const int cr = c0 + 8 * f + g;
+                    bf[f][0] = cr < m2 ? Ps[cr * PLD + k8 + t] : T(0);
+                    bf[f][1] = cr < m2 ? Ps[cr * PLD + k8 + t + 4] : T(0);
+                }
+                af[0] = ra < m2 ? Ps[ra * PLD + k8 + t] : T(0);
+                af[1] = ra + 8 < m2 ? Ps[(ra + 8) * PLD + k8 + t] : T(0);
+                af[2] = ra < m2 ? Ps[ra * PLD + k8 + t + 4] : T(0);
+                af[3] = ra + 8 < m2 ? Ps[(ra + 8) * PLD + k8 + t + 4] : T(0);
 #pragma unroll
-                        for (int e = 0; e < 2; e++) {
-                            const int r = r0 + g + 8 * h, c = c0 + ni * 8 + 2 * t + e;
-                            if (r < m2 && c < m2 && r >= c) {
-                                const T val = cv[ni][2 * h + e] - acc[ni][2 * h + e];
-                                C[(size_t)c * n + r] = val;
-                                // the next diagonal block, for (a) to read
-                                if (r < NBMAXB) Dn[c * (NBMAXB + 1) + r] = val;
-                            }
-                        }
+                for (int f = 0; f < NF; f++) mma8<SPLIT>(acc[f], af, bf[f]);
             }
+#pragma unroll
+            for (int f = 0; f < NF; f++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int r = ra + 8 * (e >> 1), c = c0 + 8 * f + 2 * t + (e & 1);
+                    put(r, c, cv[f][e] - acc[f][e]);
+                }
         };
-        // (c1) the first 32 columns of A22, all warps
-        trail(0, 1, 0, BT / 32);
+        // (c) the next diagonal block, an 8-column piece per warp, padded
+        {
+            const int jn = min(NB, m2);
+            if (warp < NB / 16 * (NB / 8))
+                block(16 * (warp / (NB / 8)), 8 * (warp % (NB / 8)), IntC<1>{},
+                      [&](int r, int c, T v) {
+                          v = r < jn && c < jn ? (r >= c ? v : T(0)) : (r == c ? T(1) : T(0));
+                          Dnext[pd_at(c, r)] = v;
+                          Dn[pd_at(c, r)] = v;
+                      });
+        }
         __syncthreads();
-        // (a) the next diagonal block by warp 0, (c2) the rest by the others
-        // (after the forward sweep's rows below: y_below -= P y_j)
         if (warp == 0) {
-            diag_block<T, NB>(A, n, j0 + jb, min(NB, m2), Ds, rdiag, flag, lane, Dn);
-            __syncwarp();
-            diag_inverse<T, NB>(Ds, rdiag, Li, lane);
-        } else {
-            if (ys != nullptr) {
-                for (int r = tid - 32; r < m2; r += BT - 32) {
-                    T s0 = T(0), s1 = T(0);
+            factor(Dnext, Wnext);
+        } else if (ys != nullptr) {
+            // y_below -= P y_j
+            for (int r = tid - 32; r < m2; r += BT - 32) {
+                T s0 = T(0), s1 = T(0);
 #pragma unroll
-                    for (int c = 0; c < NB; c += 2) {
-                        s0 += Ps[r * PLD + c] * ys[j0 + c];
-                        s1 += Ps[r * PLD + c + 1] * ys[j0 + c + 1];
-                    }
-                    ys[j0 + jb + r] -= s0 + s1;
+                for (int c = 0; c < NB; c += 2) {
+                    s0 += Ps[r * PLD + c] * ys[j0 + c];
+                    s1 += Ps[r * PLD + c + 1] * ys[j0 + c + 1];
                 }
+                ys[j0 + jb + r] -= s0 + s1;
             }
-            trail(1, ncb, 1, BT / 32 - 1);
+        }
+        if ((warp & 3) == 0) asm volatile("bar.sync 1, %0;" :: "n"(BT / 4) : "memory");
+        // the rest of the lower triangle: blocks (bi, bj) of 16 x 32, bi >=
+        // 2 bj, column by column, without the NB / 16 of the diagonal block
+        const int nrb = (m2 + 15) / 16;
+        for (;;) {
+            int q = 0;
+            if (lane == 0) q = atomicAdd(task, 1);
+            q = __shfl_sync(0xffffffffu, q, 0) + NB / 16;
+            int bj = 0;
+            while (2 * bj < nrb && q >= nrb - 2 * bj) { q -= nrb - 2 * bj; bj++; }
+            if (2 * bj >= nrb) break;
+            block(16 * (2 * bj + q), 32 * bj, IntC<4>{}, [&](int r, int c, T v) {
+                if (r < m2 && c < m2 && r >= c) C[(size_t)c * n + r] = v;
+            });
         }
         __syncthreads();
     }
@@ -372,12 +303,33 @@ __device__ void solve_one(const T *A, int n, T *b, T *Ys, T *Db, T *Dr, bool for
             Db[c * DLD + r] = (r < jb && c < jb && r >= c) ? A[(size_t)(j0 + c) * n + j0 + r] : T(0);
         }
         if (tid < jb) Dr[tid] = T(1) / A[(size_t)(j0 + tid) * n + j0 + tid];
-        for (int c = warp; c < jb; c += BT / 32) {
-            T s = T(0);
-            for (int i = j0 + jb + lane; i < n; i += 32) s += A[(size_t)(j0 + c) * n + i] * Ys[i];
+        // a warp takes its four columns of the block at once (their loads
+        // overlap)
+        {
+            constexpr int NC = NB / (BT / 32);
+            T s[NC];
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-            if (lane == 0) Ys[j0 + c] -= s;
+            for (int q = 0; q < NC; q++) s[q] = T(0);
+#pragma unroll 4
+            for (int i = j0 + jb + lane; i < n; i += 32) {
+                const T y = Ys[i];
+#pragma unroll
+                for (int q = 0; q < NC; q++) {
+                    const int c = warp + q * (BT / 32);
+                    if (c < jb) s[q] += A[(size_t)(j0 + c) * n + i] * y;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < NC; q++)
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1)
+                    s[q] += __shfl_xor_sync(0xffffffffu, s[q], off);
+            if (lane < NC && warp + lane * (BT / 32) < jb) {
+                T v = s[0];
+#pragma unroll
+                for (int q = 1; q < NC; q++) v = lane == q ? s[q] : v;
+                Ys[j0 + warp + lane * (BT / 32)] -= v;
+            }
         }
         __syncthreads();
         if (warp == 0) {
@@ -435,60 +387,148 @@ __device__ void solve_adjoint_one(const T *Lf, int n, const T *x, T *xbar, T *Lb
 // block; bars the same blocks of Lbar).  The result Abar is lower triangular
 // and the symmetric cotangent is (Abar + Abar^T)/2 with Abar's own diagonal,
 // written into both triangles of Lbar at the end.
+// Long sums leave the tensor cores every 32 terms (add_up): what these add to
+// an FP32 accumulator is truncated, and the bias would grow with the length.
 template <typename T>
-__device__ void factor_adjoint_one(const T *Lf, int n, T *Lb, T *Cs, T *Ds, T *Dbs)
+__device__ __forceinline__ void add_up(T (&sum)[4], T (&acc)[4])
+{
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        sum[e] += acc[e];
+        acc[e] = T(0);
+    }
+}
+
+// The products (the four block updates) run on the tensor cores (mma8): a
+// thread per output entry made them 90% of the adjoint's time.  Warp 0 runs
+// the unblocked reverse beside the update of Bbar by the others.
+template <typename T, int SPLIT>
+__device__ void factor_adjoint_one(const T *Lf, int n, T *Lb, T *Cs, T *Ds, T *Dbs, T *Dp, T *W8)
 {
     constexpr int NB = 32, CLD = NB + 1;
+    constexpr int WARPS = BT / 32;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t = lane & 3;
     for (int k = n; k > 0; k -= NB) {
-        const int j = max(0, k - NB), jb = k - j, m2 = n - k;
+        const int j = max(0, k - NB), jb = k - j, m2 = n - k;   // j > 0 only if jb = NB
         for (int e = tid; e < NB * NB; e += BT) {
             const int r = e % NB, c = e / NB;
             const bool in = r < jb && c < jb && r >= c;
-            Ds[c * CLD + r] = in ? Lf[(size_t)(j + c) * n + j + r] : T(0);
+            const T v = in ? Lf[(size_t)(j + c) * n + j + r] : T(0);
+            Ds[c * CLD + r] = v;
+            Dp[pd_at(c, r)] = r >= jb || c >= jb ? (r == c ? T(1) : T(0)) : v;
             Dbs[c * CLD + r] = in ? Lb[(size_t)(j + c) * n + j + r] : T(0);
         }
         __syncthreads();
-        // (1) Cbar <- Cbar D^-1, one thread per row
-        for (int r = tid; r < m2; r += BT) {
-            T x[NB];
+        // (1) Cbar <- Cbar D^-1 in strips of 16 rows, with the inverses of D's
+        // 8 x 8 diagonal blocks
+        if (m2 > 0) {
+            if (warp == 0) {
+                const int o = lane & ~7;
+                T w[8];
+                inv8_column(lane & 7, [&](int i, int q) { return Dp[pd_at(o + q, o + i)]; },
+                            [&](int i) { return T(1) / Dp[pd_at(o + i, o + i)]; }, w);
 #pragma unroll
-            for (int c = 0; c < NB; c++) x[c] = c < jb ? Lb[(size_t)(j + c) * n + k + r] : T(0);
+                for (int i = 0; i < 8; i++) W8[lane * 8 + i] = w[i];
+            }
+            __syncthreads();
+            for (int r0 = 16 * warp; r0 < m2; r0 += 16 * WARPS) {
+                T y[NB / 8][4];
 #pragma unroll
-            for (int c = NB - 1; c >= 0; c--) {
-                if (c < jb) {
-                    T s = x[c];
+                for (int q = 0; q < NB / 8; q++)
 #pragma unroll
-                    for (int c2 = c + 1; c2 < NB; c2++)
-                        if (c2 < jb) s -= x[c2] * Ds[c * CLD + c2];
-                    x[c] = s / Ds[c * CLD + c];
+                    for (int e = 0; e < 4; e++) {
+                        const int r = r0 + g + 8 * (e >> 1), c = 8 * q + 2 * t + (e & 1);
+                        y[q][e] = r < m2 && c < jb ? Lb[(size_t)(j + c) * n + k + r] : T(0);
+                    }
+#pragma unroll
+                for (int q = NB / 8 - 1; q >= 0; q--) {
+                    T x[4];
+                    strip16_product<T, SPLIT>(x, y[q], W8[(8 * q + g) * 8 + 2 * t],
+                                              W8[(8 * q + g) * 8 + 2 * t + 1]);
+#pragma unroll
+                    for (int f = 0; f < q; f++)
+                        strip16_subtract<T, SPLIT>(y[f], x, Dp[pd_at(8 * f + g, 8 * q + 2 * t)],
+                                                   Dp[pd_at(8 * f + g, 8 * q + 2 * t + 1)]);
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const int r = r0 + g + 8 * (e >> 1), c = 8 * q + 2 * t + (e & 1);
+                        if (r < m2) {
+                            Cs[r * CLD + c] = x[e];
+                            if (c < jb) Lb[(size_t)(j + c) * n + k + r] = x[e];
+                        }
+                    }
                 }
             }
+            __syncthreads();
+            // (3) Dbar -= tril(Cbar^T C): a 16 x 8 piece per warp
+            {
+                const int i0 = 16 * (warp >> 2), c0 = 8 * (warp & 3);
+                const T *Cc = Lf + (size_t)(j + min(c0 + g, jb - 1)) * n + k;
+                T acc[4] = {T(0), T(0), T(0), T(0)}, sum[4] = {T(0), T(0), T(0), T(0)};
+#pragma unroll 4
+                for (int r = 0; r < m2; r += 8) {
+                    const int ra = r + t, rb = ra + 4;
+                    const T af[4] = {ra < m2 ? Cs[ra * CLD + i0 + g] : T(0),
+                                     ra < m2 ? Cs[ra * CLD + i0 + g + 8] : T(0),
+                                     rb < m2 ? Cs[rb * CLD + i0 + g] : T(0),
+                                     rb < m2 ? Cs[rb * CLD + i0 + g + 8] : T(0)};
+                    const T bf[2] = {ra < m2 ? Cc[ra] : T(0), rb < m2 ? Cc[rb] : T(0)};
+                    mma8<SPLIT>(acc, af, bf);
+                    if ((r & 24) == 24) add_up<T>(sum, acc);
+                }
+                add_up<T>(sum, acc);
 #pragma unroll
-            for (int c = 0; c < NB; c++) {
-                if (c < jb) Lb[(size_t)(j + c) * n + k + r] = x[c];
-                Cs[r * CLD + c] = x[c];
+                for (int e = 0; e < 4; e++) {
+                    const int i = i0 + g + 8 * (e >> 1), c = c0 + 2 * t + (e & 1);
+                    if (i >= c && i < jb && c < jb) Dbs[c * CLD + i] -= sum[e];
+                }
+            }
+            __syncthreads();
+        }
+        // (2) Bbar -= Cbar R (rows k.., columns 0..j): per task 32 columns,
+        // whose R stays in registers, and 64 rows; the warps beside warp 0
+        if (warp > 0 && j > 0 && m2 > 0) {
+            const int ncb = (j + 31) / 32, nrg = (m2 + 63) / 64;
+            for (int task = warp - 1; task < ncb * nrg; task += WARPS - 1) {
+                const int c0 = 32 * (task % ncb), rg = 64 * (task / ncb);
+                T bf[4][NB / 8][2];
+#pragma unroll
+                for (int f = 0; f < 4; f++) {
+                    const int col = c0 + 8 * f + g;
+                    const T *Rc = Lf + (size_t)col * n + j;
+#pragma unroll
+                    for (int k8 = 0; k8 < NB; k8 += 8) {
+                        bf[f][k8 / 8][0] = col < j ? Rc[k8 + t] : T(0);
+                        bf[f][k8 / 8][1] = col < j ? Rc[k8 + t + 4] : T(0);
+                    }
+                }
+                for (int r0 = rg; r0 < min(m2, rg + 64); r0 += 16) {
+                    const int ra = r0 + g;
+                    T acc[4][4];
+#pragma unroll
+                    for (int f = 0; f < 4; f++)
+#pragma unroll
+                        for (int e = 0; e < 4; e++) acc[f][e] = T(0);
+#pragma unroll
+                    for (int k8 = 0; k8 < NB; k8 += 8) {
+                        const T af[4] = {ra < m2 ? Cs[ra * CLD + k8 + t] : T(0),
+                                         ra + 8 < m2 ? Cs[(ra + 8) * CLD + k8 + t] : T(0),
+                                         ra < m2 ? Cs[ra * CLD + k8 + t + 4] : T(0),
+                                         ra + 8 < m2 ? Cs[(ra + 8) * CLD + k8 + t + 4] : T(0)};
+#pragma unroll
+                        for (int f = 0; f < 4; f++) mma8<SPLIT>(acc[f], af, bf[f][k8 / 8]);
+                    }
+#pragma unroll
+                    for (int f = 0; f < 4; f++)
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            const int r = ra + 8 * (e >> 1), col = c0 + 8 * f + 2 * t + (e & 1);
+                            if (r < m2 && col < j) Lb[(size_t)col * n + k + r] -= acc[f][e];
+                        }
+                }
             }
         }
-        __syncthreads();
-        // (2) Bbar -= Cbar R   (rows k.., columns 0..j)
-        for (int e = tid; e < m2 * j; e += BT) {
-            const int r = e % m2, col = e / m2;
-            const T *Rc = Lf + (size_t)col * n + j;
-            T s = T(0);
-            for (int c = 0; c < jb; c++) s += Cs[r * CLD + c] * Rc[c];
-            Lb[(size_t)col * n + k + r] -= s;
-        }
-        // (3) Dbar -= tril(Cbar^T C)
-        for (int e = tid; e < jb * jb; e += BT) {
-            const int i = e % jb, c = e / jb;
-            if (i < c) continue;
-            const T *Cc = Lf + (size_t)(j + c) * n + k;
-            T s = T(0);
-            for (int r = 0; r < m2; r++) s += Cs[r * CLD + i] * Cc[r];
-            Dbs[c * CLD + i] -= s;
-        }
-        __syncthreads();
         // (4) unblocked reverse on the diagonal block, one warp, lane = column
         if (warp == 0) {
             for (int jj = jb - 1; jj >= 0; jj--) {
@@ -513,16 +553,81 @@ __device__ void factor_adjoint_one(const T *Lf, int n, T *Lb, T *Cs, T *Ds, T *D
             }
         }
         __syncthreads();
-        // (5) Rbar -= Cbar^T B + (Dbar + Dbar^T) R   (rows j..k, columns 0..j)
-        for (int e = tid; e < jb * j; e += BT) {
-            const int i = e % jb, col = e / jb;
-            const T *Bc = Lf + (size_t)col * n + k;
-            const T *Rc = Lf + (size_t)col * n + j;
-            T s = T(0);
-            for (int r = 0; r < m2; r++) s += Cs[r * CLD + i] * Bc[r];
-            for (int c = 0; c < jb; c++)
-                s += (Dbs[c * CLD + i] + Dbs[i * CLD + c]) * Rc[c];
-            Lb[(size_t)col * n + j + i] -= s;
+        // (5) Rbar -= Cbar^T B + (Dbar + Dbar^T) R (rows j..k, columns 0..j),
+        // 16 columns per task
+        for (int c0 = 16 * warp; c0 < j; c0 += 16 * WARPS) {
+            T acc[2][2][4], sum[2][2][4];
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+                for (int f = 0; f < 2; f++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) acc[h][f][e] = sum[h][f][e] = T(0);
+            auto add_all = [&]() {
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int f = 0; f < 2; f++) add_up<T>(sum[h][f], acc[h][f]);
+            };
+            const T *Lc[2];
+            bool cv[2];
+#pragma unroll
+            for (int f = 0; f < 2; f++) {
+                cv[f] = c0 + 8 * f + g < j;
+                Lc[f] = Lf + (size_t)min(c0 + 8 * f + g, j - 1) * n;
+            }
+#pragma unroll
+            for (int k8 = 0; k8 < NB; k8 += 8) {
+                T bf[2][2];
+#pragma unroll
+                for (int f = 0; f < 2; f++) {
+                    bf[f][0] = cv[f] ? Lc[f][j + k8 + t] : T(0);
+                    bf[f][1] = cv[f] ? Lc[f][j + k8 + t + 4] : T(0);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    T af[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const int i = 16 * h + g + 8 * (e & 1), c = k8 + t + 4 * (e >> 1);
+                        af[e] = Dbs[c * CLD + i] + Dbs[i * CLD + c];
+                    }
+#pragma unroll
+                    for (int f = 0; f < 2; f++) mma8<SPLIT>(acc[h][f], af, bf[f]);
+                }
+            }
+            add_all();
+#pragma unroll 2
+            for (int r = 0; r < m2; r += 8) {
+                const int ra = r + t, rb = ra + 4;
+                T bf[2][2];
+#pragma unroll
+                for (int f = 0; f < 2; f++) {
+                    bf[f][0] = cv[f] && ra < m2 ? Lc[f][k + ra] : T(0);
+                    bf[f][1] = cv[f] && rb < m2 ? Lc[f][k + rb] : T(0);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int i = 16 * h + g;
+                    const T af[4] = {ra < m2 ? Cs[ra * CLD + i] : T(0),
+                                     ra < m2 ? Cs[ra * CLD + i + 8] : T(0),
+                                     rb < m2 ? Cs[rb * CLD + i] : T(0),
+                                     rb < m2 ? Cs[rb * CLD + i + 8] : T(0)};
+#pragma unroll
+                    for (int f = 0; f < 2; f++) mma8<SPLIT>(acc[h][f], af, bf[f]);
+                }
+                if ((r & 24) == 24) add_all();
+            }
+            add_all();
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+                for (int f = 0; f < 2; f++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const int i = 16 * h + g + 8 * (e >> 1), col = c0 + 8 * f + 2 * t + (e & 1);
+                        if (col < j) Lb[(size_t)col * n + j + i] -= sum[h][f][e];
+                    }
         }
         for (int e = tid; e < jb * jb; e += BT) {
             const int r = e % jb, c = e / jb;
@@ -544,17 +649,18 @@ __device__ void factor_adjoint_one(const T *Lf, int n, T *Lb, T *Cs, T *Ds, T *D
 
 // ------------------------------------------------------------------ kernel
 template <typename T, int SPLIT>
-__global__ void __launch_bounds__(BT, 1)
+__global__ void __launch_bounds__(BT, batched_ctas<T>())
 k_batched(BatchArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *Ps = reinterpret_cast<T *>(smem_raw);        // [NMAX][ps_ld]
     T *Ds = Ps + NMAX * ps_ld<T>();                 // [32][33]
-    T *D2 = Ds + NBMAXB * (NBMAXB + 1);             // [32][33]
-    T *Ys = D2 + NBMAXB * (NBMAXB + 1);             // [NMAX]
+    T *D2 = Ds + BLK_ELEMS;                         // [32][33]
+    T *Dn = D2 + BLK_ELEMS;                         // [32][33]
+    T *W8 = Dn + BLK_ELEMS;                         // [2][32][8]
+    T *Ys = W8 + 2 * 8 * NBMAXB;                    // [NMAX]
     T *rdiag = Ys + NMAX;                           // [32]
-    T *Li = rdiag + NBMAXB;                         // [32][ps_ld] diagonal block inverse
-    __shared__ int idx_s, flag_s;
+    __shared__ int idx_s, flag_s, task_s;
     const int tid = threadIdx.x;
     for (;;) {
         if (tid == 0) idx_s = atomicAdd(a.counter, 1);
@@ -574,8 +680,8 @@ k_batched(BatchArgs a)
                 ys = Ys;
             }
             const int info = a.nbsel[m] == 16
-                                 ? factor_one<T, SPLIT, 16>(A, n, Ps, Ds, rdiag, &flag_s, ys, Li, D2)
-                                 : factor_one<T, SPLIT, 32>(A, n, Ps, Ds, rdiag, &flag_s, ys, Li, D2);
+                                 ? factor_one<T, SPLIT, 16>(A, n, Ps, Ds, D2, Dn, W8, rdiag, &flag_s, &task_s, ys)
+                                 : factor_one<T, SPLIT, 32>(A, n, Ps, Ds, D2, Dn, W8, rdiag, &flag_s, &task_s, ys);
             if (tid == 0) a.info[m] = info;
             __syncthreads();
             if (info == 0 && a.op == OP_POSV) solve_one<T>(A, n, b, Ys, D2, rdiag, true);
@@ -585,7 +691,7 @@ k_batched(BatchArgs a)
             solve_adjoint_one<T>(A, n, (const T *)a.B + a.off_b[m], (T *)a.C + a.off_b[m],
                                  (T *)a.D + a.off_a[m], Ys, Ps, D2, rdiag);
         } else {
-            factor_adjoint_one<T>(A, n, (T *)a.D + a.off_a[m], Ps, Ds, D2);
+            factor_adjoint_one<T, SPLIT>(A, n, (T *)a.D + a.off_a[m], Ps, Ds, D2, Dn, W8);
         }
     }
 }
@@ -784,7 +890,8 @@ static int batch_run(plasma_batch_t *p, int prec, int op, void *A, void *B, void
     a.info = info;
     a.counter = p->d_counter;
     a.op = op;
-    int grid = plasma->num_sms;          // one CTA per SM (registers, shared memory)
+    int grid = plasma->num_sms *         // what an SM holds (registers, shared memory)
+               (prec == PlasmaRealDouble ? batched_ctas<double>() : batched_ctas<float>());
     if (grid > p->batch) grid = p->batch;
     cudaStream_t s = plasma->stream;
 

@@ -10,7 +10,7 @@
 //     columns (26 of its 36 blocks resident, 208 KB; the second phase reuses
 //     the slots of the first phase's L11 and reads L21 where it lies);
 //   * one warp factors a 32 x 32 diagonal block, eight columns at a time in
-//     registers (pd_factor32);
+//     registers (blk_factor, f64_blocks.cuh);
 //   * the rows below solve x L^T = a in strips of 8 rows on DMMA, with the
 //     inverses of L's 8 x 8 diagonal blocks (a thread per row spends its time
 //     on broadcast loads of L: 5300 clocks a step against 900-2700);
@@ -39,141 +39,6 @@ constexpr int PD_NMAX = 256;
 __host__ __device__ __forceinline__ int pd_slot(int I, int J, int Rb)
 {
     return J * Rb - J * (J - 1) / 2 + (I - J);
-}
-
-// 1/sqrt(d) for normal d away from the ends of the range: the hardware's
-// approximation (relative error below 2^-20) and one third-order step,
-// r + r e (1/2 + 3/8 e) with e = 1 - d r^2.  Branch-free, so the compiler can
-// run a column's updates between its dependent steps (rsqrt() has a slow
-// path for the ends of the range; blocks that need it take pd_factor32_any).
-__device__ __forceinline__ double pd_rsqrt(double d)
-{
-    double r;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    const double e = fma(-d * r, r, 1.0);
-    return fma(r * e, fma(0.375, e, 0.5), r);
-}
-
-// 32 x 32 Cholesky of the block at S by one warp, in place (zero above the
-// diagonal on exit), and the inverses of its 8 x 8 diagonal blocks to W8.
-// Eight columns at a time: every lane factors the 8 x 8 diagonal block for
-// itself, in registers, so a pivot waits for its reciprocal square root, one
-// multiplication and one multiply-add, and no lane waits for another; its
-// own row and (lanes 0-7) a row of the identity, which becomes a column of
-// the inverse, are eliminated in the gaps.  DMMA updates the columns to the
-// right.  The loop over the four column groups is kept rolled: unrolled, a
-// block is 1500 instructions that run once, and fetching them beside the
-// other warps' code made a step 12500 clocks where 4300 were its latency.
-// False, with S partly overwritten, when a pivot is not well inside the
-// normal range (not positive, NaN, tiny or huge).
-__device__ __forceinline__ bool pd_factor32(double *S, double *W8)
-{
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    bool fine = true;
-#pragma unroll 1
-    for (int o = 0; o < 32; o += 8) {
-        double a[8][8], v[8], u[8];           // a[j][i]: column j, row i >= j
-        double dd = 1.0, rr = 1.0;
-#pragma unroll
-        for (int j = 0; j < 8; j++)
-#pragma unroll
-            for (int i = j & ~1; i < 8; i += 2) {
-                const double2 x = *reinterpret_cast<const double2 *>(S + pd_at(o + j, o + i));
-                a[j][i] = x.x;
-                a[j][i + 1] = x.y;
-            }
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            v[j] = S[pd_at(o + j, lane)];
-            u[j] = lane == j ? 1.0 : 0.0;
-        }
-#pragma unroll
-        for (int c = 0; c < 8; c++) {
-            const double d = a[c][c];
-            fine = fine && d > 1e-280 && d < 1e280;
-            const double r = pd_rsqrt(d);
-#pragma unroll
-            for (int i = c + 1; i < 8; i++) a[c][i] *= r;
-            v[c] *= r;
-            u[c] *= r;
-#pragma unroll
-            for (int j = c + 1; j < 8; j++) {
-#pragma unroll
-                for (int i = j; i < 8; i++) a[j][i] = fma(-a[c][j], a[c][i], a[j][i]);
-                v[j] = fma(-v[c], a[c][j], v[j]);
-                u[j] = fma(-u[c], a[c][j], u[j]);
-            }
-            S[pd_at(o + c, lane)] = lane > o + c ? v[c] : 0.0;
-            if (lane == o + c) {
-                dd = d;
-                rr = r;
-            }
-        }
-        // the diagonal: sqrt(d), one Newton step on d r
-        if ((unsigned)(lane - o) < 8u) {
-            const double s = dd * rr;
-            S[pd_at(lane, lane)] = fma(0.5 * rr, fma(-s, s, dd), s);
-        }
-        if (lane < 8) {
-#pragma unroll
-            for (int i = 0; i < 8; i++) W8[(o + lane) * 8 + i] = u[i];
-        }
-        __syncwarp();
-#pragma unroll
-        for (int f = 1; f < 4; f++)
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                if (8 * f <= o || 16 * h + 15 < 8 * f) continue;
-                const int r0 = 16 * h;
-                const double af[4] = {S[pd_at(o + t, r0 + g)], S[pd_at(o + t, r0 + g + 8)],
-                                      S[pd_at(o + t + 4, r0 + g)],
-                                      S[pd_at(o + t + 4, r0 + g + 8)]};
-                const double bf[2] = {-S[pd_at(o + t, 8 * f + g)],
-                                      -S[pd_at(o + t + 4, 8 * f + g)]};
-                double acc[4];
-#pragma unroll
-                for (int e = 0; e < 4; e++)
-                    acc[e] = S[pd_at(8 * f + 2 * t + (e & 1), r0 + g + 8 * (e >> 1))];
-                dmma_16x8x8(acc, af, bf);
-#pragma unroll
-                for (int e = 0; e < 4; e++)
-                    S[pd_at(8 * f + 2 * t + (e & 1), r0 + g + 8 * (e >> 1))] = acc[e];
-            }
-        __syncwarp();
-    }
-    return fine;
-}
-
-// The same for any pivots, from the copy of the block at O; returns the
-// first bad column + 1 (LAPACK's test), or 0.
-__device__ __noinline__ int pd_factor32_any(double *S, double *W8, const double *O,
-                                            double *rdiag)
-{
-    const int lane = threadIdx.x & 31;
-    int bad = 0;
-    for (int c = 0; c < 32; c++) S[pd_at(c, lane)] = O[pd_at(c, lane)];
-    __syncwarp();
-    for (int c = 0; c < 32; c++) {
-        const double d = S[pd_at(c, c)];
-        const bool ok = d > 0.0;
-        if (!ok && bad == 0) bad = c + 1;
-        const double sd = ok ? sqrt(d) : 1.0, r = 1.0 / sd;
-        const double l = lane == c ? sd : lane > c ? S[pd_at(c, lane)] * r : 0.0;
-        __syncwarp();
-        S[pd_at(c, lane)] = l;
-        if (lane == c) rdiag[c] = r;
-        __syncwarp();
-        for (int c2 = c + 1; c2 <= lane; c2++)
-            S[pd_at(c2, lane)] = fma(-l, S[pd_at(c, c2)], S[pd_at(c2, lane)]);
-        __syncwarp();
-    }
-    const int o = lane & ~7;
-    double w[8];
-    inv8_column(lane & 7, [&](int i, int q) { return S[pd_at(o + q, o + i)]; },
-                [&](int i) { return rdiag[o + i]; }, w);
-#pragma unroll
-    for (int i = 0; i < 8; i++) W8[lane * 8 + i] = w[i];
-    return bad;
 }
 
 // Rows r0 .. r0+7 of the block at X: x L^T = x, one warp
@@ -299,8 +164,8 @@ k_potrf_diag_f64(plasma_desc_t A, int k, int iinfo, plasma_devstat_t *st, int ca
             if (warp == 0) {
                 double *D = S + pd_slot(J, J, Rb) * F64_BLK;
                 int bad = 0;
-                if (!__all_sync(0xffffffffu, pd_factor32(D, W8)))
-                    bad = pd_factor32_any(D, W8, O, rdiag);
+                if (!__all_sync(0xffffffffu, blk_factor<double, 1, 32>(D, W8)))
+                    bad = blk_factor_any<double, 32>(D, W8, O, rdiag);
                 if (lane == 0) bad_s = bad;
             } else if (step == 0) {
                 each(0, 32, 32 * g, warp - 1, PD_WARPS - 1, in);
