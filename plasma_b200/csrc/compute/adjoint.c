@@ -270,14 +270,11 @@ static int Xpotrf_adjoint(plasma_enum_t prec, plasma_enum_t uplo, int n,
         return PlasmaSuccess;
     const int nb = plasma->nb;
     plasma_desc_t L, Lbar;
-    int rc = plasma_desc_general_create(prec, nb, nb, n, n, 0, 0, n, n, &L);
+    int rc = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_A, prec, PlasmaGeneral, nb, n, n, &L);
+    if (rc == PlasmaSuccess)
+        rc = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_AS, prec, PlasmaGeneral, nb, n, n, &Lbar);
     if (rc != PlasmaSuccess)
         return rc;
-    rc = plasma_desc_general_create(prec, nb, nb, n, n, 0, 0, n, n, &Lbar);
-    if (rc != PlasmaSuccess) {
-        plasma_desc_destroy(&L);
-        return rc;
-    }
     plasma_sequence_t sequence;
     plasma_request_t request;
     plasma_sequence_init(&sequence);
@@ -288,8 +285,6 @@ static int Xpotrf_adjoint(plasma_enum_t prec, plasma_enum_t uplo, int n,
     plasma_sequence_wait(&sequence);
     plasma_omp_Xdesc2lapack(Lbar, pLbar, ldlbar, PlasmaGeneral, &sequence, &request);
     plasma_sequence_wait(&sequence);
-    plasma_desc_destroy(&L);
-    plasma_desc_destroy(&Lbar);
     return sequence.status;
 }
 
@@ -334,20 +329,15 @@ static int Xpotrs_adjoint(plasma_enum_t prec, plasma_enum_t uplo, int n, int nrh
         return PlasmaSuccess;
     const int nb = plasma->nb;
     plasma_desc_t L, X, Xbar, Lbar;
-    int rc = plasma_desc_general_create(prec, nb, nb, n, n, 0, 0, n, n, &L);
+    int rc = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_A, prec, PlasmaGeneral, nb, n, n, &L);
     if (rc == PlasmaSuccess)
-        rc = plasma_desc_general_create(prec, nb, nb, n, nrhs, 0, 0, n, nrhs, &X);
+        rc = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_B, prec, PlasmaGeneral, nb, n, nrhs, &X);
     if (rc == PlasmaSuccess)
-        rc = plasma_desc_general_create(prec, nb, nb, n, nrhs, 0, 0, n, nrhs, &Xbar);
+        rc = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_X, prec, PlasmaGeneral, nb, n, nrhs, &Xbar);
     if (rc == PlasmaSuccess)
-        rc = plasma_desc_general_create(prec, nb, nb, n, n, 0, 0, n, n, &Lbar);
-    if (rc != PlasmaSuccess) {
-        plasma_desc_destroy(&L);
-        plasma_desc_destroy(&X);
-        plasma_desc_destroy(&Xbar);
-        plasma_desc_destroy(&Lbar);
+        rc = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_AS, prec, PlasmaGeneral, nb, n, n, &Lbar);
+    if (rc != PlasmaSuccess)
         return rc;
-    }
     plasma_sequence_t sequence;
     plasma_request_t request;
     plasma_sequence_init(&sequence);
@@ -361,10 +351,6 @@ static int Xpotrs_adjoint(plasma_enum_t prec, plasma_enum_t uplo, int n, int nrh
     plasma_omp_Xdesc2lapack(Xbar, pXbar, ldxbar, PlasmaGeneral, &sequence, &request);
     plasma_omp_Xdesc2lapack(Lbar, pLbar, ldlbar, uplo, &sequence, &request);
     plasma_sequence_wait(&sequence);
-    plasma_desc_destroy(&L);
-    plasma_desc_destroy(&X);
-    plasma_desc_destroy(&Xbar);
-    plasma_desc_destroy(&Lbar);
     return sequence.status;
 }
 

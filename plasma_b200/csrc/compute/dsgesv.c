@@ -424,15 +424,13 @@ int plasma_dsgesv(int n, int nrhs, double *pA, int lda, int *ipiv, double *pB, i
     if (rc != PlasmaSuccess)
         return rc;
     plasma_desc_t *rhs[4] = {&B, &X, &R, &Xs};
-    int made = 0;
-    for (; made < 4 && rc == PlasmaSuccess; made++)
-        rc = plasma_desc_general_create(made == 3 ? PlasmaRealFloat : PlasmaRealDouble, nb, nb,
-                                        n, nrhs, 0, 0, n, nrhs, rhs[made]);
-    if (rc != PlasmaSuccess) {
-        for (int i = 0; i < made - 1; i++)
-            plasma_desc_destroy(rhs[i]);
+    static const int slot[4] = {PLASMA_SLOT_DESC_B, PLASMA_SLOT_DESC_X, PLASMA_SLOT_DESC_R,
+                                PLASMA_SLOT_DESC_XS};
+    for (int i = 0; i < 4 && rc == PlasmaSuccess; i++)
+        rc = plasma_desc_kept(plasma, slot[i], i == 3 ? PlasmaRealFloat : PlasmaRealDouble,
+                              PlasmaGeneral, nb, n, nrhs, rhs[i]);
+    if (rc != PlasmaSuccess)
         return rc;
-    }
     plasma_sequence_t sequence;
     plasma_request_t request;
     plasma_sequence_init(&sequence);
@@ -444,7 +442,5 @@ int plasma_dsgesv(int n, int nrhs, double *pA, int lda, int *ipiv, double *pB, i
     plasma_sequence_wait(&sequence);
     plasma_omp_Xdesc2lapack(X, pX, ldx, PlasmaGeneral, &sequence, &request);
     plasma_sequence_wait(&sequence);
-    for (int i = 0; i < 4; i++)
-        plasma_desc_destroy(rhs[i]);
     return sequence.status;
 }

@@ -786,18 +786,15 @@ int plasma_dsposv_ex(plasma_enum_t uplo, int n, int nrhs,
         (retval = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_AS, PlasmaRealFloat, PlasmaLower,
                                    nb, npad, npad, &As)) != 0)
         return retval;
-    if ((retval = plasma_desc_general_create(PlasmaRealDouble, nb, nb, n, nrhs,
-                                             0, 0, n, nrhs, &B)) != 0 ||
-        (retval = plasma_desc_general_create(PlasmaRealDouble, nb, nb, n, nrhs,
-                                             0, 0, n, nrhs, &X)) != 0 ||
-        (retval = plasma_desc_general_create(PlasmaRealDouble, nb, nb, n, nrhs,
-                                             0, 0, n, nrhs, &R)) != 0 ||
-        (retval = plasma_desc_general_create(PlasmaRealFloat, nb, nb, npad, nrhs,
-                                             0, 0, npad, nrhs, &Xs)) != 0) {
-        plasma_error("plasma_desc_general_create() failed");
-        plasma_desc_destroy(&B);
-        plasma_desc_destroy(&X); plasma_desc_destroy(&R);
-        plasma_desc_destroy(&Xs);
+    if ((retval = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_B, PlasmaRealDouble, PlasmaGeneral,
+                                   nb, n, nrhs, &B)) != 0 ||
+        (retval = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_X, PlasmaRealDouble, PlasmaGeneral,
+                                   nb, n, nrhs, &X)) != 0 ||
+        (retval = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_R, PlasmaRealDouble, PlasmaGeneral,
+                                   nb, n, nrhs, &R)) != 0 ||
+        (retval = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_XS, PlasmaRealFloat, PlasmaGeneral,
+                                   nb, npad, nrhs, &Xs)) != 0) {
+        plasma_error("tile copies of the right-hand sides failed");
         return retval;
     }
     double *Rnorm = (double *)malloc(sizeof(double) * nrhs);
@@ -834,9 +831,6 @@ int plasma_dsposv_ex(plasma_enum_t uplo, int n, int nrhs,
     plasma_omp_Xdesc2lapack(X, pX, ldx, PlasmaGeneral, &sequence, &request);
     plasma_sequence_wait(&sequence);
 
-    plasma_desc_destroy(&B);
-    plasma_desc_destroy(&X); plasma_desc_destroy(&R);
-    plasma_desc_destroy(&Xs);
     free(Rnorm);
     free(Xnorm);
     return sequence.status;

@@ -443,7 +443,7 @@ static int Xband(plasma_enum_t prec, int op, plasma_enum_t uplo, int n, int kd, 
         return retval;
     const int nb = plasma->nb;
     if (op != OP_TRF) {
-        retval = plasma_desc_general_create(prec, nb, nb, n, nrhs, 0, 0, n, nrhs, &B);
+        retval = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_B, prec, PlasmaGeneral, nb, n, nrhs, &B);
         if (retval != PlasmaSuccess)
             return retval;
     }
@@ -469,8 +469,6 @@ static int Xband(plasma_enum_t prec, int op, plasma_enum_t uplo, int n, int kd, 
     if (op != OP_TRF)
         plasma_omp_Xdesc2lapack(B, pB, ldb, PlasmaGeneral, &sequence, &request);
     plasma_sequence_wait(&sequence);
-    if (op != OP_TRF)
-        plasma_desc_destroy(&B);
     return sequence.status;
 }
 

@@ -176,7 +176,7 @@ static int Xpotrs(plasma_enum_t prec, plasma_enum_t uplo, int n, int nrhs,
                                   &A);
     if (retval != PlasmaSuccess)
         return retval;
-    retval = plasma_desc_general_create(prec, nb, nb, n, nrhs, 0, 0, n, nrhs, &B);
+    retval = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_B, prec, PlasmaGeneral, nb, n, nrhs, &B);
     if (retval != PlasmaSuccess)
         return retval;
     plasma_sequence_t sequence;
@@ -192,7 +192,6 @@ static int Xpotrs(plasma_enum_t prec, plasma_enum_t uplo, int n, int nrhs,
     plasma_omp_Xdesc2lapack(B, pB, ldb, PlasmaGeneral, &sequence, &request);
     plasma_sequence_wait(&sequence);
 
-    plasma_desc_destroy(&B);
     return sequence.status;
 }
 
@@ -228,7 +227,7 @@ static int Xposv(plasma_enum_t prec, plasma_enum_t uplo, int n, int nrhs,
     A = plasma_desc_view(F, 0, 0, n, n);
     if (np > n)
         plasma_cuda_set_diag(plasma->stream, F, n, np, 1.0);
-    retval = plasma_desc_general_create(prec, nb, nb, n, nrhs, 0, 0, n, nrhs, &B);
+    retval = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_B, prec, PlasmaGeneral, nb, n, nrhs, &B);
     if (retval != PlasmaSuccess)
         return retval;
     plasma_sequence_t sequence;
@@ -258,7 +257,6 @@ static int Xposv(plasma_enum_t prec, plasma_enum_t uplo, int n, int nrhs,
     plasma_omp_Xdesc2lapack(B, pB, ldb, PlasmaGeneral, &sequence, &request);
     plasma_sequence_wait(&sequence);
 
-    plasma_desc_destroy(&B);
     return sequence.status;
 }
 
