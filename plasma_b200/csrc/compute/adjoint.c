@@ -116,8 +116,8 @@ void plasma_pXpotrf_adjoint(plasma_context_t *plasma, plasma_enum_t uplo,
     plasma_view_t phi = view(W1, 1, 1);
     phi.diag_scale = 1;
     plasma_cuda_copy_view(s, st, n, n, phi, view(W2, 0, 0));
-    /* W2 = L^-T Phi(P)^T = (Phi(P) L^-1)^T */
-    plasma_cuda_trsm_sweep(s, st, uplo, PlasmaTrans, L, W2, winv, 0);
+    /* W2 = L^-T Phi(P)^T = (Phi(P) L^-1)^T, upper triangular */
+    plasma_cuda_trsm_sweep_tri(s, st, uplo, PlasmaTrans, L, W2, winv, 0, 1);
     /* W1 = Phi(P) L^-1, then W1 = L^-T Phi(P) L^-1 */
     plasma_cuda_copy_view(s, st, n, n, view(W2, 1, 0), view(W1, 0, 0));
     plasma_cuda_trsm_sweep(s, st, uplo, PlasmaTrans, L, W1, winv, 1);

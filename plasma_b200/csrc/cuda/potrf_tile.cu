@@ -10,9 +10,12 @@
 //    (the nt-k-1 plasma_core_dtrsm tasks of compute/pzpotrf.c:50-56).  Each
 //    CTA keeps 32 rows of one tile in shared memory and eliminates column by
 //    column; L_kk is read from L2.
-//  * k_trtri_tiles: inverses of all diagonal tiles of a factor, one CTA per
-//    tile, used by the blocked triangular solves of potrs.
+//  * inverses of all diagonal tiles of a factor, used by the blocked
+//    triangular solves with many right-hand sides: tiles of 64, 128 and 256
+//    from their 64 x 64 diagonal blocks by products (k_trtri_base,
+//    k_trtri_join), others by elimination, one CTA per tile (k_trtri_tiles).
 #include "common.cuh"
+#include "inv64.cuh"
 
 namespace {
 
@@ -227,6 +230,123 @@ k_trtri_tiles(plasma_desc_t A, int uplo, T *W, const plasma_devstat_t *st)
     }
 }
 
+// ---------------------------------------------------------------------------
+// The same inverses for nb = 64, 128, 256, formed in FP64 (also for FP32
+// factors): the 64 x 64 diagonal blocks by inv_lower64, then
+// [A 0; B C]^-1 = [A^-1 0; -C^-1 B A^-1  C^-1] with halves of 64 and of 128
+// rows, the products on DMMA.  Rows and columns past the matrix are the
+// identity, blocks above the diagonal zero.  What bounds the elimination of
+// k_trtri_tiles is its chain of nb steps with two barriers and global reads
+// each: 3.64 ms for 16 tiles of 256, against 3 launches of some 20 us.
+// ---------------------------------------------------------------------------
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_trtri_base(plasma_desc_t A, int uplo, T *W, const plasma_devstat_t *st)
+{
+    extern __shared__ double tb_smem[];
+    double (*Ls)[65] = reinterpret_cast<double (*)[65]>(tb_smem);
+    double (*Iv)[65] = Ls + 64;
+    double (*Tm)[33] = reinterpret_cast<double (*)[33]>(Iv + 64);
+    if (plasma_failed(st)) return;
+    const int nb = A.mb, k = blockIdx.x, d = blockIdx.y;
+    const TileView<T> L = tile_view<T>(A, uplo, k, k);
+    const int tid = threadIdx.x, o = 64 * d;
+    for (int e = tid; e < 64 * 64; e += 256) {
+        const int x = e % 64, y = e / 64, i = L.trans ? y : x, c = L.trans ? x : y;
+        Ls[i][c] = o + i < L.rows && o + c < L.rows && i >= c ? (double)L.at(o + i, o + c)
+                                                              : (i == c ? 1.0 : 0.0);
+        Iv[i][c] = 0.0;
+    }
+    __syncthreads();
+    inv_lower64(Ls, Iv, Tm, false);
+    T *w = W + (size_t)k * nb * nb + (size_t)o * nb;
+    for (int e = tid; e < 64 * 64; e += 256)
+        w[(size_t)(e / 64) * nb + o + e % 64] = (T)Iv[e % 64][e / 64];
+    for (int e = tid; e < 64 * o; e += 256) w[(size_t)(e / o) * nb + e % o] = T(0);
+}
+
+// One CTA per (tile, pair of halves of h rows, 64 columns of the result): a
+// warp owns 16 rows.
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_trtri_join(plasma_desc_t A, int uplo, int h, T *W, const plasma_devstat_t *st)
+{
+    extern __shared__ double tj_smem[];          // B A^-1: [h][68]
+    if (plasma_failed(st)) return;
+    const int nb = A.mb, k = blockIdx.x;
+    const int o = 2 * h * (blockIdx.y / (h / 64)), j0 = 64 * (blockIdx.y % (h / 64));
+    const TileView<T> L = tile_view<T>(A, uplo, k, k);
+    T *w = W + (size_t)k * nb * nb;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int i0 = 16 * warp;
+    double acc[8][4];
+    auto clear = [&]() {
+#pragma unroll
+        for (int f = 0; f < 8; f++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[f][e] = 0.0;
+    };
+    auto Bv = [&](int i, int c) {                 // B(i, c), zero past the matrix
+        return o + h + i < L.rows && o + c < L.rows ? (double)L.at(o + h + i, o + c) : 0.0;
+    };
+    clear();
+    if (i0 < h) {
+        for (int q = j0; q < h; q += 8) {         // A^-1 is lower: rows q >= column j0
+            const double af[4] = {Bv(i0 + g, q + t), Bv(i0 + g + 8, q + t), Bv(i0 + g, q + t + 4),
+                                  Bv(i0 + g + 8, q + t + 4)};
+#pragma unroll
+            for (int f = 0; f < 8; f++) {
+                const T *col = w + (size_t)(o + j0 + 8 * f + g) * nb + o + q;
+                const double bf[2] = {(double)col[t], (double)col[t + 4]};
+                dmma_16x8x8(acc[f], af, bf);
+            }
+        }
+#pragma unroll
+        for (int f = 0; f < 8; f++)
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                tj_smem[(i0 + g + 8 * (e >> 1)) * 68 + 8 * f + 2 * t + (e & 1)] = acc[f][e];
+    }
+    __syncthreads();
+    if (i0 >= h) return;
+    clear();
+    for (int q = 0; q < i0 + 16; q += 8) {        // C^-1 is lower
+        const T *c0 = w + (size_t)(o + h + q + t) * nb + o + h + i0 + g, *c4 = c0 + (size_t)4 * nb;
+        const double af[4] = {(double)c0[0], (double)c0[8], (double)c4[0], (double)c4[8]};
+#pragma unroll
+        for (int f = 0; f < 8; f++) {
+            const double bf[2] = {tj_smem[(q + t) * 68 + 8 * f + g],
+                                  tj_smem[(q + t + 4) * 68 + 8 * f + g]};
+            dmma_16x8x8(acc[f], af, bf);
+        }
+    }
+#pragma unroll
+    for (int f = 0; f < 8; f++)
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            w[(size_t)(o + j0 + 8 * f + 2 * t + (e & 1)) * nb + o + h + i0 + g + 8 * (e >> 1)] =
+                (T)-acc[f][e];
+}
+
+template <typename T>
+void launch_trtri_join(cudaStream_t s, plasma_devstat_t *st, int uplo, const plasma_desc_t &A,
+                       T *W)
+{
+    constexpr int BASE = (2 * 64 * 65 + 64 * 33) * (int)sizeof(double);
+    static unsigned long long attr = 0;
+    if (plasma_first_on_device(&attr)) {
+        cudaFuncSetAttribute(k_trtri_base<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, BASE);
+        cudaFuncSetAttribute(k_trtri_join<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             128 * 68 * (int)sizeof(double));
+    }
+    k_trtri_base<T><<<dim3(A.mt, A.mb / 64), 256, BASE, s>>>(A, uplo, W, st);
+    for (int h = 64; h < A.mb; h *= 2) {
+        PLASMA_COUNT_LAUNCH();
+        k_trtri_join<T><<<dim3(A.mt, A.mb / (2 * h) * (h / 64)), 256, h * 68 * sizeof(double), s>>>(
+            A, uplo, h, W, st);
+    }
+}
+
 template <typename T>
 void launch_potrf_tile(cudaStream_t s, plasma_devstat_t *st, int call,
                        int uplo, const plasma_desc_t &A, int k, int iinfo)
@@ -327,6 +447,13 @@ extern "C" void plasma_cuda_trtri_tiles(cudaStream_t s, plasma_devstat_t *st,
 {
     if (A.mt == 0) return;
     PLASMA_COUNT_LAUNCH();
+    if (A.mb == 64 || A.mb == 128 || A.mb == 256) {
+        if (A.precision == PlasmaRealDouble)
+            launch_trtri_join<double>(s, st, uplo, A, (double *)W);
+        else
+            launch_trtri_join<float>(s, st, uplo, A, (float *)W);
+        return;
+    }
     if (A.precision == PlasmaRealDouble)
         launch_trtri<double>(s, st, uplo, A, (double *)W);
     else

@@ -12,6 +12,7 @@
 //                                     (the gemm tasks of pztrsm.c:131-141).
 // The sweeps are HBM bound: each reads the triangle of the factor once.
 #include "common.cuh"
+#include "mma.cuh"
 
 #include <string.h>
 
@@ -46,13 +47,13 @@ __device__ __forceinline__ void warp_row(const T *row, int cb, int ce,
 // out(k) = op(W_k) * B(k, chunk), op = identity (forward) or transpose.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-k_diag_apply(plasma_desc_t B, int k, const T *W, int nbw, int trans,
+k_diag_apply(plasma_desc_t B, int k, int n0, const T *W, int nbw, int trans,
              const plasma_devstat_t *st)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T (*Bs)[kCols + 1] = reinterpret_cast<T (*)[kCols + 1]>(smem_raw);
     if (plasma_failed(st)) return;
-    const int n = blockIdx.x;
+    const int n = n0 + blockIdx.x;
     const int c0 = blockIdx.y * kCols;
     const int rows = plasma_tile_mview(B, k);
     const int cols = min(kCols, plasma_tile_nview(B, n) - c0);
@@ -94,6 +95,108 @@ k_diag_apply(plasma_desc_t B, int k, const T *W, int nbw, int trans,
         for (int j = 0; j < kCols; j++)
             if (j < cols) b[(size_t)(c0 + j) * ldb + i] = acc[j];
     }
+}
+
+// The same product for many right-hand sides, on the tensor cores: one CTA per
+// 32 columns of B(k, :), whose tile rows it holds in shared memory, a warp per
+// nb/8 = 16 MI rows of the result; W_k is read from L2 in operand form, the
+// part on and below its diagonal only.  2 x 256 x 256 x 4096 flops a step: 15
+// us at the FP64 rate; the thread-per-row kernel above takes 103 us.
+constexpr int DM_COLS = 32;
+
+template <typename T, int MI>
+__global__ void __launch_bounds__(kThreads)
+k_diag_mma(plasma_desc_t B, int k, int n0, const T *W, int trans, const plasma_devstat_t *st)
+{
+    constexpr int NB = 128 * MI, LDS = DM_COLS + Pad<T>::v, NF = DM_COLS / 8;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *Bs = reinterpret_cast<T *>(smem_raw);              // [NB][LDS]
+    if (plasma_failed(st)) return;
+    const int n = n0 + blockIdx.x, c0 = blockIdx.y * DM_COLS;
+    const int rows = plasma_tile_mview(B, k);
+    const int cols = min(DM_COLS, plasma_tile_nview(B, n) - c0);
+    if (cols <= 0) return;
+    const int ldb = plasma_tile_mmain(B, k);
+    T *b = (T *)plasma_tile_addr(B, k, n) + (size_t)c0 * ldb;
+    const T *w = W + (size_t)k * NB * NB;
+    for (int e = threadIdx.x; e < NB * DM_COLS; e += kThreads) {
+        const int r = e % NB, c = e / NB;
+        Bs[r * LDS + c] = r < rows && c < cols ? b[(size_t)c * ldb + r] : T(0);
+    }
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int i0 = 16 * MI * warp;
+    T acc[MI][NF][4], sum[MI][NF][4];
+#pragma unroll
+    for (int m = 0; m < MI; m++)
+#pragma unroll
+        for (int f = 0; f < NF; f++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[m][f][e] = sum[m][f][e] = T(0);
+    // operator entry (i, q): W(i, q) or W(q, i), both lower triangles of W
+    auto op = [&](int i, int q) {
+        return trans ? w[(size_t)i * NB + q] : w[(size_t)q * NB + i];
+    };
+    const int q0 = trans ? i0 : 0, q1 = trans ? NB : i0 + 16 * MI;
+    T an[MI][4];
+    auto fetch = [&](int q) {
+#pragma unroll
+        for (int m = 0; m < MI; m++)
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                an[m][e] = op(i0 + 16 * m + g + 8 * (e & 1), q + t + 4 * (e >> 1));
+    };
+    fetch(q0);
+    for (int q = q0; q < q1; q += 8) {
+        T a[MI][4], bf[NF][2];
+#pragma unroll
+        for (int m = 0; m < MI; m++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) a[m][e] = an[m][e];
+        if (q + 8 < q1) fetch(q + 8);
+#pragma unroll
+        for (int f = 0; f < NF; f++) {
+            bf[f][0] = Bs[(q + t) * LDS + 8 * f + g];
+            bf[f][1] = Bs[(q + t + 4) * LDS + 8 * f + g];
+        }
+#pragma unroll
+        for (int m = 0; m < MI; m++)
+#pragma unroll
+            for (int f = 0; f < NF; f++) mma8<3>(acc[m][f], a[m], bf[f]);
+        // FP32: the tensor cores truncate long sums; leave them every 32 terms
+        if (sizeof(T) == 8 ? q + 8 >= q1 : ((q & 24) == 24 || q + 8 >= q1)) {
+#pragma unroll
+            for (int m = 0; m < MI; m++)
+#pragma unroll
+                for (int f = 0; f < NF; f++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        sum[m][f][e] += acc[m][f][e];
+                        acc[m][f][e] = T(0);
+                    }
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < MI; m++)
+#pragma unroll
+        for (int f = 0; f < NF; f++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int r = i0 + 16 * m + g + 8 * (e >> 1), c = 8 * f + 2 * t + (e & 1);
+                if (r < rows && c < cols) b[(size_t)c * ldb + r] = sum[m][f][e];
+            }
+}
+
+template <typename T, int MI>
+void launch_diag_mma(cudaStream_t s, plasma_devstat_t *st, const plasma_desc_t &B, int k, int n0,
+                     const T *W, int trans)
+{
+    constexpr int SMEM = 128 * MI * (DM_COLS + Pad<T>::v) * (int)sizeof(T);
+    static unsigned long long attr = 0;
+    if (plasma_first_on_device(&attr))
+        cudaFuncSetAttribute(k_diag_mma<T, MI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    k_diag_mma<T, MI><<<dim3(B.nt - n0, B.nb / DM_COLS), kThreads, SMEM, s>>>(B, k, n0, W, trans,
+                                                                             st);
 }
 
 // B(m, chunk) -= op(L) * B(k, chunk) for the tiles m in [mlo, mhi)
@@ -156,9 +259,12 @@ k_solve_update(plasma_desc_t A, int uplo, plasma_desc_t B, int k, int mlo,
 // diagonal down (logical lower view), so step k only reaches tile rows
 // [k+1, k+kt) forward and [k-kt+1, k) backward (the reference's band solve,
 // compute/pztbsm.c, visits the same tiles).
+// tri: B is upper triangular by tiles (zero left of tile column k in tile row
+// k) and the sweep goes backward, so it stays so: step k takes the columns
+// from tile column k on only.
 template <typename T>
 void sweep(cudaStream_t s, plasma_devstat_t *st, int uplo, int trans,
-           const plasma_desc_t &A, const plasma_desc_t &B, const T *W, int kt)
+           const plasma_desc_t &A, const plasma_desc_t &B, const T *W, int kt, int tri)
 {
     const int mt = B.mt;
     const int nbw = A.mb;
@@ -178,9 +284,15 @@ void sweep(cudaStream_t s, plasma_devstat_t *st, int uplo, int trans,
     const bool gemm = B.n >= 64 && A.mb == B.mb;
     for (int step = 0; step < mt; step++) {
         int k = trans ? mt - 1 - step : step;
+        const int n0 = tri ? k : 0;
         PLASMA_COUNT_LAUNCH();
-        k_diag_apply<T><<<dim3(B.nt, chunks), kThreads, smem, s>>>(
-            B, k, W, nbw, trans, st);
+        if (gemm && B.nb == nbw && nbw == 256)
+            launch_diag_mma<T, 2>(s, st, B, k, n0, W, trans);
+        else if (gemm && B.nb == nbw && nbw == 128)
+            launch_diag_mma<T, 1>(s, st, B, k, n0, W, trans);
+        else
+            k_diag_apply<T><<<dim3(B.nt - n0, chunks), kThreads, smem, s>>>(
+                B, k, n0, W, nbw, trans, st);
         int mlo = trans ? 0 : k + 1;
         int mhi = trans ? k : mt;
         if (kt > 0) {
@@ -188,7 +300,7 @@ void sweep(cudaStream_t s, plasma_devstat_t *st, int uplo, int trans,
             else mhi = min(mt, k + kt);
         }
         if (gemm && mhi > mlo &&
-            plasma_cuda_sweep_update_mma(s, st, uplo, trans, A, B, k, mlo, mhi)) {
+            plasma_cuda_sweep_update_mma(s, st, uplo, trans, A, B, k, mlo, mhi, n0)) {
             // square tiles, a multiple of 128: the tensor-core sweep update
             // (cuda/update.cu)
         } else if (gemm && mhi > mlo && kt == 0) {
@@ -237,6 +349,16 @@ extern "C" void plasma_cuda_trsm_sweep(cudaStream_t s, plasma_devstat_t *st,
                                        plasma_desc_t A, plasma_desc_t B,
                                        void *W, int have_w)
 {
+    plasma_cuda_trsm_sweep_tri(s, st, uplo, trans, A, B, W, have_w, 0);
+}
+
+// The same with tri != 0 for a backward sweep over a B that is upper
+// triangular by tiles (and stays so).
+extern "C" void plasma_cuda_trsm_sweep_tri(cudaStream_t s, plasma_devstat_t *st,
+                                           plasma_enum_t uplo, plasma_enum_t trans,
+                                           plasma_desc_t A, plasma_desc_t B,
+                                           void *W, int have_w, int tri)
+{
     if (B.mt == 0 || B.nt == 0) return;
     if (!have_w)
         plasma_cuda_trtri_tiles(s, st, uplo, A, W);
@@ -246,9 +368,9 @@ extern "C" void plasma_cuda_trsm_sweep(cudaStream_t s, plasma_devstat_t *st,
     double n = B.m, nrhs = B.n, es = plasma_element_size(A.precision);
     int prof = plasma_prof_begin(s);
     if (A.precision == PlasmaRealDouble)
-        sweep<double>(s, st, uplo, t, A, B, (const double *)W, kt);
+        sweep<double>(s, st, uplo, t, A, B, (const double *)W, kt, tri);
     else
-        sweep<float>(s, st, uplo, t, A, B, (const float *)W, kt);
+        sweep<float>(s, st, uplo, t, A, B, (const float *)W, kt, tri);
     // one triangle of the factor (or its band) read once, B read and
     // written once
     double w = kt > 0 ? fmin(n, (double)kt * A.mb) : n;

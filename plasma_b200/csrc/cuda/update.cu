@@ -303,6 +303,7 @@ struct SweepArgs {
     int uplo, trans;          // trans: backward sweep (L^T)
     int k, mlo, mhi;
     int sbm, ncb;             // row halves per tile, 64-column blocks of B
+    int col0;                 // first column
 };
 
 template <typename T>
@@ -341,7 +342,7 @@ k_sweep_mma(SweepArgs g, int nitems, const plasma_devstat_t *st)
         const int i0 = si * DBM;
         const int rows = plasma_tile_mview(g.B, m);
         if (i0 >= rows) continue;
-        const int jcol = jb * DBN;                    // first column of B
+        const int jcol = g.col0 + jb * DBN;           // first column of B
         const int jt = jcol / nb, jo = jcol - jt * nb;
         const int cols = min(DBN, plasma_tile_nview(g.B, jt) - jo);
         if (cols <= 0) continue;              // past a ragged last column tile
@@ -626,20 +627,20 @@ extern "C" void plasma_cuda_update(cudaStream_t s, plasma_devstat_t *st,
 
 // One update step of a tile sweep with many right-hand sides (see
 // k_sweep_mma): B rows of tiles [mlo, mhi) -= the factor block coupling them
-// with tile row k times B(k, :).  FP64 on DMMA, FP32 as three TF32
+// with tile row k times B(k, :), for the column tiles from n0 on.  FP64 on DMMA, FP32 as three TF32
 // products.  Returns 0 (nothing launched) when the tiling does not fit
 // (square tiles, a multiple of 128).
 extern "C" int plasma_cuda_sweep_update_mma(cudaStream_t s, plasma_devstat_t *st,
                                             plasma_enum_t uplo, int trans,
                                             plasma_desc_t L, plasma_desc_t B, int k,
-                                            int mlo, int mhi)
+                                            int mlo, int mhi, int n0)
 {
     if (L.precision != B.precision ||
         (L.precision != PlasmaRealDouble && L.precision != PlasmaRealFloat) ||
         L.mb != L.nb || B.mb != L.mb || B.nb != L.nb || L.mb % DBM != 0 ||
         L.i != 0 || L.j != 0 || B.i != 0 || B.j != 0)
         return 0;
-    if (mhi <= mlo || B.n == 0) return 1;
+    if (mhi <= mlo || B.n == 0 || n0 >= B.nt) return 1;
     SweepArgs g;
     g.L = L;
     g.B = B;
@@ -650,7 +651,8 @@ extern "C" int plasma_cuda_sweep_update_mma(cudaStream_t s, plasma_devstat_t *st
     g.mhi = mhi;
     g.sbm = L.mb / DBM;
     // 64-column blocks per column tile, times the column tiles
-    g.ncb = ((B.nb + DBN - 1) / DBN) * B.nt;
+    g.ncb = ((B.nb + DBN - 1) / DBN) * (B.nt - n0);
+    g.col0 = n0 * B.nb;
     const long long nitems = (long long)(mhi - mlo) * g.sbm * g.ncb;
     PLASMA_COUNT_LAUNCH();
     if (L.precision == PlasmaRealDouble) {

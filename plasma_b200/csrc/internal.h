@@ -201,11 +201,16 @@ void plasma_cuda_trtri_tiles(cudaStream_t s, plasma_devstat_t *st,
  * FP32 three-product TF32); 0 when the tiling does not fit (cuda/update.cu). */
 int plasma_cuda_sweep_update_mma(cudaStream_t s, plasma_devstat_t *st,
                                   plasma_enum_t uplo, int trans, plasma_desc_t L,
-                                  plasma_desc_t B, int k, int mlo, int mhi);
+                                  plasma_desc_t B, int k, int mlo, int mhi, int n0);
 void plasma_cuda_trsm_sweep(cudaStream_t s, plasma_devstat_t *st,
                             plasma_enum_t uplo, plasma_enum_t trans,
                             plasma_desc_t A, plasma_desc_t B,
                             void *W, int have_w);
+/* tri: a backward sweep over a B that is upper triangular by tiles. */
+void plasma_cuda_trsm_sweep_tri(cudaStream_t s, plasma_devstat_t *st,
+                                plasma_enum_t uplo, plasma_enum_t trans,
+                                plasma_desc_t A, plasma_desc_t B,
+                                void *W, int have_w, int tri);
 
 /* Diagonal-tile Cholesky of tile (k,k) (uplo Lower or Upper), writing
  * info = iinfo + j on a non-positive pivot in column j (1-based).  If winv is
