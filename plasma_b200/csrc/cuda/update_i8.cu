@@ -23,9 +23,10 @@
 // holding Inf or NaN makes its products NaN.
 //
 // k_panel_i8: digits of a panel, one CTA per 32 rows; global layout by units
-// of 64 rows: [unit][K / 32][digit][8-row group][16-byte half][8 rows][16 B],
-// the no-swizzle K-major operand form, so that operands are plain bulk
-// copies.
+// of 128 rows: [unit][K / 32][digit][8-row group][16-byte half][8 rows][16
+// B], the no-swizzle K-major operand form, so that a stage of the row operand
+// is one bulk copy of 28 KB (as fourteen of 2 KB their issue took longer than
+// the stage's products).
 //
 // k_update_i8: one CTA per run of 128 x 64 blocks of C of one column block.
 //   warp 0    : bulk copies -- the column block's digits (64 rows x K x 7,
@@ -36,8 +37,12 @@
 //               in shared memory: for digit p of the rows one product of
 //               N = 64 (7 - p) columns adds to the sums p .. 6 at once (two
 //               where that exceeds 256).  10 MMAs per 32 columns of K;
-//   warps 4-11: per block, joins the sums and frees tensor memory, then
-//               updates C while the next block's products run.
+//   warps 2-9 : per block, read C while the products run, join the sums,
+//               subtract and free tensor memory, store C.
+// n = 8192, first bulk step (3422 blocks, two waves): 6.3 us a block and SM
+// with no epilogue at all (the products are 3.9 us of tensor pipe at full
+// rate; the rest is the wave's start and the hand-over of tensor memory, of
+// which there is only one set); 9.4 us with C read after the products.
 // Every wait is bounded (tc.cuh).
 #include "common.cuh"
 #include "tc.cuh"
@@ -48,10 +53,10 @@ constexpr int I8_S = 7;                        // digits
 constexpr int I8_M = 128, I8_N = 64;
 constexpr int I8_KB = 32;                      // K per stage and MMA
 constexpr int I8_UNIT = I8_S * 64 * I8_KB;     // 14 KB: 64 rows, 32 columns
-constexpr int I8_STAGE = 2 * I8_UNIT;
+constexpr int I8_STAGE = 2 * I8_UNIT;          // 128 rows
 constexpr int I8_STAGES = 4;
-constexpr int I8_THREADS = 384;
-constexpr int I8_EPI_WARP0 = 4, I8_EPI_WARPS = 8;
+constexpr int I8_THREADS = 320;
+constexpr int I8_EPI_WARP0 = 2, I8_EPI_WARPS = 8;
 constexpr int I8_NBMAX = 256;
 constexpr int i8_smem(int nb) { return I8_STAGES * I8_STAGE + nb / I8_KB * I8_UNIT + 1024; }
 static_assert(i8_smem(I8_NBMAX) <= 226 * 1024, "shared memory");
@@ -103,8 +108,8 @@ k_panel_i8(plasma_desc_t A, int k, signed char *dig, double *scale, const plasma
     const int s = 55 - e, s1 = s / 2;
     const double f1 = __longlong_as_double((long long)(1023 + s1) << 52);
     const double f2 = __longlong_as_double((long long)(1023 + s - s1) << 52);
-    signed char *u = dig + ((size_t)(m * (nb / 64) + row / 64) * nkb + warp) * I8_UNIT +
-                     (row % 64) / 8 * 256 + (row % 8) * 16;
+    signed char *u = dig + ((size_t)(m * (nb / 128) + row / 128) * nkb + warp) * I8_STAGE +
+                     (row % 128) / 8 * 256 + (row % 8) * 16;
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         uint32_t d[I8_S][4];
@@ -129,7 +134,7 @@ k_panel_i8(plasma_desc_t A, int k, signed char *dig, double *scale, const plasma
         }
 #pragma unroll
         for (int p = 0; p < I8_S; p++)
-            *(uint4 *)(u + p * 2048 + h * 128) = make_uint4(d[p][0], d[p][1], d[p][2], d[p][3]);
+            *(uint4 *)(u + p * 4096 + h * 128) = make_uint4(d[p][0], d[p][1], d[p][2], d[p][3]);
     }
 }
 
@@ -219,6 +224,13 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, int (&r)[8])
                  : "r"(taddr));
 }
 
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c)
+{
+    long long d;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+    return d;
+}
+
 // exact for |v| < 2^51
 __device__ __forceinline__ double small_ll_to_double(long long v)
 {
@@ -237,7 +249,7 @@ k_update_i8(I8Args g, plasma_devstat_t *st)
     const int first = blockIdx.x * g.ipc;
     const int nit = min(g.ipc, g.nitems - first);
     if (nit <= 0) return;
-    const int nb = g.A.mb, nkb = nb / I8_KB, units = nb / 64;
+    const int nb = g.A.mb, nkb = nb / I8_KB, units = nb / 128;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     unsigned char *ring = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char *resb = ring + I8_STAGES * I8_STAGE;
@@ -253,7 +265,7 @@ k_update_i8(I8Args g, plasma_devstat_t *st)
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 2) {
+    if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      :: "r"(smem_u32(&tmem_base_s)), "r"(512u));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -270,8 +282,9 @@ k_update_i8(I8Args g, plasma_devstat_t *st)
         I8Cursor c;
         c.start(g, first);
         for (int j = 0; j < nit && ok; j++, load_b = c.last_of_column(), c.next()) {
-            const signed char *da = g.dig + (size_t)(c.m * units + 2 * c.si) * nkb * I8_UNIT;
-            const signed char *db = g.dig + (size_t)(c.n * units + c.sj) * nkb * I8_UNIT;
+            const signed char *da = g.dig + (size_t)(c.m * units + c.si) * nkb * I8_STAGE;
+            const signed char *db = g.dig + (size_t)(c.n * units + c.sj / 2) * nkb * I8_STAGE +
+                                    c.sj % 2 * 2048;
             if (load_b) {
                 // the products with the block held so far are complete
                 if (loads > 0 && !mbar_wait(&bempty_bar, (loads - 1) & 1, &abort_s)) break;
@@ -286,19 +299,13 @@ k_update_i8(I8Args g, plasma_devstat_t *st)
                 }
                 if (load_b) {
                     mbar_expect_tx(&bfull_bar[kb], I8_UNIT);
-                    bulk_load(resb + kb * I8_UNIT, db + (size_t)kb * I8_UNIT, I8_UNIT,
-                              &bfull_bar[kb]);
-                }
-                // rows 0-63 and 64-127: digit p of both side by side
-                unsigned char *sp = ring + s * I8_STAGE;
-                mbar_expect_tx(&full_bar[s], I8_STAGE);
-#pragma unroll
-                for (int h = 0; h < 2; h++)
 #pragma unroll
                     for (int p = 0; p < I8_S; p++)
-                        bulk_load(sp + p * 4096 + h * 2048,
-                                  da + (size_t)(h * nkb + kb) * I8_UNIT + p * 2048, 2048,
-                                  &full_bar[s]);
+                        bulk_load(resb + kb * I8_UNIT + p * 2048,
+                                  db + (size_t)kb * I8_STAGE + p * 4096, 2048, &bfull_bar[kb]);
+                }
+                mbar_expect_tx(&full_bar[s], I8_STAGE);
+                bulk_load(ring + s * I8_STAGE, da + (size_t)kb * I8_STAGE, I8_STAGE, &full_bar[s]);
             }
         }
     } else if (warp == 1 && lane == 0) {
@@ -345,11 +352,20 @@ k_update_i8(I8Args g, plasma_devstat_t *st)
         for (int j = 0; j < nit; j++, cur.next()) {
             const int m = cur.m, n = cur.n, si = cur.si, sj = cur.sj;
             const int row = si * I8_M + 32 * q + lane;
-            const double si_ = g.scale[(size_t)m * nb + row];
+            const double sr = -g.scale[(size_t)m * nb + row];
+            const int rows = plasma_tile_mview(g.A, m), cols = plasma_tile_mview(g.A, n);
+            double *C = (double *)plasma_tile_addr(g.A, m, n) + row;
+            const size_t ldc = plasma_tile_mmain(g.A, m);
+            const int j0 = sj * I8_N + c0;
+            const double *sc = g.scale + (size_t)n * nb + j0;
+            // columns j0 .. jn-1 of this row are updated
+            const int jn = row < rows ? min(cols, m == n ? row + 1 : cols) : 0;
+            double c[32];
+#pragma unroll
+            for (int i = 0; i < 32; i++) c[i] = j0 + i < jn ? C[(size_t)(j0 + i) * ldc] : 0.0;
             const bool ok = __all_sync(0xffffffffu, mbar_wait(&tfull_bar, j & 1, &abort_s));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            double P[32];
 #pragma unroll
             for (int cc = 0; cc < 32; cc += 8) {
                 int t[I8_S][8];
@@ -359,35 +375,22 @@ k_update_i8(I8Args g, plasma_devstat_t *st)
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
-                    // sum over t of 2^(8 (6 - t)) times the sums, in two exact halves
-                    const long long hi = (((((long long)t[0][i] << 8) + t[1][i]) << 8) + t[2][i]) * 256 + t[3][i];
-                    const long long lo = ((((long long)t[4][i] << 8) + t[5][i]) << 8) + t[6][i];
-                    P[cc + i] = fma(small_ll_to_double(hi), 16777216.0, small_ll_to_double(lo));
+                    // sum over t of 2^(8 (6 - t)) times the sums, in two exact
+                    // halves (the first pair fits 32 bits: at most 2^22 and 2^23)
+                    const long long hi = mad_wide(t[0][i] * 256 + t[1][i], 65536,
+                                                  mad_wide(t[2][i], 256, t[3][i]));
+                    const long long lo = mad_wide(t[4][i], 65536, mad_wide(t[5][i], 256, t[6][i]));
+                    const double P = fma(small_ll_to_double(hi), 16777216.0, small_ll_to_double(lo));
+                    // C -= 2^(e_i + e_j - 62) P, the factor in two exact steps
+                    c[cc + i] = fma(P * sr, __ldg(sc + cc + i), c[cc + i]);
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&tempty_bar);
-            // C -= 2^(e_i + e_j - 62) P, the factor applied in two exact steps
-            const int rows = plasma_tile_mview(g.A, m), cols = plasma_tile_mview(g.A, n);
-            double *C = (double *)plasma_tile_addr(g.A, m, n) + row;
-            const size_t ldc = plasma_tile_mmain(g.A, m);
-            const double *sc = g.scale + (size_t)n * nb;
-            const int j0 = sj * I8_N + c0;
-            // columns j0 .. jn-1 of this row are updated
-            const int jn = row < rows ? min(cols, m == n ? row + 1 : cols) : 0;
 #pragma unroll
-            for (int h = 0; h < 32; h += 16) {
-                double c[16];
-#pragma unroll
-                for (int i = 0; i < 16; i++)
-                    c[i] = j0 + h + i < jn ? C[(size_t)(j0 + h + i) * ldc] : 0.0;
-#pragma unroll
-                for (int i = 0; i < 16; i++)
-                    if (j0 + h + i < jn)
-                        C[(size_t)(j0 + h + i) * ldc] =
-                            fma(-(P[h + i] * si_), __ldg(sc + j0 + h + i), c[i]);
-            }
+            for (int i = 0; i < 32; i++)
+                if (j0 + i < jn) C[(size_t)(j0 + i) * ldc] = c[i];
         }
     }
     // ---------------- teardown
@@ -402,7 +405,8 @@ k_update_i8(I8Args g, plasma_devstat_t *st)
         }
         __syncthreads();
     }
-    if (warp == 2) {
+    if (warp == 1) {
+        __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
                      :: "r"(tmem), "r"(512u));
