@@ -32,6 +32,7 @@
 #include "common.cuh"
 #include "inv64.cuh"
 #include "mma.cuh"
+#include "tc.cuh"
 
 #include <float.h>
 #include <limits.h>
@@ -666,33 +667,49 @@ k_colmax(plasma_desc_t D, double *out, const plasma_devstat_t *st)
 // ---------------------------------------------------------------------------
 // The panel of tile column k (kb <= 64 columns) in one launch, resident in
 // the shared memory of a cluster of CL_CTAS CTAs: CTA c holds panel rows
-// [c R, (c+1) R), column-major.  Per column j: every CTA finds its candidate
-// (the first largest magnitude among its rows >= j) and publishes it with a
-// copy of that row -- and, if it holds row j, a copy of row j -- in a slot of
-// its shared memory (two slots, alternating with j); one cluster barrier;
-// every CTA reads the candidates, picks the pivot p (first largest, as
-// LAPACK's idamax), takes the pivot row from p's owner, and the owners of
-// rows j and p write the swapped rows; then the rows below j are scaled and
-// take the rank-1 update inside the sub-block of CL_IB columns.  After a
-// sub-block its rows are published (one more cluster barrier), every CTA
-// solves them with the unit-lower sub-block diagonal (U12 = L11^-1 A12) and
-// updates its rows below (A22 -= L21 U12).  Every CTA runs the same barrier
-// sequence; a zero pivot records info (the first one, as k_lu_pivot) and
-// the factorization goes on without scaling that column.
+// [c R, (c+1) R), column-major, a thread the rows tid, tid + 128, ...; the
+// CL_IB columns of the running sub-block are in its registers.
+//
+// A column is one chain of latencies (pivot search, exchange, scaling, the
+// next column's entries), so it has no barrier: every warp picks its candidate
+// (the first largest magnitude, as LAPACK's idamax) with warp reductions and
+// sends key, position and the row's CL_IB entries to all CTAs with st.async;
+// the copies complete on each CTA's mbarrier (two, alternating with the
+// column: a warp sends column j + 1 only after it has read column j, so a slot
+// is free when column j + 2 arrives); every warp picks the pivot from the
+// candidates (one a lane) and updates its rows.  Rows do not move: a row
+// keeps its place and carries its position, the interchange swaps two
+// positions, and the rows go to their positions when the panel is written.
+// After a sub-block every CTA reads the pivot rows' remaining columns, solves
+// them with the unit-lower sub-block diagonal (U12 = L11^-1 A12, written to
+// the panel by the CTAs in turn) and updates its rows (A22 -= L21 U12).
+// A zero pivot records info (the first one, as k_lu_pivot) and the
+// factorization goes on without scaling that column.  A 64-column FP32
+// panel of 4096 rows took 168 us with the candidates read across the cluster
+// between barriers and the rows interchanged in shared memory; it takes 96 us
+// (four rows a thread), 79 (two) and 74 (one): about 1.1 us a column is the
+// exchange and the chain around it.  One record per CTA behind a CTA barrier
+// instead of one per warp: 119 us.
 // ---------------------------------------------------------------------------
 constexpr int CL_CTAS = 8;
-constexpr int CL_THREADS = 256;
+constexpr int CL_THREADS = 128;
+constexpr int CL_WARPS = CL_THREADS / 32;
 constexpr int CL_KB = 64;
 constexpr int CL_IB = 16;
+static_assert(CL_CTAS * CL_WARPS == 32, "one candidate a lane");
 
 template <typename T> struct ClLayout {
-    // shared memory after the panel (R x CL_KB): two publication slots of a
-    // candidate row and a row-j copy, the sub-block rows published and the
-    // local copy of them, the pivot row, the row j copy read back
-    static constexpr int EXTRA = (2 * 2 * CL_KB + 2 * CL_IB * CL_KB + 2 * CL_KB) * sizeof(T) +
-                                 2 * (sizeof(T) + sizeof(int)) + 64 * (sizeof(T) + 4) + 64;
+    // shared memory after the panel (CL_KB columns, an odd stride apart): the
+    // candidates' headers and rows (two columns), U12 by columns, the
+    // sub-block's diagonal, each warp's outgoing record, the mbarriers and
+    // the pivot rows' places
+    static constexpr int EXTRA = 2 * 32 * 16 + 2 * 32 * CL_IB * (int)sizeof(T) +
+                                 (CL_KB - CL_IB) * CL_IB * (int)sizeof(T) +
+                                 CL_IB * CL_IB * (int)sizeof(T) +
+                                 CL_WARPS * (16 + CL_IB * (int)sizeof(T)) + 16 + CL_IB * 4;
     static constexpr int MAX_SMEM = 227 * 1024 - 256;      // room for the static part
-    static constexpr int MAX_R = (MAX_SMEM - EXTRA) / (CL_KB * (int)sizeof(T));
+    static constexpr int MAX_R = ((MAX_SMEM - EXTRA) / (CL_KB * (int)sizeof(T)) - 1) | 1;
+    static constexpr int MAX_RPT = (MAX_R + CL_THREADS - 1) / CL_THREADS;
 };
 
 __device__ __forceinline__ uint32_t cl_addr(const void *p, uint32_t rank)
@@ -719,29 +736,94 @@ __device__ __forceinline__ int cl_ld_int(uint32_t a)
     asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     return v;
 }
+// 16 bytes to another CTA of the cluster, counted on its mbarrier
+__device__ __forceinline__ void cl_send(uint32_t a, uint4 v, uint32_t bar)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], "
+                 "{%1, %2, %3, %4}, [%5];"
+                 ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar) : "memory");
+}
 __device__ __forceinline__ void cl_sync()
 {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
                  "barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <typename T>
+// |x| as an integer of the same order, 0 for a NaN (never chosen before a
+// number), and its largest over a warp
+__device__ __forceinline__ uint32_t pivot_key(float x)
+{
+    return x != x ? 0u : (__float_as_uint(x) & 0x7fffffffu) + 1u;
+}
+__device__ __forceinline__ unsigned long long pivot_key(double x)
+{
+    return x != x ? 0ull
+                  : ((unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull) + 1ull;
+}
+__device__ __forceinline__ uint32_t warp_max(uint32_t k)
+{
+    return __reduce_max_sync(0xffffffffu, k);
+}
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long k)
+{
+    const uint32_t hi = __reduce_max_sync(0xffffffffu, (uint32_t)(k >> 32));
+    const uint32_t lo =
+        __reduce_max_sync(0xffffffffu, (uint32_t)(k >> 32) == hi ? (uint32_t)k : 0u);
+    return (unsigned long long)hi << 32 | lo;
+}
+// 16 entries at a 16-byte boundary, 16 bytes a load or store
+__device__ __forceinline__ void ld_row(const float *t, float (&u)[16])
+{
+#pragma unroll
+    for (int c = 0; c < 16; c += 4) {
+        const float4 w = *reinterpret_cast<const float4 *>(t + c);
+        u[c] = w.x; u[c + 1] = w.y; u[c + 2] = w.z; u[c + 3] = w.w;
+    }
+}
+__device__ __forceinline__ void ld_row(const double *t, double (&u)[16])
+{
+#pragma unroll
+    for (int c = 0; c < 16; c += 2) {
+        const double2 w = *reinterpret_cast<const double2 *>(t + c);
+        u[c] = w.x; u[c + 1] = w.y;
+    }
+}
+__device__ __forceinline__ void st_row(float *t, const float (&u)[16])
+{
+#pragma unroll
+    for (int c = 0; c < 16; c += 4)
+        *reinterpret_cast<float4 *>(t + c) = make_float4(u[c], u[c + 1], u[c + 2], u[c + 3]);
+}
+__device__ __forceinline__ void st_row(double *t, const double (&u)[16])
+{
+#pragma unroll
+    for (int c = 0; c < 16; c += 2)
+        *reinterpret_cast<double2 *>(t + c) = make_double2(u[c], u[c + 1]);
+}
+template <typename T> struct PivotKey { typedef uint32_t type; };
+template <> struct PivotKey<double> { typedef unsigned long long type; };
+
+template <typename T, int RPT>
 __global__ void __cluster_dims__(CL_CTAS, 1, 1) __launch_bounds__(CL_THREADS, 1)
 k_lu_panel_cl(plasma_desc_t A, int k, int kb, int R, int *ipiv, plasma_devstat_t *st,
               int call)
 {
+    typedef typename PivotKey<T>::type K;
+    constexpr int V = 16 / (int)sizeof(T);                 // entries in 16 bytes
+    constexpr int CHUNKS = 1 + CL_IB / V;                  // of a record: header, row
+    constexpr uint32_t TX = 32 * 16 * CHUNKS;              // arriving for a column
     extern __shared__ __align__(16) unsigned char cl_raw[];
-    T *P = reinterpret_cast<T *>(cl_raw);                  // [CL_KB][R]
-    T *pub_row = P + (size_t)CL_KB * R;                    // [2][2][CL_KB]
-    T *blk = pub_row + 4 * CL_KB;                          // [CL_IB][CL_KB] published
-    T *u12 = blk + CL_IB * CL_KB;                          // [CL_IB][CL_KB] local copy
-    T *prow = u12 + CL_IB * CL_KB;                         // [CL_KB]
-    T *rowj = prow + CL_KB;                                // [CL_KB]
-    T *pub_val = rowj + CL_KB;                             // [2]
-    int *pub_idx = reinterpret_cast<int *>(pub_val + 2);   // [2]
-    T *red_v = reinterpret_cast<T *>(pub_idx + 2);         // [CL_THREADS / 32]
-    int *red_i = reinterpret_cast<int *>(red_v + CL_THREADS / 32);
-    __shared__ int flag_s, piv_s, bi_s;
+    const int RS = R | 1;
+    T *P = reinterpret_cast<T *>(cl_raw);                  // [CL_KB][RS]
+    uint4 *rec_h = reinterpret_cast<uint4 *>(P + (size_t)CL_KB * RS);   // [2][32]
+    T *rec_r = reinterpret_cast<T *>(rec_h + 2 * 32);      // [2][32][CL_IB]
+    T *l11 = rec_r + 2 * 32 * CL_IB;                       // [CL_IB][CL_IB], by columns
+    T *u12 = l11 + CL_IB * CL_IB;                          // [CL_KB - CL_IB][CL_IB]
+    uint4 *out = reinterpret_cast<uint4 *>(u12 + (CL_KB - CL_IB) * CL_IB);   // [warp][CHUNKS]
+    uint64_t *bar = reinterpret_cast<uint64_t *>(out + CL_WARPS * CHUNKS);   // [2]
+    int *place = reinterpret_cast<int *>(bar + 2);         // [CL_IB]
+    __shared__ int flag_s;
+    __shared__ volatile int abort_s;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint32_t me;
@@ -752,187 +834,224 @@ k_lu_panel_cl(plasma_desc_t A, int k, int kb, int R, int *ipiv, plasma_devstat_t
     const int nown = max(0, min(R, M - row0));             // rows held here
 
     // a uniform start: everyone follows rank 0's reading of the status
-    if (tid == 0) flag_s = plasma_failed(st) ? 1 : 0;
+    if (tid == 0) {
+        flag_s = plasma_failed(st) ? 1 : 0;
+        abort_s = 0;
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        mbar_expect_tx(&bar[0], TX);
+        mbar_expect_tx(&bar[1], TX);
+    }
     cl_sync();
     const int failed = cl_ld_int(cl_addr(&flag_s, 0));
     cl_sync();                     // rank 0 stays until everyone has read it
     if (failed) return;
 
-    // a thread per row: the row's kb entries are ld apart in its tile, and
-    // a warp's rows are adjacent (coalesced); 16 loads in flight
-    for (int r = tid; r < R; r += CL_THREADS) {
-        if (r >= nown) {
-            for (int c = 0; c < kb; c++) P[(size_t)c * R + r] = T(0);
-            continue;
+    // a row's kb entries are ld apart in its tile, and a warp's rows are
+    // adjacent (coalesced); 16 RPT loads in flight
+    int pos[RPT];                  // the row's position in the panel, -1 for none
+    int at[RPT];                   // its place in a column of P (in range for none)
+#pragma unroll
+    for (int q = 0; q < RPT; q++) {
+        const int r = q * CL_THREADS + tid;
+        pos[q] = r < nown ? row0 + r : -1;
+        at[q] = min(r, R - 1);
+    }
+    T v[RPT][CL_IB];
+    for (int c0 = 0; c0 < kb; c0 += CL_IB) {
+#pragma unroll
+        for (int q = 0; q < RPT; q++) {
+            if (pos[q] < 0) continue;
+            const T *src = panel_at<T>(A, k, pos[q], c0);
+            const int ld = plasma_tile_mmain(A, k + pos[q] / mb);
+#pragma unroll
+            for (int c = 0; c < CL_IB; c++) v[q][c] = c0 + c < kb ? src[(size_t)c * ld] : T(0);
         }
-        const T *src = panel_at<T>(A, k, row0 + r, 0);
-        const int ld = plasma_tile_mmain(A, k + (row0 + r) / mb);
-        for (int c0 = 0; c0 < kb; c0 += 16) {
-            T v[16];
 #pragma unroll
-            for (int q = 0; q < 16; q++) v[q] = c0 + q < kb ? src[(size_t)(c0 + q) * ld] : T(0);
+        for (int q = 0; q < RPT; q++) {
+            if (pos[q] < 0) continue;
 #pragma unroll
-            for (int q = 0; q < 16; q++)
-                if (c0 + q < kb) P[(size_t)(c0 + q) * R + r] = v[q];
+            for (int c = 0; c < CL_IB; c++)
+                if (c0 + c < kb) P[(size_t)(c0 + c) * RS + at[q]] = v[q][c];
         }
     }
-    __syncthreads();
 
     for (int s0 = 0; s0 < kb; s0 += CL_IB) {
         const int ce = min(kb, s0 + CL_IB);
-        // this thread's candidate for the next column: found by a scan at the
-        // start of a sub-block, then by each column's rank-1 update
-        T bv = T(-1);
-        int bi = INT_MAX;
-        for (int r = tid; r < nown; r += CL_THREADS)
-            if (row0 + r >= s0) max_pick(bv, bi, (T)fabs(P[(size_t)s0 * R + r]), row0 + r);
+#pragma unroll
+        for (int q = 0; q < RPT; q++)
+#pragma unroll
+            for (int c = 0; c < CL_IB; c++)
+                v[q][c] = pos[q] >= 0 && s0 + c < kb ? P[(size_t)(s0 + c) * RS + at[q]] : T(0);
+        // the columns in a loop, for a small body: v[q][0] is column j, and a
+        // step moves the entries down by one (what is moved in at the end is
+        // past the sub-block and never used)
+#pragma unroll 1
         for (int j = s0; j < ce; j++) {
             const int par = j & 1;
-            T *slot = pub_row + par * 2 * CL_KB;
-            // 1. this CTA's candidate for column j and its row
-            block_best(bv, bi, red_v, red_i);
-            if (tid == 0) {
-                pub_val[par] = bv;
-                pub_idx[par] = bi;
-                bi_s = bi;
-            }
-            __syncthreads();
-            const int cb = bi_s;
-            const int rj = j - row0;
-            for (int c = tid; c < kb; c += CL_THREADS) {
-                slot[c] = cb != INT_MAX ? P[(size_t)c * R + (cb - row0)] : T(0);
-                if (rj >= 0 && rj < nown) slot[CL_KB + c] = P[(size_t)c * R + rj];
-            }
-            cl_sync();
-            // 2. the pivot (first largest magnitude over the CTAs'
-            // candidates, warp 0) and, in the same round of remote reads,
-            // every CTA's candidate row and row j (a thread per column)
-            const int cj = j / R;
-            T cand[CL_CTAS];
-            if (tid < kb) {
+            // 1. this warp's candidate for column j, to every CTA
+            K bk = 0;
+            int bp = INT_MAX;
 #pragma unroll
-                for (int q = 0; q < CL_CTAS; q++)
-                    cand[q] = cl_ld(cl_addr(&slot[tid], (uint32_t)q), T(0));
-                rowj[tid] = cl_ld(cl_addr(&slot[CL_KB + tid], (uint32_t)cj), T(0));
+            for (int q = 0; q < RPT; q++) {
+                const K x = pivot_key(v[q][0]);
+                if (pos[q] >= j && (x > bk || (x == bk && pos[q] < bp))) { bk = x; bp = pos[q]; }
             }
+            const K wk = warp_max(bk);
+            const int wp = __reduce_min_sync(0xffffffffu, bk == wk ? bp : INT_MAX);
+            uint4 *o = out + warp * CHUNKS;
+            if (wp == INT_MAX) {                           // no row left in this warp
+                if (lane < CHUNKS) o[lane] = make_uint4(0, 0, INT_MAX, 0);
+            } else if (bp == wp) {
+#pragma unroll
+                for (int q = 0; q < RPT; q++)
+                    if (pos[q] == wp) {
+                        o[0] = make_uint4((uint32_t)wk, (uint32_t)((unsigned long long)wk >> 32),
+                                          wp, row0 + q * CL_THREADS + tid);
+                        st_row(reinterpret_cast<T *>(o + 1), v[q]);
+                    }
+            }
+            __syncwarp();
+            const int rec = par * 32 + (int)me * CL_WARPS + warp;
+#pragma unroll
+            for (int e0 = 0; e0 < CL_CTAS * CHUNKS; e0 += 32) {
+                const int e = e0 + lane, ch = e / CL_CTAS;
+                if (e < CL_CTAS * CHUNKS) {
+                    const void *to = ch == 0 ? (const void *)(rec_h + rec)
+                                             : (const void *)(rec_r + rec * CL_IB + (ch - 1) * V);
+                    cl_send(cl_addr(to, e % CL_CTAS), o[ch], cl_addr(&bar[par], e % CL_CTAS));
+                }
+            }
+            // 2. the pivot: the first largest of the cluster's candidates
+            const bool ok = mbar_wait(&bar[par], (j >> 1) & 1, &abort_s);
+            if (tid == 0 && ok && j + 2 < kb) mbar_expect_tx(&bar[par], TX);
+            __syncwarp();
+            const uint4 h = rec_h[par * 32 + lane];
+            const K ck = (K)((unsigned long long)h.y << 32 | h.x);
+            const K mk = warp_max(ck);
+            int p = __reduce_min_sync(0xffffffffu, ck == mk ? (int)h.z : INT_MAX);
+            const int w = __ffs(__ballot_sync(0xffffffffu, ck == mk && (int)h.z == p)) - 1;
+            p = max(j, min(p, M - 1));                     // in range also after a timeout
+            const T *pr = rec_r + (par * 32 + w) * CL_IB;
+            T u[CL_IB];
+            ld_row(pr, u);
+            // a column of NaNs counts as a zero pivot
+            const T piv = mk == 0 ? T(0) : u[0];
             if (warp == 0) {
-                T v = T(-1);
-                int i = INT_MAX;
-                if (lane < CL_CTAS) {
-                    v = cl_ld(cl_addr(&pub_val[par], lane), T(0));
-                    i = cl_ld_int(cl_addr(&pub_idx[par], lane));
+                const int from = __shfl_sync(0xffffffffu, (int)h.w, w);
+                if (lane == 0) place[j - s0] = max(0, min(from, M - 1));
+                // the pivot row's part of U in the sub-block (l11 holds it
+                // until the sub-block ends)
+                if (lane < CL_IB) l11[(j - s0) * CL_IB + lane] = pr[lane];
+                if (me == 0 && lane == 0) {
+                    ipiv[d0 + j] = d0 + p + 1;
+                    if (piv == T(0)) plasma_fail(st, d0 + j + 1, call);
                 }
+            }
+            // 3. the interchange, then the rows below j (a pivot row's
+            // registers are not used again)
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1)
-                    max_pick(v, i, __shfl_xor_sync(0xffffffffu, v, o),
-                             __shfl_xor_sync(0xffffffffu, i, o));
-                if (lane == 0) piv_s = i == INT_MAX ? j : i;   // a column of NaNs
-            }
-            __syncthreads();
-            const int p = piv_s;
-            const int cp = p / R;
-            // 3. the pivot row is the candidate row of p's owner
-            if (tid < kb) {
-                T x = cand[0];
+            for (int q = 0; q < RPT; q++) pos[q] = pos[q] == p ? j : pos[q] == j ? p : pos[q];
+            // LAPACK's dgetf2: a reciprocal unless the pivot is tiny
+            const T rp = T(1) / piv;
+            T l[RPT];
+            if ((T)fabs(piv) >= tiny<T>()) {
 #pragma unroll
-                for (int q = 1; q < CL_CTAS; q++)
-                    if (q == cp) x = cand[q];
-                prow[tid] = x;
+                for (int q = 0; q < RPT; q++) l[q] = v[q][0] * rp;
+            } else {
+                for (int q = 0; q < RPT; q++) l[q] = piv != T(0) ? v[q][0] / piv : v[q][0];
             }
-            __syncthreads();
-            const T piv = prow[j];
-            if (me == 0 && tid == 0) {
-                ipiv[d0 + j] = d0 + p + 1;
-                if (piv == T(0)) plasma_fail(st, d0 + j + 1, call);
+#pragma unroll
+            for (int q = 0; q < RPT; q++) {
+                if (pos[q] > j) P[(size_t)j * RS + at[q]] = l[q];
+                if (piv == T(0)) l[q] = T(0);
             }
-            // 4. the swap (a thread per column), then the rows below j:
-            // scaled, rank-1 update inside the sub-block, and the candidate
-            // for column j+1 on the way
-            if (p != j) {
-                for (int c = tid; c < kb; c += CL_THREADS) {
-                    if (cj == (int)me) P[(size_t)c * R + (j - row0)] = prow[c];
-                    if (cp == (int)me) P[(size_t)c * R + (p - row0)] = rowj[c];
-                }
-                __syncthreads();
-            }
-            const bool rcp = (T)fabs(piv) >= tiny<T>();
-            const T rp = piv != T(0) ? T(1) / piv : T(0);
-            bv = T(-1);
-            bi = INT_MAX;
-            for (int r = tid; r < nown; r += CL_THREADS) {
-                const int pr = row0 + r;
-                if (pr <= j) continue;
-                if (piv != T(0)) {
-                    // LAPACK's dgetf2: a reciprocal unless the pivot is tiny
-                    T *lr = &P[(size_t)j * R + r];
-                    const T l = rcp ? *lr * rp : *lr / piv;
-                    *lr = l;
-                    for (int c = j + 1; c < ce; c++) P[(size_t)c * R + r] -= l * prow[c];
-                }
-                if (j + 1 < ce)
-                    max_pick(bv, bi, (T)fabs(P[(size_t)(j + 1) * R + r]), pr);
+            if (piv == T(0))
+#pragma unroll
+                for (int c = 1; c < CL_IB; c++) u[c] = T(0);
+#pragma unroll
+            for (int q = 0; q < RPT; q++) {
+#pragma unroll
+                for (int c = 1; c < CL_IB; c++) v[q][c - 1] = v[q][c] - l[q] * u[c];
+                v[q][CL_IB - 1] = T(0);
             }
         }
         __syncthreads();
+        for (int e = tid; e < CL_IB * CL_IB; e += CL_THREADS) {
+            const int i = e / CL_IB, c = i + e % CL_IB;
+            if (i % CL_CTAS == (int)me && s0 + c < ce)
+                *panel_at<T>(A, k, s0 + i, s0 + c) = l11[e];
+        }
         if (ce >= kb) break;
-        // 5. the sub-block's rows to every CTA, U12 = L11^-1 A12, A22 -= L21 U12
-        const int nsb = ce - s0;
-        for (int e = tid; e < nsb * kb; e += CL_THREADS) {
-            const int i = e / kb, c = e % kb, r = s0 + i - row0;
-            if (r >= 0 && r < nown) blk[i * CL_KB + c] = P[(size_t)c * R + r];
-        }
+        // 4. the pivot rows' multipliers and other columns, U12 = L11^-1 A12
+        // (a thread per column), A22 -= L21 U12; a row that was a pivot stays
+        // as it is, so the reads need no second barrier
+        const int nc = kb - ce;
         cl_sync();
-        for (int e = tid; e < nsb * kb; e += CL_THREADS) {
-            const int i = e / kb, c = e % kb;
-            u12[i * CL_KB + c] = cl_ld(cl_addr(&blk[i * CL_KB + c], (uint32_t)((s0 + i) / R)),
-                                       T(0));
+        constexpr int PULL = CL_KB * CL_IB / CL_THREADS;
+        T x[PULL];
+#pragma unroll
+        for (int e = 0; e < PULL; e++) {
+            const int i = (e * CL_THREADS + tid) % CL_IB, c = (e * CL_THREADS + tid) / CL_IB;
+            const int g = place[i];
+            x[e] = T(0);
+            if (s0 + c < kb && (c >= CL_IB || c < i))
+                x[e] = cl_ld(cl_addr(&P[(size_t)(s0 + c) * RS + g % R], g / R), T(0));
+        }
+#pragma unroll
+        for (int e = 0; e < PULL; e++) l11[e * CL_THREADS + tid] = x[e];   // and u12 after it
+        __syncthreads();
+        if (tid < nc) {
+            T y[CL_IB];
+            ld_row(u12 + tid * CL_IB, y);
+#pragma unroll
+            for (int q = 0; q < CL_IB; q++) {
+                T lq[CL_IB];                               // column q of L11
+                ld_row(l11 + q * CL_IB, lq);
+#pragma unroll
+                for (int i = q + 1; i < CL_IB; i++) y[i] -= lq[i] * y[q];
+            }
+            st_row(u12 + tid * CL_IB, y);
+#pragma unroll
+            for (int i = 0; i < CL_IB; i++)
+                if (i % CL_CTAS == (int)me) *panel_at<T>(A, k, s0 + i, ce + tid) = y[i];
         }
         __syncthreads();
-        for (int c = ce + tid; c < kb; c += CL_THREADS) {
-            for (int i = 1; i < nsb; i++) {
-                T v = u12[i * CL_KB + c];
-                for (int q = 0; q < i; q++) v -= u12[i * CL_KB + s0 + q] * u12[q * CL_KB + c];
-                u12[i * CL_KB + c] = v;
-            }
+#pragma unroll
+        for (int q = 0; q < RPT; q++)
+#pragma unroll
+            for (int c = 0; c < CL_IB; c++) v[q][c] = P[(size_t)(s0 + c) * RS + at[q]];
+#pragma unroll 2
+        for (int c = 0; c < nc; c++) {
+            T u[CL_IB], y[RPT];
+            ld_row(u12 + c * CL_IB, u);
+            T *pc = P + (size_t)(ce + c) * RS;
+#pragma unroll
+            for (int q = 0; q < RPT; q++) y[q] = pc[at[q]];
+#pragma unroll
+            for (int i = 0; i < CL_IB; i++)
+#pragma unroll
+                for (int q = 0; q < RPT; q++) y[q] -= v[q][i] * u[i];
+#pragma unroll
+            for (int q = 0; q < RPT; q++)
+                if (pos[q] >= ce) pc[at[q]] = y[q];
         }
-        __syncthreads();
-        // rows pr >= ce take A22 -= L21 U12 (nsb = CL_IB here), two rows of
-        // a thread at a time so each U12 entry read serves both
-        for (int r = tid; r < nown; r += 2 * CL_THREADS) {
-            const int r2 = r + CL_THREADS;
-            T l[2][CL_IB];
-            bool on[2];
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int rr = h ? r2 : r, pr = row0 + rr;
-                on[h] = rr < nown && pr >= ce;
-                if (rr < nown && pr >= s0 && pr < ce)
-                    for (int c = ce; c < kb; c++)
-                        P[(size_t)c * R + rr] = u12[(pr - s0) * CL_KB + c];
-#pragma unroll
-                for (int q = 0; q < CL_IB; q++)
-                    l[h][q] = on[h] ? P[(size_t)(s0 + q) * R + rr] : T(0);
-            }
-            if (!on[0] && !on[1]) continue;
-            for (int c = ce; c < kb; c++) {
-                T v0 = on[0] ? P[(size_t)c * R + r] : T(0);
-                T v1 = on[1] ? P[(size_t)c * R + r2] : T(0);
-#pragma unroll
-                for (int q = 0; q < CL_IB; q++) {
-                    const T u = u12[q * CL_KB + c];
-                    v0 -= l[0][q] * u;
-                    v1 -= l[1][q] * u;
-                }
-                if (on[0]) P[(size_t)c * R + r] = v0;
-                if (on[1]) P[(size_t)c * R + r2] = v1;
-            }
-        }
-        __syncthreads();
     }
-    for (int r = tid; r < nown; r += CL_THREADS) {
-        T *dst = panel_at<T>(A, k, row0 + r, 0);
-        const int ld = plasma_tile_mmain(A, k + (row0 + r) / mb);
-        for (int c = 0; c < kb; c++) dst[(size_t)c * ld] = P[(size_t)c * R + r];
+    // a pivot row's part of U is written
+#pragma unroll
+    for (int q = 0; q < RPT; q++) {
+        if (pos[q] < 0) continue;
+        const int lim = min(kb, pos[q]);
+        T *dst = panel_at<T>(A, k, pos[q], 0);
+        const int ld = plasma_tile_mmain(A, k + pos[q] / mb);
+        for (int c = 0; c < lim; c++)
+            dst[(size_t)c * ld] = P[(size_t)c * RS + at[q]];
+    }
+    if (abort_s && tid == 0) {
+        plasma_fail(st, PlasmaErrorInternal, 0);
+        // a bounded time for the copies still under way
+        for (int i = 0; i < 1000; i++) __nanosleep(1000);
     }
     // no CTA leaves while another may still read its shared memory
     cl_sync();
@@ -956,18 +1075,34 @@ template <typename T> bool panel_cluster_ok(int kb, int M)
     return kb <= CL_KB && (M + CL_CTAS - 1) / CL_CTAS <= ClLayout<T>::MAX_R;
 }
 
+template <typename T, int RPT>
+void panel_cluster(cudaStream_t s, plasma_devstat_t *st, int call, plasma_desc_t A, int k,
+                   int kb, int R, int *ipiv)
+{
+    const size_t smem = (size_t)CL_KB * (R | 1) * sizeof(T) + ClLayout<T>::EXTRA;
+    static unsigned long long attr = 0;
+    if (plasma_first_on_device(&attr))
+        cudaFuncSetAttribute(k_lu_panel_cl<T, RPT>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             ClLayout<T>::MAX_SMEM);
+    PLASMA_COUNT_LAUNCH();
+    k_lu_panel_cl<T, RPT><<<CL_CTAS, CL_THREADS, smem, s>>>(A, k, kb, R, ipiv, st, call);
+}
+
+// rows a thread: the fewest that hold the CTA's R
 template <typename T>
 void panel_cluster(cudaStream_t s, plasma_devstat_t *st, int call, plasma_desc_t A, int k,
                    int kb, int M, int *ipiv)
 {
     const int R = (M + CL_CTAS - 1) / CL_CTAS;
-    const size_t smem = (size_t)CL_KB * R * sizeof(T) + ClLayout<T>::EXTRA;
-    static unsigned long long attr = 0;
-    if (plasma_first_on_device(&attr))
-        cudaFuncSetAttribute(k_lu_panel_cl<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             ClLayout<T>::MAX_SMEM);
-    PLASMA_COUNT_LAUNCH();
-    k_lu_panel_cl<T><<<CL_CTAS, CL_THREADS, smem, s>>>(A, k, kb, R, ipiv, st, call);
+    if (R <= CL_THREADS)
+        panel_cluster<T, 1>(s, st, call, A, k, kb, R, ipiv);
+    else if (R <= 2 * CL_THREADS)
+        panel_cluster<T, 2>(s, st, call, A, k, kb, R, ipiv);
+    else if (R <= 4 * CL_THREADS)
+        panel_cluster<T, 4>(s, st, call, A, k, kb, R, ipiv);
+    else
+        panel_cluster<T, ClLayout<T>::MAX_RPT>(s, st, call, A, k, kb, R, ipiv);
 }
 }  // namespace
 

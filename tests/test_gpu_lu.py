@@ -194,3 +194,61 @@ def test_dsgesv_fp64_lu_mixed_panels(L):
     assert info == 0 and it == -31
     assert valid_pivots(piv, n)
     assert solve_residual(a, x, b) < TOL * EPS
+
+
+# the one-launch panel at the ends of its ranges: column blocks of 16, 128-row
+# groups a CTA (n / 8 rows each), rows that are no multiple of the cluster
+@pytest.mark.parametrize("n", [15, 16, 17, 63, 65, 130, 1024, 1025, 2048, 2056, 4097])
+def test_panel_pivots(L, n):
+    """The interchanges of the FP32 factor are partial pivoting: in the exact
+    (FP64) elimination of the interchanged rows no candidate exceeds the pivot
+    by more than the two entries' FP32 errors, each at most n u max|U|, u the
+    FP32 unit roundoff -- |l_ij| <= 1 + 2 n u max|U| / |u_jj|."""
+    set_nb(L, 64)
+    rng = np.random.default_rng(n)
+    a, b = rng.standard_normal((n, n)), rng.standard_normal((n, 2))
+    info, it, x, piv = dsgesv(L, a, b)
+    assert info == 0 and it >= 0
+    assert valid_pivots(piv, n)
+    rows = np.arange(n)
+    for j in range(n):
+        rows[[j, piv[j] - 1]] = rows[[piv[j] - 1, j]]
+    lu = torch.linalg.lu_factor(torch.from_numpy(a[rows]).cuda(), pivot=False)[0]
+    d, umax = lu.diagonal().abs(), lu.triu().abs().max()
+    bound = 1 + 2 * n * 2.0 ** -24 * umax / d
+    assert bool((lu.tril(-1).abs() <= bound[None, :]).all())
+    assert solve_residual(a, x, b) < TOL * EPS
+
+
+@pytest.mark.parametrize("n,nb", [(100, 64), (100, 16), (1100, 64)])
+def test_panel_ties(L, n, nb):
+    """Among equal magnitudes the first row is the pivot (idamax).  A = [I 0; S I]
+    with entries +-1 in S: each column's candidates all have magnitude 1, the
+    elimination is exact, and no row moves."""
+    set_nb(L, nb)
+    rng = np.random.default_rng(n)
+    h = n // 2
+    lo = np.eye(n)
+    lo[h:, :h] = rng.choice([-1.0, 1.0], (n - h, h))
+    b = rng.standard_normal((n, 1))
+    info, it, x, piv = dsgesv(L, lo, b)
+    assert info == 0
+    np.testing.assert_array_equal(piv, np.arange(1, n + 1))
+
+
+@pytest.mark.parametrize("n,nb", [(100, 64), (300, 64), (300, 16)])
+def test_interchanges_compose(L, n, nb):
+    """A permutation matrix of a given order: the pivots are the swaps that
+    undo it, and A x = b is a gather."""
+    set_nb(L, nb)
+    perm = np.random.default_rng(n).permutation(n)
+    a = np.zeros((n, n))
+    a[np.arange(n), perm] = 2.0
+    b = np.arange(1.0, n + 1)[:, None]
+    info, it, x, piv = dsgesv(L, a, b)
+    assert info == 0
+    np.testing.assert_array_equal(x[perm, 0], b[:, 0] / 2)
+    rows = np.arange(n)
+    for j in range(n):
+        rows[[j, piv[j] - 1]] = rows[[piv[j] - 1, j]]
+    np.testing.assert_array_equal(perm[rows], np.arange(n))
