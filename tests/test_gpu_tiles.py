@@ -159,3 +159,45 @@ def test_fp32_ragged(L, n, nb):
         low = low if uplo == LO else low.T
         assert np.linalg.norm(low @ low.T - a) <= TOL * n * SEPS * np.linalg.norm(a)
         np.testing.assert_array_equal(other(f, k), other(a.astype(np.float32), k))
+
+
+# FP64 steps with 3072 trailing rows or more update from integer digits: one
+# and a few such steps, tile orders 128 and 256, a ragged last tile, and rows
+# whose scales differ by up to 2^400.  Backward error of any Cholesky
+# factorization with products summed to n terms (Higham, Accuracy and
+# Stability, theorem 10.3), entry by entry: |A - L L^T| <= (n + 1) u |L| |L^T|,
+# whose (i, j) entry is at most sqrt(a_ii a_jj); the check's own product takes
+# as much again.
+@pytest.mark.parametrize("n,nb,spread", [(3328, 256, 0), (3329, 256, 0), (3585, 128, 0),
+                                         (3500, 256, 400)])
+@pytest.mark.parametrize("uplo", [LO, UP])
+def test_digit_update(L, n, nb, spread, uplo):
+    a = gen.likelihood(n, 1, seed=n)[0]
+    d = 2.0 ** np.random.default_rng(n).integers(-spread // 2, spread // 2 + 1, n)
+    info, f = potrf(L, a * d[:, None] * d[None, :], nb, uplo=uplo)
+    assert info == 0
+    lf = (np.tril(f) if uplo == LO else np.triu(f).T) / d[:, None]
+    s = np.sqrt(np.diag(a))
+    err = np.abs(lf @ lf.T - a) / (s[:, None] * s[None, :])
+    assert err.max() <= 2 * (n + 1) * EPS / 2
+
+
+@pytest.mark.parametrize("bad", [-1.0, np.nan])
+@pytest.mark.parametrize("col", [100, 300, 3200])
+def test_digit_update_info(L, col, bad):
+    a = gen.likelihood(3400, 1, seed=9)[0]
+    a[col, col] = bad
+    info, _ = potrf(L, a, 256)
+    assert info == col + 1
+
+
+# the right-hand sides' kept tiles: larger and smaller systems in turn
+def test_sizes_in_turn(L):
+    assert L.plasma_set(pb.PlasmaNb, 64) == 0
+    for n, nrhs in [(300, 3), (40, 1), (700, 70), (65, 2), (700, 71), (300, 3)]:
+        a, b = gen.likelihood(n, nrhs, seed=n + nrhs)
+        for dtype, eps, fn in ((np.float64, EPS, L.plasma_dposv), (np.float32, SEPS, L.plasma_sposv)):
+            af, x = np.asfortranarray(a.astype(dtype)), np.asfortranarray(b.astype(dtype))
+            assert fn(LO, n, nrhs, af.ctypes.data, n, x.ctypes.data, n) == 0
+            r = np.abs(a @ x.astype(np.float64) - b).max()
+            assert r <= TOL * eps * n * np.abs(a).sum(1).max() * np.abs(x).max()
