@@ -74,7 +74,7 @@ def parse():
 METRIC = ("dsposv vs dposv time-to-FP64-backward-err at n=32768 on 1 B200; "
           "GFLOP/s, % roofline")
 MODES = {"fp32": 0, "tf32": 1, "bf16": 2, "auto": 3}
-UPDATE_DRAM_BYTES_PER_TILE = {"fp32": 384465}
+UPDATE_DRAM_BYTES_PER_TILE = {"fp32": 365605}
 REFINE = {"ir": 0, "gmres": 1, "auto": 2}
 
 
@@ -731,7 +731,7 @@ def _dsposv_cell(L, pb, A, B, X, xt, n, nrhs, mode, refine, steps, warmup):
 
 def run_mixed(args):
     """The mixed-precision configuration in full: kappa in {1e2, 1e5, 1e8} x
-    factor precision in {FP32 (three TF32 products), TF32, BF16}, each refined
+    factor precision in {FP32 (three FP16 products), TF32, BF16}, each refined
     by IR for kappa <= 1e5 and by GMRES-IR for kappa = 1e8, at n = --n
     (32768), nrhs = 1, on device-resident operands.  Per cell: info, iter,
     the report of plasma_dsposv_ex (factor precision used, attempts, GMRES
@@ -1104,14 +1104,15 @@ def main():
 
     upd = prof["update"]
     # all factor modes run the trailing update on the tcgen05 tensor cores;
-    # fp32 forms every FP32 product as three TF32 products (lo*hi + hi*lo +
-    # hi*hi), so its tensor work is three times the algorithmic flops
-    mode_peak = {"fp32": ("tf32", peaks.get("tf32"), 3), "tf32": ("tf32", peaks.get("tf32"), 1),
+    # fp32 forms every FP32 product as three FP16 products (lo*hi + hi*lo +
+    # hi*hi), so its tensor work is three times the algorithmic flops; FP16
+    # runs at the BF16 rate
+    mode_peak = {"fp32": ("bf16", peaks.get("bf16"), 3), "tf32": ("tf32", peaks.get("tf32"), 1),
                  "bf16": ("bf16", peaks.get("bf16"), 1), "auto": ("bf16", peaks.get("bf16"), 1)}
     pk_name, pk, passes = mode_peak[args.mode]
     achieved = passes * upd["flops"] / upd["ms"] / 1e9 if upd["ms"] > 0 else None
     # DRAM bytes per 256 x 256 tile-update of the CTA-pair update kernel, read
-    # + write, from one ncu capture (profiles/k_update_pair_tf32x3_n8192.md: a
+    # + write, from one ncu capture (profiles/k_update_pair_fp16x3_n8192.md: a
     # bulk launch of 325 tile-updates); a launch's traffic grows with the
     # tiles it updates
     # (the algorithmic C read + write is 524288 bytes per tile-update)
@@ -1142,7 +1143,7 @@ def main():
                      "tensor_products_per_flop": passes,
                      "achieved_algorithmic": (achieved / passes) if achieved else None,
                      "peak_source": f"{pk_name} cuBLAS GEMM measured live (of measured)"
-                     if pk_name != "bf16" else "MEASURED_PEAKS.json bf16_tflops (of measured)",
+                     if pk_name != "bf16" else f"bf16_tflops of {peaks.get('source')}",
                      "traffic": traffic, "traffic_unit": "bytes per launch",
                      "launches": upd["launches"],
                      "avg_launch_ms": upd["ms"] / max(1, upd["launches"])},
