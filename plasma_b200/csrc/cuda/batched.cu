@@ -27,7 +27,7 @@
 //       tensor work on the same scheduler doubles the time of a pivot.
 // 4096 systems, n in [16, 512], FP64 factor and solve: 8.1 ms a call with the
 // diagonal blocks factored and inverted by one warp, 6.6 ms in this form; the
-// FP32 gradient of 1024 systems 15.4 -> 5.2 ms.
+// FP32 gradient of 1024 systems 15.4 -> 5.3 ms.
 // The solve follows in the same CTA while the factor is in L2: forward by
 // block (diagonal block by one warp, the rows below by all threads),
 // backward by block (column dot products by warps, then the diagonal block).
