@@ -144,6 +144,8 @@ __device__ __forceinline__ bool blk_factor(T *S, T *W8)
             v[j] = S[pd_at(o + j, lane)];
             u[j] = lane == j ? T(1) : T(0);
         }
+        // every lane has read the diagonal block before its rows are written
+        __syncwarp();
 #pragma unroll
         for (int c = 0; c < 8; c++) {
             const T d = a[c][c];
