@@ -924,7 +924,7 @@ k_lu_panel_cl(plasma_desc_t A, int k, int kb, int R, int *ipiv, plasma_devstat_t
                 }
             }
             // 2. the pivot: the first largest of the cluster's candidates
-            const bool ok = mbar_wait(&bar[par], (j >> 1) & 1, &abort_s);
+            const bool ok = mbar_wait_cluster(&bar[par], (j >> 1) & 1, &abort_s);
             if (tid == 0 && ok && j + 2 < kb) mbar_expect_tx(&bar[par], TX);
             __syncwarp();
             const uint4 h = rec_h[par * 32 + lane];

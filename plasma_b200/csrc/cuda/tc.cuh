@@ -54,6 +54,34 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity,
     return true;
 }
 
+__device__ __forceinline__ bool mbar_try_cluster(uint64_t *bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
+
+// The same with cluster-scope acquire, for barriers on which other CTAs of the
+// cluster arrive or complete their writes: the default scope is this CTA, and
+// would not order reads of what the others wrote.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity,
+                                                  volatile int *abort_flag)
+{
+    long long t0 = clock64();
+    while (!mbar_try_cluster(bar, parity)) {
+        if (*abort_flag) return false;
+        if (clock64() - t0 > 4000000000LL) {
+            *abort_flag = 1;
+            return false;
+        }
+    }
+    return true;
+}
+
 __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map,
                                             uint64_t *bar, int c0, int c1, int c2,
                                             int c3)

@@ -439,33 +439,6 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr)
                  :: "r"(cluster_addr) : "memory");
 }
 
-__device__ __forceinline__ bool mbar_try_cluster(uint64_t *bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return ok != 0;
-}
-
-// Bounded wait with cluster-scope acquire (barriers that CTAs of the pair
-// arrive on): false after ~2 s or when this CTA already gave up.
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity,
-                                                  volatile int *abort_flag)
-{
-    long long t0 = clock64();
-    while (!mbar_try_cluster(bar, parity)) {
-        if (*abort_flag) return false;
-        if (clock64() - t0 > 4000000000LL) {
-            *abort_flag = 1;
-            return false;
-        }
-    }
-    return true;
-}
-
 // TMA load into this CTA's shared memory whose completion is counted on the
 // barrier at shared::cluster address `bar` (the leader's)
 __device__ __forceinline__ void tma_load_4d_pair(void *dst, const CUtensorMap *map,
