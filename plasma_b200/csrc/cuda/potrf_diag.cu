@@ -105,7 +105,8 @@ k_potrf_diag_f64(plasma_desc_t A, int k, int iinfo, plasma_devstat_t *st, int ca
     __shared__ double rdiag[32], W8[32 * 8];
     __shared__ int bad_s;
     __shared__ int task_s[2 * PD_NMAX / 32];   // next task of every step
-    if (plasma_failed(st)) return;
+    // one answer for the whole block, as its warps wait for one another
+    if (__syncthreads_or(plasma_failed(st))) return;
     double *T = (double *)plasma_tile_addr(A, k, k);
     const int ld = plasma_tile_mmain(A, k);
     const int n = plasma_tile_mview(A, k);

@@ -245,7 +245,8 @@ k_update_i8(I8Args g, plasma_devstat_t *st)
     __shared__ uint64_t bfull_bar[I8_NBMAX / I8_KB], bempty_bar, tfull_bar, tempty_bar;
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_s;
-    if (plasma_failed(st)) return;
+    // one answer for the whole block, as its warps wait for one another
+    if (__syncthreads_or(plasma_failed(st))) return;
     const int first = blockIdx.x * g.ipc;
     const int nit = min(g.ipc, g.nitems - first);
     if (nit <= 0) return;

@@ -195,7 +195,8 @@ k_update_tc(const __grid_constant__ CUtensorMap opmap,
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_s;
 
-    if (plasma_failed(st)) return;
+    // one answer for the whole block, as its warps wait for one another
+    if (__syncthreads_or(plasma_failed(st))) return;
     const long long first = (long long)blockIdx.x * g.ipc;
     if (first >= g.nitems) return;
     const int nit = (int)min((long long)g.ipc, g.nitems - first);

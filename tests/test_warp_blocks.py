@@ -1,5 +1,7 @@
-"""The one-warp block factors of f64_blocks.cuh under every order in which the
-hardware may run a warp's lanes between two warp barriers.
+"""Synchronisation inside a block, without a GPU: the one-warp block factors of
+f64_blocks.cuh under every order in which the hardware may run a warp's lanes
+between two warp barriers, and how kernels with warps in different roles read
+the failure status.
 
 Lanes of a warp need not advance together (independent thread scheduling), so
 shared memory that one lane writes and another reads has to be separated by a
@@ -178,3 +180,23 @@ def test_lane_orders(warp, dtype, nb, general, how):
     for q in range(nb // 8):
         inv = np.linalg.inv(ref[8 * q:8 * q + 8, 8 * q:8 * q + 8])
         assert np.abs(w8[8 * q:8 * q + 8].T - inv).max() <= 64 * nb * eps
+
+
+def test_status_is_read_once_per_block():
+    """The status word may change while a kernel starts: a pivot that fails on
+    one stream does so beside updates on others.  Where the warps of a block
+    wait for one another (mbarriers, named barriers), they must all follow one
+    reading, or those that go on wait for those that left."""
+    bare = re.compile(r"if \(plasma_failed\(st\)\) return;")
+    roles = re.compile(r"mbar_wait|\"bar\.sync")
+    wrong = []
+    cuda = os.path.dirname(HEADER)
+    for name in sorted(os.listdir(cuda)):
+        if not name.endswith(".cu"):
+            continue
+        text = open(os.path.join(cuda, name)).read()
+        for m in re.finditer(r"__global__[^;{]*?\b(k_\w+)\(", text):
+            body = definition(text[m.start():], "__global__")
+            if roles.search(body) and bare.search(body):
+                wrong.append(f"{name}: {m.group(1)}")
+    assert not wrong
