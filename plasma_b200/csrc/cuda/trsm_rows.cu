@@ -192,6 +192,9 @@ k_trsm_rows_f64(plasma_desc_t A, int uplo, int backward, const double *W, plasma
                     }
                 }
                 if (!ok) break;
+                // the flags were read by single lanes: order the copies of all
+                // lanes after that (a vote does not)
+                __syncwarp();
                 const int s = s0 + j, k = backward ? nblk - 1 - s : s;
                 const int kr = min(RW_SB, n - k * RW_SB);
                 const int sl = (step0 + j) % RW_RING;
