@@ -361,7 +361,6 @@ static void upload_and_factor(plasma_context_t *plasma, const upload_t *up,
         plasma_request_fail(sequence, request, PlasmaErrorOutOfMemory);
         return;
     }
-    #pragma omp parallel for schedule(static)
     for (int i = 0; i < As.gm; i++)
         diag[i] = i < n ? (float)up->pA[(size_t)i * up->lda + i] : 1.0f;
     plasma_pXpotrf_arrivals(plasma, PlasmaLower, As, sequence, request, call, mode, ng,

@@ -27,6 +27,7 @@
 #include "../internal.h"
 
 #include <cuda_runtime_api.h>
+#include <omp.h>
 #include <stdint.h>
 #include <stdlib.h>
 #include <string.h>
@@ -81,6 +82,17 @@ static void copy_bytes(char *d, const char *s, size_t bytes)
     memcpy(d, s, bytes);
 }
 
+/* The threads of a chunk's copy: all but two.  The calling thread waits for
+ * the device in a spinning loop, and the thread that runs the host functions
+ * is CUDA's own; a team as large as the machine shares a CPU with one of
+ * them, and every chunk then waits at the team's barrier for the thread that
+ * is off its CPU until the scheduler's next turn. */
+static int stage_threads(void)
+{
+    const int n = omp_get_max_threads() - 2;
+    return n > 1 ? n : 1;
+}
+
 /* One chunk between the user's array and a slot, split into segments of
  * STAGE_SEGMENT bytes of one column each, spread over the OpenMP threads;
  * frees its job. */
@@ -89,7 +101,7 @@ static void CUDART_CB stage_run(void *p)
     stage_job_t *j = (stage_job_t *)p;
     const size_t segs = (j->width + STAGE_SEGMENT - 1) / STAGE_SEGMENT;
     const long total = (long)(segs * j->height);
-    #pragma omp parallel for schedule(static)
+    #pragma omp parallel for schedule(static) num_threads(stage_threads())
     for (long t = 0; t < total; t++) {
         const size_t c = (size_t)t / segs;
         const size_t o = ((size_t)t % segs) * STAGE_SEGMENT;
