@@ -321,7 +321,12 @@ static void upload_and_factor(plasma_context_t *plasma, const upload_t *up,
     plasma_pXpotrf_reserve(plasma, PlasmaLower, As, mode, 1);
     double *stage = (double *)plasma_scratch(plasma, PLASMA_SLOT_STAGING,
                                              (size_t)n * (size_t)n * sizeof(double));
-    if (stage == NULL) {
+    /* the walk scales panel rows by the diagonal before its columns are in.
+     * Allocated before the first copy as well: after a failure nothing may
+     * read the caller's arrays any more */
+    float *diag = (float *)malloc((size_t)As.gm * sizeof(float));
+    if (stage == NULL || diag == NULL) {
+        free(diag);
         plasma_request_fail(sequence, request, PlasmaErrorOutOfMemory);
         return;
     }
@@ -355,12 +360,6 @@ static void upload_and_factor(plasma_context_t *plasma, const upload_t *up,
     }
     plasma_cuda_lansy_inf(cp, plasma->dquiet, PlasmaLower, A, d_anorm, symv_work);
     cudaEventRecord(plasma->ev[5], cp);
-    /* the walk scales panel rows by the diagonal before its columns are in */
-    float *diag = (float *)malloc((size_t)As.gm * sizeof(float));
-    if (diag == NULL) {
-        plasma_request_fail(sequence, request, PlasmaErrorOutOfMemory);
-        return;
-    }
     for (int i = 0; i < As.gm; i++)
         diag[i] = i < n ? (float)up->pA[(size_t)i * up->lda + i] : 1.0f;
     plasma_pXpotrf_arrivals(plasma, PlasmaLower, As, sequence, request, call, mode, ng,
@@ -533,6 +532,12 @@ static void Xdsposv(plasma_context_t *plasma, plasma_enum_t uplo,
         RF.dscale = NULL;
         if (a == 0 && up != NULL && !up->on_device) {
             upload_and_factor(plasma, up, A, As, d_anorm, sw, call, mode, sequence, request);
+            if (sequence->status != PlasmaSuccess) {     /* no memory: nothing was read */
+                if (rep) {
+                    cudaEventDestroy(e0); cudaEventDestroy(e1); cudaEventDestroy(e2);
+                }
+                return;
+            }
             cudaMemcpyAsync(&Anorm, d_anorm, sizeof(double), cudaMemcpyDeviceToHost, S);
             fstatus = take_status(plasma);
             factor_failed = fstatus != 0;

@@ -61,3 +61,46 @@ def test_pageable_keeps_pace(policy):
         """, env)
     pageable, locked = map(float, out.split())
     assert pageable <= 4 * locked
+
+
+def test_no_host_memory(tmp_path):
+    """dsposv out of host memory reports it before it has enqueued a copy of
+    the caller's matrix: what still read the arrays after the call failed
+    would show as launches of the upload's kernels (one per column group)."""
+    shim = tmp_path / "shim.c"
+    shim.write_text("""
+        #include <errno.h>
+        #include <stddef.h>
+        extern void *__libc_malloc(size_t);
+        static size_t refuse;
+        void refuse_malloc(size_t n) { refuse = n; }
+        size_t refusal_left(void) { return refuse; }
+        void *malloc(size_t n)
+        {
+            if (n != 0 && n == refuse) { refuse = 0; errno = ENOMEM; return NULL; }
+            return __libc_malloc(n);
+        }
+        """)
+    so = tmp_path / "shim.so"
+    subprocess.run(["gcc", "-shared", "-fPIC", "-fno-builtin", "-o", str(so), str(shim)],
+                   check=True)
+    child("""
+        n, nb = 5000, 192
+        L.plasma_set(pb.PlasmaTuning, pb.PlasmaDisabled)
+        L.plasma_set(pb.PlasmaNb, nb)
+        a = np.full((n, n), 0.25) + n * np.eye(n)
+        b, x, it = np.ones((1, n)), np.zeros((1, n)), ct.c_int()
+        def solve():
+            return L.plasma_dsposv(pb.PlasmaLower, n, 1, a.ctypes.data, n, b.ctypes.data, n,
+                                   x.ctypes.data, n, ct.byref(it))
+        assert solve() == 0
+        self = ct.CDLL(None)
+        self.refuse_malloc.argtypes, self.refusal_left.restype = [ct.c_size_t], ct.c_size_t
+        before = L.plasma_kernel_launches()
+        self.refuse_malloc(4 * ((n + nb - 1) // nb * nb))       # one float a row
+        rc = solve()
+        assert self.refusal_left() == 0
+        assert rc == pb.PlasmaErrorOutOfMemory, rc
+        assert L.plasma_kernel_launches() - before < 10
+        assert solve() == 0 and np.abs(x @ a - b).max() < 1e-12
+        """, {"LD_PRELOAD": str(so)})
