@@ -42,7 +42,9 @@ def test_pageable_keeps_pace(policy):
     out = child("""
         n = 4100
         a = np.full((n, n), 0.25) + n * np.eye(n)
-        pin = torch.from_numpy(a.copy()).pin_memory()
+        # (numpy only: a parallel region of torch on this thread is another team,
+        # and the runtime waits in another way once there are two)
+        pin = torch.empty(n, n, dtype=torch.float64, pin_memory=True).numpy()
         def best(make):
             t = []
             for _ in range(6):
@@ -55,8 +57,8 @@ def test_pageable_keeps_pace(policy):
             x = a.copy()
             return x, x.ctypes.data
         def locked():
-            pin.copy_(torch.from_numpy(a))
-            return pin, pin.data_ptr()
+            pin[...] = a
+            return pin, pin.ctypes.data
         print(best(pageable), best(locked))
         """, env)
     pageable, locked = map(float, out.split())
