@@ -269,12 +269,15 @@ static int Xpotrf_adjoint(plasma_enum_t prec, plasma_enum_t uplo, int n,
     if (n == 0)
         return PlasmaSuccess;
     const int nb = plasma->nb;
+    const plasma_kept_t kept = plasma_kept_sizes(plasma);
     plasma_desc_t L, Lbar;
     int rc = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_A, prec, PlasmaGeneral, nb, n, n, &L);
     if (rc == PlasmaSuccess)
         rc = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_AS, prec, PlasmaGeneral, nb, n, n, &Lbar);
-    if (rc != PlasmaSuccess)
+    if (rc != PlasmaSuccess) {
+        plasma_kept_trim(plasma, &kept);
         return rc;
+    }
     plasma_sequence_t sequence;
     plasma_request_t request;
     plasma_sequence_init(&sequence);
@@ -285,6 +288,7 @@ static int Xpotrf_adjoint(plasma_enum_t prec, plasma_enum_t uplo, int n,
     plasma_sequence_wait(&sequence);
     plasma_omp_Xdesc2lapack(Lbar, pLbar, ldlbar, PlasmaGeneral, &sequence, &request);
     plasma_sequence_wait(&sequence);
+    plasma_kept_trim(plasma, &kept);
     return sequence.status;
 }
 
@@ -328,6 +332,7 @@ static int Xpotrs_adjoint(plasma_enum_t prec, plasma_enum_t uplo, int n, int nrh
     if (imin(n, nrhs) == 0)
         return PlasmaSuccess;
     const int nb = plasma->nb;
+    const plasma_kept_t kept = plasma_kept_sizes(plasma);
     plasma_desc_t L, X, Xbar, Lbar;
     int rc = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_A, prec, PlasmaGeneral, nb, n, n, &L);
     if (rc == PlasmaSuccess)
@@ -336,8 +341,10 @@ static int Xpotrs_adjoint(plasma_enum_t prec, plasma_enum_t uplo, int n, int nrh
         rc = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_X, prec, PlasmaGeneral, nb, n, nrhs, &Xbar);
     if (rc == PlasmaSuccess)
         rc = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_AS, prec, PlasmaGeneral, nb, n, n, &Lbar);
-    if (rc != PlasmaSuccess)
+    if (rc != PlasmaSuccess) {
+        plasma_kept_trim(plasma, &kept);
         return rc;
+    }
     plasma_sequence_t sequence;
     plasma_request_t request;
     plasma_sequence_init(&sequence);
@@ -351,6 +358,7 @@ static int Xpotrs_adjoint(plasma_enum_t prec, plasma_enum_t uplo, int n, int nrh
     plasma_omp_Xdesc2lapack(Xbar, pXbar, ldxbar, PlasmaGeneral, &sequence, &request);
     plasma_omp_Xdesc2lapack(Lbar, pLbar, ldlbar, uplo, &sequence, &request);
     plasma_sequence_wait(&sequence);
+    plasma_kept_trim(plasma, &kept);
     return sequence.status;
 }
 

@@ -429,8 +429,10 @@ int plasma_dsgesv(int n, int nrhs, double *pA, int lda, int *ipiv, double *pB, i
     for (int i = 0; i < 4 && rc == PlasmaSuccess; i++)
         rc = plasma_desc_kept(plasma, slot[i], i == 3 ? PlasmaRealFloat : PlasmaRealDouble,
                               PlasmaGeneral, nb, n, nrhs, rhs[i]);
-    if (rc != PlasmaSuccess)
+    if (rc != PlasmaSuccess) {
+        plasma_kept_trim(plasma, NULL);
         return rc;
+    }
     plasma_sequence_t sequence;
     plasma_request_t request;
     plasma_sequence_init(&sequence);
@@ -442,5 +444,6 @@ int plasma_dsgesv(int n, int nrhs, double *pA, int lda, int *ipiv, double *pB, i
     plasma_sequence_wait(&sequence);
     plasma_omp_Xdesc2lapack(X, pX, ldx, PlasmaGeneral, &sequence, &request);
     plasma_sequence_wait(&sequence);
+    plasma_kept_trim(plasma, NULL);
     return sequence.status;
 }

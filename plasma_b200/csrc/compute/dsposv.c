@@ -799,6 +799,7 @@ int plasma_dsposv_ex(plasma_enum_t uplo, int n, int nrhs,
         (retval = plasma_desc_kept(plasma, PLASMA_SLOT_DESC_XS, PlasmaRealFloat, PlasmaGeneral,
                                    nb, npad, nrhs, &Xs)) != 0) {
         plasma_error("tile copies of the right-hand sides failed");
+        plasma_kept_trim(plasma, NULL);
         return retval;
     }
     double *Rnorm = (double *)malloc(sizeof(double) * nrhs);
@@ -834,7 +835,7 @@ int plasma_dsposv_ex(plasma_enum_t uplo, int n, int nrhs,
     plasma_sequence_wait(&sequence);
     plasma_omp_Xdesc2lapack(X, pX, ldx, PlasmaGeneral, &sequence, &request);
     plasma_sequence_wait(&sequence);
-
+    plasma_kept_trim(plasma, NULL);
     free(Rnorm);
     free(Xnorm);
     return sequence.status;

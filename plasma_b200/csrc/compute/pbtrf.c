@@ -469,6 +469,7 @@ static int Xband(plasma_enum_t prec, int op, plasma_enum_t uplo, int n, int kd, 
     if (op != OP_TRF)
         plasma_omp_Xdesc2lapack(B, pB, ldb, PlasmaGeneral, &sequence, &request);
     plasma_sequence_wait(&sequence);
+    plasma_kept_trim(plasma, NULL);
     return sequence.status;
 }
 

@@ -191,7 +191,7 @@ static int Xpotrs(plasma_enum_t prec, plasma_enum_t uplo, int n, int nrhs,
     plasma_sequence_wait(&sequence);
     plasma_omp_Xdesc2lapack(B, pB, ldb, PlasmaGeneral, &sequence, &request);
     plasma_sequence_wait(&sequence);
-
+    plasma_kept_trim(plasma, NULL);
     return sequence.status;
 }
 
@@ -256,7 +256,7 @@ static int Xposv(plasma_enum_t prec, plasma_enum_t uplo, int n, int nrhs,
         plasma_omp_Xdesc2lapack(A, pA, lda, uplo, &sequence, &request);
     plasma_omp_Xdesc2lapack(B, pB, ldb, PlasmaGeneral, &sequence, &request);
     plasma_sequence_wait(&sequence);
-
+    plasma_kept_trim(plasma, NULL);
     return sequence.status;
 }
 

@@ -322,29 +322,88 @@ int plasma_call_begin(plasma_context_t *c, plasma_sequence_t *sequence,
     return id;
 }
 
+/* Operands that stay allocated between calls: up to this size a cudaMalloc and
+ * cudaFree are a good part of a call's time (0.5 to 2 ms, and now and then
+ * much more); the calls whose right-hand sides or adjoint operands are larger
+ * take a tenth of a second and more, and other allocators of the process
+ * need the memory. */
+#define PLASMA_KEPT_MAX ((size_t)1 << 30)
+
+static void scratch_drain(plasma_context_t *c)
+{
+    cudaStreamSynchronize(c->stream);
+    for (int i = 0; i < PLASMA_NUM_STREAMS; i++)
+        cudaStreamSynchronize(c->aux[i]);
+}
+
+static void scratch_free(plasma_context_t *c, int slot)
+{
+    cudaFree(c->scratch[slot]);
+    c->scratch[slot] = NULL;
+    c->scratch_bytes[slot] = 0;
+}
+
+static int scratch_alloc(plasma_context_t *c, int slot, size_t bytes)
+{
+    plasma_note_cuda_error();
+    plasma_alloc_count_g++;
+    if (cudaMalloc(&c->scratch[slot], bytes) != cudaSuccess) {
+        plasma_note_cuda_error();
+        c->scratch[slot] = NULL;
+        return 0;
+    }
+    c->scratch_bytes[slot] = bytes;
+    return 1;
+}
+
 void *plasma_scratch(plasma_context_t *c, int slot, size_t bytes)
 {
+    if (slot == PLASMA_SLOT_DESC_A)
+        c->scratch_used = 0;
+    c->scratch_used |= 1u << slot;
     if (bytes <= c->scratch_bytes[slot])
         return c->scratch[slot];
     if (c->scratch[slot]) {
         /* growing: wait for every user of the old buffer */
-        cudaStreamSynchronize(c->stream);
-        for (int i = 0; i < PLASMA_NUM_STREAMS; i++)
-            cudaStreamSynchronize(c->aux[i]);
-        cudaFree(c->scratch[slot]);
-        c->scratch[slot] = NULL;
-        c->scratch_bytes[slot] = 0;
+        scratch_drain(c);
+        scratch_free(c, slot);
     }
-    size_t want = bytes + bytes / 8 + (1u << 20);
-    plasma_note_cuda_error();
-    plasma_alloc_count_g++;
-    if (cudaMalloc(&c->scratch[slot], want) != cudaSuccess) {
-        plasma_note_cuda_error();
-        c->scratch[slot] = NULL;
-        return NULL;
-    }
-    c->scratch_bytes[slot] = want;
-    return c->scratch[slot];
+    /* with room to grow, else exactly what is needed, else the same once the
+     * slots that this call does not use are free */
+    if (scratch_alloc(c, slot, bytes + bytes / 8 + (1u << 20)) || scratch_alloc(c, slot, bytes))
+        return c->scratch[slot];
+    int freed = 0;
+    for (int i = 0; i < PLASMA_SCRATCH_SLOTS; i++)
+        if (c->scratch[i] && !(c->scratch_used >> i & 1)) {
+            if (!freed++)
+                scratch_drain(c);
+            scratch_free(c, i);
+        }
+    if (freed && scratch_alloc(c, slot, bytes))
+        return c->scratch[slot];
+    return NULL;
+}
+
+plasma_kept_t plasma_kept_sizes(plasma_context_t *c)
+{
+    return (plasma_kept_t){c->scratch_bytes[PLASMA_SLOT_DESC_A],
+                           c->scratch_bytes[PLASMA_SLOT_DESC_AS]};
+}
+
+void plasma_kept_trim(plasma_context_t *c, const plasma_kept_t *adjoint)
+{
+    static const int rhs[4] = {PLASMA_SLOT_DESC_B, PLASMA_SLOT_DESC_X, PLASMA_SLOT_DESC_R,
+                               PLASMA_SLOT_DESC_XS};
+    for (int i = 0; i < 4; i++)
+        if (c->scratch_bytes[rhs[i]] > PLASMA_KEPT_MAX)
+            scratch_free(c, rhs[i]);
+    if (adjoint == NULL)
+        return;
+    const int op[2] = {PLASMA_SLOT_DESC_A, PLASMA_SLOT_DESC_AS};
+    const size_t before[2] = {adjoint->a, adjoint->as};
+    for (int i = 0; i < 2; i++)
+        if (c->scratch_bytes[op[i]] > PLASMA_KEPT_MAX && c->scratch_bytes[op[i]] > before[i])
+            scratch_free(c, op[i]);
 }
 
 void *plasma_pinned(plasma_context_t *c, size_t bytes)

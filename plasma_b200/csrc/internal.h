@@ -95,9 +95,11 @@ typedef struct {
     plasma_request_t *pending[PLASMA_MAX_PENDING_CALLS];
     plasma_sequence_t *pending_seq[PLASMA_MAX_PENDING_CALLS];
 
-    /* growable device scratch slots (never shrink until finalize) */
+    /* growable device scratch slots (kept until finalize, but see
+     * plasma_scratch and plasma_kept_trim) */
     void  *scratch[PLASMA_SCRATCH_SLOTS];
     size_t scratch_bytes[PLASMA_SCRATCH_SLOTS];
+    unsigned scratch_used;          /* slots the present call has asked for */
     void  *pinned;
     size_t pinned_bytes;
     cudaEvent_t ev[8];                        /* DAG edges (reused)        */
@@ -134,8 +136,18 @@ int plasma_call_begin(plasma_context_t *plasma, plasma_sequence_t *sequence,
 
 /* Device scratch of at least `bytes` in one of the slots above.  The buffer
  * stays valid until the same slot is requested with a larger size; all users
- * are ordered on the context streams, and growth waits for them. */
+ * are ordered on the context streams, and growth waits for them.  When there
+ * is no memory for it, the slots that the present call has not asked for give
+ * theirs back (a LAPACK-layout call begins with its request for
+ * PLASMA_SLOT_DESC_A). */
 void *plasma_scratch(plasma_context_t *plasma, int slot, size_t bytes);
+/* At the end of a LAPACK-layout call, its stream drained: operand slots that
+ * are too large to keep (PLASMA_KEPT_MAX) are freed.  The right-hand sides'
+ * always; with `adjoint`, those of L and Lbar if this call made them larger
+ * than they were (`before`: their bytes then). */
+typedef struct { size_t a, as; } plasma_kept_t;
+plasma_kept_t plasma_kept_sizes(plasma_context_t *plasma);
+void plasma_kept_trim(plasma_context_t *plasma, const plasma_kept_t *adjoint);
 void *plasma_pinned(plasma_context_t *plasma, size_t bytes);
 
 /* Queries whether p is device memory of the context's device. */

@@ -106,3 +106,68 @@ def test_no_host_memory(tmp_path):
         assert L.plasma_kernel_launches() - before < 10
         assert solve() == 0 and np.abs(x @ a - b).max() < 1e-12
         """, {"LD_PRELOAD": str(so)})
+
+
+MEMORY = """
+        MB = 1 << 20
+        L.plasma_set(pb.PlasmaTuning, pb.PlasmaDisabled)
+        L.plasma_set(pb.PlasmaNb, 256)
+        def free():
+            torch.cuda.synchronize()
+            return torch.cuda.mem_get_info()[0]
+        def spd(n, dtype=torch.float64):
+            return torch.full((n, n), 0.25, device="cuda", dtype=dtype) + \\
+                   n * torch.eye(n, device="cuda", dtype=dtype)
+        def factor(a):
+            return L.plasma_dpotrf(pb.PlasmaLower, a.shape[0], a.data_ptr(), a.shape[0])
+        held = []
+        def leave(mb):
+            torch.cuda.empty_cache()
+            held.append(torch.empty(max(free() - mb * MB, 0), dtype=torch.uint8, device="cuda"))
+            return free() // MB
+        assert factor(spd(5000)) == 0            # loads the kernels
+        """
+
+
+def test_scratch_that_just_fits():
+    """A tile copy that fits, but not with an eighth on top, is allocated at
+    its own size: n = 20000 packed takes 1580 MB, 197 more with headroom."""
+    child(MEMORY + """
+        a = spd(20000)
+        L.plasma_set_stream(ct.c_void_p(1))
+        kept = free()
+        left = leave(1640)
+        assert 1600 <= left <= 1740, left
+        assert factor(a) == 0
+        """)
+
+
+def test_idle_slots_give_way():
+    """Right-hand sides that an earlier call left in their slot do not keep a
+    later call from the memory it needs."""
+    child(MEMORY + """
+        n, nrhs = 4096, 24000                   # 752 MiB of right-hand sides
+        f, b = spd(n), torch.ones(nrhs, n, device="cuda", dtype=torch.float64)
+        L.plasma_set_stream(ct.c_void_p(1))
+        assert L.plasma_dposv(pb.PlasmaLower, n, nrhs, f.data_ptr(), n, b.data_ptr(), n) == 0
+        del f, b
+        a = spd(20000)
+        left = leave(1000)
+        assert left <= 1100, left
+        assert factor(a) == 0
+        """)
+
+
+def test_large_operands_are_returned():
+    """Right-hand sides and adjoint operands above 1 GiB do not stay allocated
+    after the call: what remains of an adjoint is its n x n work matrices."""
+    child(MEMORY + """
+        n = 12288                               # 1152 MiB a matrix
+        a = spd(n)
+        L.plasma_set_stream(ct.c_void_p(1))
+        g = torch.eye(n, device="cuda", dtype=torch.float64)
+        torch.cuda.empty_cache()
+        before = free()
+        assert L.plasma_dpotrf_adjoint(pb.PlasmaLower, n, a.data_ptr(), n, g.data_ptr(), n) == 0
+        assert before - free() <= 2 * 1152 * 1.125 * MB + 256 * MB
+        """)
