@@ -35,11 +35,11 @@ __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b)
 // accumulator.  It serves unchanged as the A operand of the next product
 // when the K index is taken in the order 2t, then 2t+1: the B operands of
 // columns 8q .. 8q+7 are then B(8q + 2t, g) and B(8q + 2t + 1, g).
-__device__ __forceinline__ void strip_mma(double (&d)[2], const double (&x)[2], double sign,
-                                          double b0, double b1)
+__device__ __forceinline__ void strip_mma(double (&d)[2], const double (&x)[2], double b0,
+                                          double b1)
 {
-    dmma_8x8x4(d, sign * x[0], b0);
-    dmma_8x8x4(d, sign * x[1], b1);
+    dmma_8x8x4(d, x[0], b0);
+    dmma_8x8x4(d, x[1], b1);
 }
 
 // The inverse of the 8 x 8 lower-triangular block whose entry (i, q) is
@@ -56,23 +56,29 @@ __device__ __forceinline__ void inv8_column(int j, L l, R r, T (&w)[8])
     }
 }
 
-// Y L^T = X for 8 rows and the 32 columns of a diagonal block, in place:
-// y[q] = columns 8q .. 8q+7.  D: the block (pd_at layout); W8: the inverses
-// of its 8 x 8 diagonal blocks, entry (i, j) of block q at
+// Y L^T = X - S for 8 rows and the 32 columns of a diagonal block, in place:
+// y[q] = columns 8q .. 8q+7 of X, then of Y; s[q] those of S, what solved
+// columns to the left owe (destroyed).  D: the block (pd_at layout); W8: the
+// inverses of its 8 x 8 diagonal blocks, entry (i, j) of block q at
 // W8[(8 q + j) * 8 + i].  Only 8 x 8 blocks are inverted, so the result
 // differs from plain substitution by no more than their condition, and the
-// solve runs at the pace of four dependent pairs of products.
-__device__ __forceinline__ void strip_solve32(double (&y)[4][2], const double *D,
-                                              const double *W8)
+// solve runs at the pace of four dependent pairs of products.  The products
+// are summed apart from X, which takes one rounding: added to X one by one,
+// each would round at the size of X (order 300 in tiles of 128, entries below
+// the diagonal: 3.3 u against 2.6 u for a well-conditioned Gram matrix).
+__device__ __forceinline__ void strip_solve32(double (&y)[4][2], double (&s)[4][2],
+                                              const double *D, const double *W8)
 {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
         double x[2] = {0.0, 0.0};
-        strip_mma(x, y[q], 1.0, W8[(8 * q + 2 * t) * 8 + g], W8[(8 * q + 2 * t + 1) * 8 + g]);
+#pragma unroll
+        for (int e = 0; e < 2; e++) y[q][e] -= s[q][e];
+        strip_mma(x, y[q], W8[(8 * q + 2 * t) * 8 + g], W8[(8 * q + 2 * t + 1) * 8 + g]);
 #pragma unroll
         for (int f = q + 1; f < 4; f++)
-            strip_mma(y[f], x, -1.0, D[pd_at(8 * q + 2 * t, 8 * f + g)],
+            strip_mma(s[f], x, D[pd_at(8 * q + 2 * t, 8 * f + g)],
                       D[pd_at(8 * q + 2 * t + 1, 8 * f + g)]);
         y[q][0] = x[0];
         y[q][1] = x[1];

@@ -46,12 +46,15 @@ __device__ __forceinline__ void pd_solve_strip(double *X, const double *D, const
                                                int r0)
 {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    double y[4][2];
+    double y[4][2], s[4][2];
 #pragma unroll
     for (int q = 0; q < 4; q++)
 #pragma unroll
-        for (int e = 0; e < 2; e++) y[q][e] = X[pd_at(8 * q + 2 * t + e, r0 + g)];
-    strip_solve32(y, D, W8);
+        for (int e = 0; e < 2; e++) {
+            y[q][e] = X[pd_at(8 * q + 2 * t + e, r0 + g)];
+            s[q][e] = 0.0;
+        }
+    strip_solve32(y, s, D, W8);
 #pragma unroll
     for (int q = 0; q < 4; q++)
 #pragma unroll

@@ -88,7 +88,7 @@ k_trsm_f64(plasma_desc_t A, int k, int mlo, int vec, const plasma_devstat_t *st)
             for (int e = 0; e < 2; e++)
                 y[q][e] = row < rows ? B[(size_t)(32 * J + 8 * q + 2 * t + e) * ldb + row] : 0.0;
     };
-    double y[4][2], nx[4][2];
+    double y[4][2], nx[4][2], sum[4][2];      // sum: X_{<J} L(J,<J)^T
     fetch(0, nx);
 
     // the inverses of the 8 x 8 diagonal blocks, a thread per column
@@ -112,7 +112,10 @@ k_trsm_f64(plasma_desc_t A, int k, int mlo, int vec, const plasma_devstat_t *st)
 #pragma unroll
         for (int q = 0; q < 4; q++)
 #pragma unroll
-            for (int e = 0; e < 2; e++) y[q][e] = nx[q][e];
+            for (int e = 0; e < 2; e++) {
+                y[q][e] = nx[q][e];
+                sum[q][e] = 0.0;
+            }
         if (J + 1 < nblk) fetch(J + 1, nx);
         for (int I = 0; I <= J; I++, b++) {
             cp_async_wait<TF_RING - 2>();
@@ -126,11 +129,11 @@ k_trsm_f64(plasma_desc_t A, int k, int mlo, int vec, const plasma_devstat_t *st)
                 const double x[2] = {x01.x, x01.y};
 #pragma unroll
                 for (int f = 0; f < 4; f++)
-                    strip_mma(y[f], x, -1.0, D[pd_at(8 * q + 2 * t, 8 * f + g)],
+                    strip_mma(sum[f], x, D[pd_at(8 * q + 2 * t, 8 * f + g)],
                               D[pd_at(8 * q + 2 * t + 1, 8 * f + g)]);
             }
         }
-        strip_solve32(y, Lr + (b % TF_RING) * F64_BLK, W8 + 32 * J * 8);
+        strip_solve32(y, sum, Lr + (b % TF_RING) * F64_BLK, W8 + 32 * J * 8);
         b++;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
