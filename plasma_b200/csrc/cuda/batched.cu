@@ -446,8 +446,9 @@ __device__ void factor_adjoint_one(const T *Lf, int n, T *Lb, T *Cs, T *Ds, T *D
 #pragma unroll
                 for (int q = NB / 8 - 1; q >= 0; q--) {
                     T x[4];
-                    strip16_product<T, SPLIT>(x, y[q], W8[(8 * q + g) * 8 + 2 * t],
-                                              W8[(8 * q + g) * 8 + 2 * t + 1]);
+                    const T *w = W8 + 64 * q;
+                    strip16_inverse<T, SPLIT>(x, y[q], w[8 * g + 2 * t], w[8 * g + 2 * t + 1],
+                                              w[18 * t], w[18 * t + 9]);
 #pragma unroll
                     for (int f = 0; f < q; f++)
                         strip16_subtract<T, SPLIT>(y[f], x, Dp[pd_at(8 * f + g, 8 * q + 2 * t)],

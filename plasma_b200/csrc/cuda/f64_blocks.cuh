@@ -267,6 +267,25 @@ __device__ __forceinline__ void strip16_subtract(T (&y)[4], const T (&x)[4], T b
     for (int e = 0; e < 4; e++) y[e] -= d[e];
 }
 
+// d <- x B for a triangular B (an inverse in W8) whose diagonal entries of this
+// lane's columns are w0 = B(2t, 2t) and w1 = B(2t+1, 2t+1).  FP32: the tensor
+// cores truncate a sum at its own size, which here is the result's, and all
+// in one direction; the diagonal's terms, the largest in general, stay out of
+// it and are added rounded.
+template <typename T, int SPLIT>
+__device__ __forceinline__ void strip16_inverse(T (&d)[4], const T (&x)[4], T b0, T b1, T w0,
+                                                T w1)
+{
+    if (sizeof(T) == 8) {
+        strip16_product<T, SPLIT>(d, x, b0, b1);
+        return;
+    }
+    const int g = (threadIdx.x >> 2) & 7, t = threadIdx.x & 3;
+    strip16_product<T, SPLIT>(d, x, g == 2 * t ? T(0) : b0, g == 2 * t + 1 ? T(0) : b1);
+#pragma unroll
+    for (int e = 0; e < 4; e++) d[e] = fma(x[e], e & 1 ? w1 : w0, d[e]);
+}
+
 // strip_solve32 for 16 rows and NB columns
 template <typename T, int SPLIT, int NB>
 __device__ __forceinline__ void strip16_solve(T (&y)[NB / 8][4], const T *D, const T *W8)
@@ -275,8 +294,9 @@ __device__ __forceinline__ void strip16_solve(T (&y)[NB / 8][4], const T *D, con
 #pragma unroll
     for (int q = 0; q < NB / 8; q++) {
         T x[4];
-        strip16_product<T, SPLIT>(x, y[q], W8[(8 * q + 2 * t) * 8 + g],
-                                  W8[(8 * q + 2 * t + 1) * 8 + g]);
+        const T *w = W8 + 64 * q;
+        strip16_inverse<T, SPLIT>(x, y[q], w[16 * t + g], w[16 * t + 8 + g], w[18 * t],
+                                  w[18 * t + 9]);
 #pragma unroll
         for (int f = q + 1; f < NB / 8; f++)
             strip16_subtract<T, SPLIT>(y[f], x, D[pd_at(8 * q + 2 * t, 8 * f + g)],

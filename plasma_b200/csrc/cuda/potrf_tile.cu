@@ -291,7 +291,8 @@ k_trtri_join(plasma_desc_t A, int uplo, int h, T *W, const plasma_devstat_t *st)
     };
     clear();
     if (i0 < h) {
-        for (int q = j0; q < h; q += 8) {         // A^-1 is lower: rows q >= column j0
+        // A^-1 is lower: rows q >= column j0, the (largest) diagonal's terms last
+        for (int q = h - 8; q >= j0; q -= 8) {
             const double af[4] = {Bv(i0 + g, q + t), Bv(i0 + g + 8, q + t), Bv(i0 + g, q + t + 4),
                                   Bv(i0 + g + 8, q + t + 4)};
 #pragma unroll

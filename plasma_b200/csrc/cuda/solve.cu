@@ -137,7 +137,11 @@ k_diag_mma(plasma_desc_t B, int k, int n0, const T *W, int trans, const plasma_d
     auto op = [&](int i, int q) {
         return trans ? w[(size_t)i * NB + q] : w[(size_t)q * NB + i];
     };
-    const int q0 = trans ? i0 : 0, q1 = trans ? NB : i0 + 16 * MI;
+    // the nonzero part of W, 8 columns (rows of B) a step, the diagonal last:
+    // its terms are the largest in general, and a sum that begins with them
+    // rounds at their size from there on
+    const int steps = (trans ? NB - i0 : i0 + 16 * MI) / 8;
+    const int qs = trans ? -8 : 8;
     T an[MI][4];
     auto fetch = [&](int q) {
 #pragma unroll
@@ -146,14 +150,15 @@ k_diag_mma(plasma_desc_t B, int k, int n0, const T *W, int trans, const plasma_d
             for (int e = 0; e < 4; e++)
                 an[m][e] = op(i0 + 16 * m + g + 8 * (e & 1), q + t + 4 * (e >> 1));
     };
-    fetch(q0);
-    for (int q = q0; q < q1; q += 8) {
+    int q = trans ? NB - 8 : 0;
+    fetch(q);
+    for (int i = 0; i < steps; i++, q += qs) {
         T a[MI][4], bf[NF][2];
 #pragma unroll
         for (int m = 0; m < MI; m++)
 #pragma unroll
             for (int e = 0; e < 4; e++) a[m][e] = an[m][e];
-        if (q + 8 < q1) fetch(q + 8);
+        if (i + 1 < steps) fetch(q + qs);
 #pragma unroll
         for (int f = 0; f < NF; f++) {
             bf[f][0] = Bs[(q + t) * LDS + 8 * f + g];
@@ -163,8 +168,9 @@ k_diag_mma(plasma_desc_t B, int k, int n0, const T *W, int trans, const plasma_d
         for (int m = 0; m < MI; m++)
 #pragma unroll
             for (int f = 0; f < NF; f++) mma8<3>(acc[m][f], a[m], bf[f]);
-        // FP32: the tensor cores truncate long sums; leave them every 32 terms
-        if (sizeof(T) == 8 ? q + 8 >= q1 : ((q & 24) == 24 || q + 8 >= q1)) {
+        // FP32: the tensor cores truncate what they add to a sum; the terms
+        // leave them 8 at a time
+        if (sizeof(T) == 4 || i + 1 == steps) {
 #pragma unroll
             for (int m = 0; m < MI; m++)
 #pragma unroll
