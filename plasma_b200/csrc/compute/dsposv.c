@@ -318,7 +318,7 @@ static void upload_and_factor(plasma_context_t *plasma, const upload_t *up,
     const int n = A.m, nb = A.nb;
     /* every slot the factorization uses is sized before the first copy: a
      * slot that grows waits for all streams, the copy stream included */
-    plasma_pXpotrf_reserve(plasma, PlasmaLower, As, mode, 1);
+    plasma_pXpotrf_reserve(plasma, PlasmaLower, As, mode | PLASMA_FACTOR_REFINED, 1);
     double *stage = (double *)plasma_scratch(plasma, PLASMA_SLOT_STAGING,
                                              (size_t)n * (size_t)n * sizeof(double));
     /* the walk scales panel rows by the diagonal before its columns are in.
@@ -362,8 +362,8 @@ static void upload_and_factor(plasma_context_t *plasma, const upload_t *up,
     cudaEventRecord(plasma->ev[5], cp);
     for (int i = 0; i < As.gm; i++)
         diag[i] = i < n ? (float)up->pA[(size_t)i * up->lda + i] : 1.0f;
-    plasma_pXpotrf_arrivals(plasma, PlasmaLower, As, sequence, request, call, mode, ng,
-                            gstart, plasma->ev_group, diag);
+    plasma_pXpotrf_arrivals(plasma, PlasmaLower, As, sequence, request, call,
+                            mode | PLASMA_FACTOR_REFINED, ng, gstart, plasma->ev_group, diag);
     free(diag);
     cudaStreamWaitEvent(S, plasma->ev[5], 0);
 }
@@ -565,7 +565,8 @@ static void Xdsposv(plasma_context_t *plasma, plasma_enum_t uplo,
             plasma_cuda_scale_shift(S, As, uplo_s, dvec, (float)(plan[a].scaled * u));
             RF.dscale = dvec;
         }
-        plasma_pXpotrf_mode(plasma, uplo_s, As, sequence, request, call, mode);
+        plasma_pXpotrf_mode(plasma, uplo_s, As, sequence, request, call,
+                            mode | PLASMA_FACTOR_REFINED);
         fstatus = take_status(plasma);
         factor_failed = fstatus != 0;
         if (rep)

@@ -212,21 +212,24 @@ k_trsm_tc(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUte
         // at `bl` bytes further)
         auto products = [&](uint32_t d, const unsigned char *b, int bl, int n, uint32_t first) {
             const uint32_t idesc = ts_idesc(n);
+            // a sum in tensor memory is truncated at every addition, whatever is
+            // added: the small products go first, over all of K, while it is
+            // small
+            if (parts == 2) {
 #pragma unroll
-            for (int kk = 0; kk < TS_B / 8; kk++) {
-                const uint64_t bh = smem_desc(b + kk * 8 * 128, TS_CHUNK, TS_SBO, 1u);
-                const uint32_t ah = tmem + c_ahi + 8 * kk;
-                const uint32_t acc = (kk > 0 || first) ? 1u : 0u;
-                if (parts == 2) {
+                for (int kk = 0; kk < TS_B / 8; kk++) {
+                    const uint64_t bh = smem_desc(b + kk * 8 * 128, TS_CHUNK, TS_SBO, 1u);
                     const uint64_t blo = smem_desc(b + bl + kk * 8 * 128, TS_CHUNK, TS_SBO, 1u);
-                    const uint32_t al = tmem + c_alo + 8 * kk;
-                    mma_ta(tmem + d, al, bh, idesc, acc);         // small terms first
-                    mma_ta(tmem + d, ah, blo, idesc, 1u);
-                    mma_ta(tmem + d, ah, bh, idesc, 1u);
-                } else {
-                    mma_ta(tmem + d, ah, bh, idesc, acc);
+                    mma_ta(tmem + d, tmem + c_alo + 8 * kk, bh, idesc,
+                           (kk > 0 || first) ? 1u : 0u);
+                    mma_ta(tmem + d, tmem + c_ahi + 8 * kk, blo, idesc, 1u);
                 }
             }
+#pragma unroll
+            for (int kk = 0; kk < TS_B / 8; kk++)
+                mma_ta(tmem + d, tmem + c_ahi + 8 * kk,
+                       smem_desc(b + kk * 8 * 128, TS_CHUNK, TS_SBO, 1u), idesc,
+                       (kk > 0 || first || parts == 2) ? 1u : 0u);
         };
         for (int j = 0; j < nblk; j++) {
             if (!mbar_wait(&y_bar, j & 1, &abort_s)) break;
@@ -533,7 +536,7 @@ extern "C" int plasma_cuda_trsm_tc(cudaStream_t s, plasma_devstat_t *st, int mod
     const int split = mode == PLASMA_TC_TF32 || mode == PLASMA_TC_BF16 ? 1 : 3;
     const int parts = split == 3 ? 2 : 1;
     int poff = 0, pstride = 0;
-    const bool half = mode == PLASMA_TC_FP16X3;
+    const bool half = mode == PLASMA_TC_FP16X3 || mode == PLASMA_TC_FP16X3S;
     const bool write_panel = panel != nullptr &&
                              ((half && scale != nullptr) || mode == PLASMA_TC_TF32);
     if (write_panel) plasma_cuda_panel_layout(A, k, full, &poff, &pstride);

@@ -20,8 +20,15 @@
 //            s_i = 2^14 / 2^ceil(log2 sqrt(A(i,i))) nothing overflows, products
 //            keep 22 bits down to 2^-16 of the row's bound and an absolute
 //            2^-39 of it below that, against the 2^-24 rounding of the sums.
-//            (n = 32768: all trailing updates of a factor 77 ms with three
-//            TF32 products of the same split.)
+//            A sum in tensor memory is truncated at every addition, whatever is
+//            added.  For factors that the caller gets, K is walked twice: the
+//            two small products first, while the sum is small, then hi*hi with
+//            the high part of A read again.  One walk truncates three times a
+//            step at the size of the sum (Gram matrix of order 3001, in units
+//            of 2^-24: diagonal 1.9, below it 4.9, against 1.5 and 3.1; the
+//            FP32 sums of the ragged tiles before, 1.0 and 3.7).  It costs a
+//            factor of order 5003 1.3%, and would cost dsposv at n = 32768, whose
+//            factor is refined in FP64, 71.0 instead of 64.8 ms.
 //   BF16X6 : the panel split in three BF16 parts, a = h + m + l (h = bf16(a),
 //            m = bf16(a - h), l = bf16(a - h - m)), and a*b formed from the six
 //            products whose order is at most 2^-16 (l*h, h*l, m*m, m*h, h*m,
@@ -180,7 +187,7 @@ struct TileCursor {
     __device__ __forceinline__ bool last_of_column() const { return m == mt - 1; }
 };
 
-template <int MODE>
+template <int MODE, int PASSES>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 k_update_tc(const __grid_constant__ CUtensorMap opmap,
             const __grid_constant__ CUtensorMap cmap, TcArgs g,
@@ -240,17 +247,21 @@ k_update_tc(const __grid_constant__ CUtensorMap opmap,
             int m, n, si;
             tc_item(g, first + j, m, n, si);
             const int i0 = si * TC_M;
-            for (int kb = 0; kb < nkb; kb++, it++) {
+            for (int kp = 0; kp < PASSES * nkb; kp++, it++) {
                 const int s = it % TC_STAGES;
+                const bool again = PASSES == 2 && kp >= nkb;  // the high parts alone
+                const int kb = again ? kp - nkb : kp;
                 if (it >= TC_STAGES &&
                     !mbar_wait(&empty_bar[s], ((it / TC_STAGES) - 1) & 1, &abort_s)) {
                     ok = false;
                     break;
                 }
                 unsigned char *sp = stage_base + s * TC_STAGE_BYTES;
-                mbar_expect_tx(&full_bar[s], (uint32_t)stage_bytes);
+                mbar_expect_tx(&full_bar[s], (uint32_t)(again ? stage_bytes / G::PARTS
+                                                              : stage_bytes));
 #pragma unroll
                 for (int p = 0; p < G::PARTS; p++) {
+                    if (again && p > 0) break;
                     unsigned char *sa = sp + p * G::A_BYTES;
                     unsigned char *sb = sp + G::PARTS * G::A_BYTES + p * b_bytes;
                     const int toff = g.poff + p * g.mt;
@@ -273,7 +284,7 @@ k_update_tc(const __grid_constant__ CUtensorMap opmap,
                 break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t acc_t = tmem + (uint32_t)(a * nb);
-            for (int kb = 0; kb < nkb; kb++, it++) {
+            for (int kp = 0; kp < PASSES * nkb; kp++, it++) {
                 const int s = it % TC_STAGES;
                 if (!mbar_wait(&full_bar[s], (it / TC_STAGES) & 1, &abort_s)) {
                     ok = false;
@@ -285,22 +296,21 @@ k_update_tc(const __grid_constant__ CUtensorMap opmap,
                 unsigned char *sb_hi = sp + G::PARTS * G::A_BYTES;
 #pragma unroll
                 for (int kk = 0; kk < G::BK / G::KI; kk++) {
-                    const uint32_t acc_on = (kb | kk) != 0;
+                    const uint32_t acc_on = (kp | kk) != 0;
                     uint64_t da = smem_desc(sa_hi + kk * G::KI * 128, G::CHUNK, G::SBO,
                                             G::LAYOUT);
                     uint64_t db = smem_desc(sb_hi + kk * G::KI * 128, G::CHUNK, G::SBO,
                                             G::LAYOUT);
-                    if (MODE == MODE_FP16X3) {
+                    if (MODE == MODE_FP16X3 && (PASSES == 1 || kp < nkb)) {
                         unsigned char *sa_lo = sp + G::A_BYTES;
                         unsigned char *sb_lo = sb_hi + b_bytes;
                         uint64_t dal = smem_desc(sa_lo + kk * G::KI * 128, G::CHUNK, G::SBO,
                                                  G::LAYOUT);
                         uint64_t dbl = smem_desc(sb_lo + kk * G::KI * 128, G::CHUNK, G::SBO,
                                                  G::LAYOUT);
-                        // small terms first
                         mma<MODE>(acc_t, dal, db, idesc, acc_on);
                         mma<MODE>(acc_t, da, dbl, idesc, 1u);
-                        mma<MODE>(acc_t, da, db, idesc, 1u);
+                        if (PASSES == 1) mma<MODE>(acc_t, da, db, idesc, 1u);
                     } else {
                         mma<MODE>(acc_t, da, db, idesc, acc_on);
                     }
@@ -489,7 +499,7 @@ __device__ __forceinline__ uint32_t instr_desc_pair(int mode)
            ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
 }
 
-template <int MODE>
+template <int MODE, int PASSES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
 k_update_pair(const __grid_constant__ CUtensorMap opmap,
               const __grid_constant__ CUtensorMap cmap, TcArgs g,
@@ -581,8 +591,10 @@ k_update_pair(const __grid_constant__ CUtensorMap opmap,
                     !mbar_wait_cluster(&bempty_bar, (nb_loads - 1) & 1, &abort_s)) break;
                 nb_loads++;
             }
-            for (int kb = 0; kb < nkb; kb++, it++) {
+            for (int kp = 0; kp < PASSES * nkb; kp++, it++) {
                 const int s = it % STAGES;
+                const bool again = PASSES == 2 && kp >= nkb;  // the high part of A alone
+                const int kb = again ? kp - nkb : kp;
                 if (it >= STAGES &&
                     !mbar_wait_cluster(&empty_bar[s], ((it / STAGES) - 1) & 1, &abort_s)) {
                     ok = false;
@@ -592,18 +604,20 @@ k_update_pair(const __grid_constant__ CUtensorMap opmap,
                 const uint32_t fb = full_lead0 + (uint32_t)(s * sizeof(uint64_t));
                 const uint32_t fbb = RESB ? bfull_lead0 + (uint32_t)(kb * sizeof(uint64_t)) : fb;
                 if (leader) {
-                    mbar_expect_tx(&full_bar[s], 2u * (uint32_t)STAGE_BYTES);
-                    if (RESB && load_b)
+                    mbar_expect_tx(&full_bar[s],
+                                   2u * (uint32_t)(again ? HALF : STAGE_BYTES));
+                    if (RESB && load_b && !again)
                         mbar_expect_tx(&bfull_bar[kb], 2u * (uint32_t)(G::PARTS * HALF));
                 }
 #pragma unroll
                 for (int p = 0; p < G::PARTS; p++) {
+                    if (again && p > 0) break;
                     const int toff = g.poff + p * g.mt;
                     unsigned char *sb = RESB ? resb + (kb * G::PARTS + p) * HALF
                                              : sp + (G::PARTS + p) * HALF;
                     tma_load_4d_pair(sp + p * HALF, &opmap, fb, 0, kb * G::BK,
                                      row0 / G::MNBOX, m + toff);
-                    if (load_b)
+                    if (load_b && !again)
                         tma_load_4d_pair(sb, &opmap, fbb, 0, kb * G::BK,
                                          row0 / G::MNBOX, n + toff);
                 }
@@ -624,11 +638,13 @@ k_update_pair(const __grid_constant__ CUtensorMap opmap,
                 break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t acc_t = tmem + (uint32_t)(a * NB);
-            for (int kb = 0; kb < nkb; kb++, it++) {
+            for (int kp = 0; kp < PASSES * nkb; kp++, it++) {
                 const int s = it % STAGES;
+                const int kb = PASSES == 1 || kp < nkb ? kp : kp - nkb;
                 if (!mbar_wait_cluster(&full_bar[s], (it / STAGES) & 1, &abort_s) ||
-                    (new_b && !mbar_wait_cluster(&bfull_bar[RESB ? kb : 0], (nb_loads - 1) & 1,
-                                                 &abort_s))) {
+                    (new_b && (PASSES == 1 || kp < nkb) &&
+                     !mbar_wait_cluster(&bfull_bar[RESB ? kb : 0], (nb_loads - 1) & 1,
+                                        &abort_s))) {
                     ok = false;
                     break;
                 }
@@ -638,19 +654,19 @@ k_update_pair(const __grid_constant__ CUtensorMap opmap,
                 unsigned char *sb_hi = RESB ? resb + kb * G::PARTS * HALF : sp + G::PARTS * HALF;
 #pragma unroll
                 for (int kk = 0; kk < G::BK / G::KI; kk++) {
-                    const uint32_t acc_on = (kb | kk) != 0;
+                    const uint32_t acc_on = (kp | kk) != 0;
                     uint64_t da = smem_desc(sa_hi + kk * G::KI * 128, G::CHUNK, G::SBO,
                                             G::LAYOUT);
                     uint64_t db = smem_desc(sb_hi + kk * G::KI * 128, G::CHUNK, G::SBO,
                                             G::LAYOUT);
-                    if (MODE == MODE_FP16X3) {
+                    if (MODE == MODE_FP16X3 && (PASSES == 1 || kp < nkb)) {
                         uint64_t dal = smem_desc(sa_hi + HALF + kk * G::KI * 128, G::CHUNK,
                                                  G::SBO, G::LAYOUT);
                         uint64_t dbl = smem_desc(sb_hi + HALF + kk * G::KI * 128, G::CHUNK,
                                                  G::SBO, G::LAYOUT);
                         mma_pair<MODE>(acc_t, dal, db, idesc, acc_on);
                         mma_pair<MODE>(acc_t, da, dbl, idesc, 1u);
-                        mma_pair<MODE>(acc_t, da, db, idesc, 1u);
+                        if (PASSES == 1) mma_pair<MODE>(acc_t, da, db, idesc, 1u);
                     } else if (MODE == MODE_BF16X6) {
                         // parts h, m, l at offsets 0, HALF, 2 HALF; small terms first
                         uint64_t dam = smem_desc(sa_hi + HALF + kk * G::KI * 128, G::CHUNK,
@@ -793,28 +809,28 @@ bool encode_c_map(CUtensorMap *map, const plasma_desc_t &A)
     return r == CUDA_SUCCESS;
 }
 
-template <int MODE>
+template <int MODE, int PASSES = 1>
 void launch_update(cudaStream_t s, const CUtensorMap &map, const CUtensorMap &cmap,
                    const TcArgs &g, unsigned grid, plasma_devstat_t *st)
 {
     static unsigned long long attr = 0;
     if (plasma_first_on_device(&attr)) {
-        cudaFuncSetAttribute(k_update_tc<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(k_update_tc<MODE, PASSES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              Geo<MODE>::SMEM);
     }
-    k_update_tc<MODE><<<grid, TC_THREADS, Geo<MODE>::SMEM, s>>>(map, cmap, g, st);
+    k_update_tc<MODE, PASSES><<<grid, TC_THREADS, Geo<MODE>::SMEM, s>>>(map, cmap, g, st);
 }
 
-template <int MODE>
+template <int MODE, int PASSES = 1>
 void launch_pair(cudaStream_t s, const CUtensorMap &map, const CUtensorMap &cmap,
                  const TcArgs &g, unsigned grid, plasma_devstat_t *st)
 {
     static unsigned long long attr = 0;
     if (plasma_first_on_device(&attr)) {
-        cudaFuncSetAttribute(k_update_pair<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(k_update_pair<MODE, PASSES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              PairGeo<MODE>::SMEM);
     }
-    k_update_pair<MODE><<<grid, TC_THREADS, PairGeo<MODE>::SMEM, s>>>(map, cmap, g, st);
+    k_update_pair<MODE, PASSES><<<grid, TC_THREADS, PairGeo<MODE>::SMEM, s>>>(map, cmap, g, st);
 }
 
 // Items per CTA (one CTA per SM) with the smallest estimated makespan,
@@ -858,7 +874,8 @@ void panel_layout(const plasma_desc_t &A, int k, int full, int *poff, int *pstri
 
 int mode_parts(int mode)
 {
-    return mode == PLASMA_TC_FP16X3 ? 2 : mode == PLASMA_TC_BF16X6 ? 3 : 1;
+    return mode == PLASMA_TC_FP16X3 || mode == PLASMA_TC_FP16X3S ? 2
+         : mode == PLASMA_TC_BF16X6 ? 3 : 1;
 }
 }  // namespace
 
@@ -882,7 +899,7 @@ extern "C" int plasma_cuda_update_tc_ok(plasma_desc_t A, plasma_enum_t uplo)
 // (full = 0) or all panels of the factor (full = 1).
 extern "C" size_t plasma_cuda_panel_bytes(int mode, plasma_desc_t A, int full)
 {
-    if (mode < PLASMA_TC_TF32 || mode > PLASMA_TC_FP16X3) return 0;
+    if (mode < PLASMA_TC_TF32 || mode > PLASMA_TC_FP16X3S) return 0;
     int poff, pstride;
     panel_layout(A, 0, full, &poff, &pstride);
     const size_t esz = mode == PLASMA_TC_TF32 ? 4 : 2;
@@ -899,6 +916,8 @@ extern "C" int plasma_cuda_update_tc(cudaStream_t s, plasma_devstat_t *st,
 {
     if (nhi <= nlo) return 1;
     const int nb = A.mb;
+    const int passes = mode == PLASMA_TC_FP16X3S ? 2 : 1;
+    if (mode == PLASMA_TC_FP16X3S) mode = PLASMA_TC_FP16X3;
     long long tiles = 0;
     for (int n = nlo; n < nhi; n++) tiles += A.mt - n;
     const long long nitems = tiles * (nb / TC_M);
@@ -983,14 +1002,20 @@ extern "C" int plasma_cuda_update_tc(cudaStream_t s, plasma_devstat_t *st,
     if (use_pair) {
         switch (mode) {
         case PLASMA_TC_TF32: launch_pair<MODE_TF32>(s, map, cmap, g, grid, st); break;
-        case PLASMA_TC_FP16X3: launch_pair<MODE_FP16X3>(s, map, cmap, g, grid, st); break;
+        case PLASMA_TC_FP16X3:
+            if (passes == 2) launch_pair<MODE_FP16X3, 2>(s, map, cmap, g, grid, st);
+            else launch_pair<MODE_FP16X3>(s, map, cmap, g, grid, st);
+            break;
         case PLASMA_TC_BF16X6: launch_pair<MODE_BF16X6>(s, map, cmap, g, grid, st); break;
         default: launch_pair<MODE_BF16>(s, map, cmap, g, grid, st); break;
         }
     } else {
         switch (mode) {
         case PLASMA_TC_TF32: launch_update<MODE_TF32>(s, map, cmap, g, grid, st); break;
-        case PLASMA_TC_FP16X3: launch_update<MODE_FP16X3>(s, map, cmap, g, grid, st); break;
+        case PLASMA_TC_FP16X3:
+            if (passes == 2) launch_update<MODE_FP16X3, 2>(s, map, cmap, g, grid, st);
+            else launch_update<MODE_FP16X3>(s, map, cmap, g, grid, st);
+            break;
         default: launch_update<MODE_BF16>(s, map, cmap, g, grid, st); break;
         }
     }
@@ -1103,6 +1128,7 @@ extern "C" void plasma_cuda_panel_round(cudaStream_t s, plasma_devstat_t *st,
         k_panel_round<MODE_BF16><<<grid, 256, 0, s>>>(A, k, panel, poff, pstride, scale, st);
         break;
     case PLASMA_TC_FP16X3:
+    case PLASMA_TC_FP16X3S:
         k_panel_round<MODE_FP16X3><<<grid, 256, 0, s>>>(A, k, panel, poff, pstride, scale, st);
         break;
     case PLASMA_TC_BF16X6:

@@ -309,6 +309,10 @@ void plasma_cuda_lacpy(cudaStream_t s, plasma_devstat_t *st,
                                 (FP32; 256-wide tiles)                     */
 #define PLASMA_TC_FP16X3 4   /* lo*hi + hi*lo + hi*hi of a half-precision
                                 split with row scales (FP32)               */
+#define PLASMA_TC_FP16X3S 5  /* the same, small products first over all of K:
+                                factors that the caller gets               */
+/* added to a PlasmaFactor* mode: the factor serves refinement only */
+#define PLASMA_FACTOR_REFINED 256
 int plasma_cuda_update_tc_ok(plasma_desc_t A, plasma_enum_t uplo);
 /* Operand copies of the panels: full = 0 holds one panel (the caller
  * alternates two buffers), full = 1 every panel of the factor, so that an
