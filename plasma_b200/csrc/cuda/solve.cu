@@ -133,13 +133,16 @@ k_diag_mma(plasma_desc_t B, int k, int n0, const T *W, int trans, const plasma_d
         for (int f = 0; f < NF; f++)
 #pragma unroll
             for (int e = 0; e < 4; e++) acc[m][f][e] = sum[m][f][e] = T(0);
-    // operator entry (i, q): W(i, q) or W(q, i), both lower triangles of W
+    // operator entry (i, q): W(i, q) or W(q, i), both lower triangles of W;
+    // in FP32 without the diagonal, which the end adds rounded (the tensor
+    // cores truncate what they add to a sum)
     auto op = [&](int i, int q) {
+        if (sizeof(T) == 4 && i == q) return T(0);
         return trans ? w[(size_t)i * NB + q] : w[(size_t)q * NB + i];
     };
-    // the nonzero part of W, 8 columns (rows of B) a step, the diagonal last:
-    // its terms are the largest in general, and a sum that begins with them
-    // rounds at their size from there on
+    // the nonzero part of W, 8 columns (rows of B) a step, towards the
+    // diagonal: its terms are the largest in general, and a sum that begins
+    // with them rounds at their size from there on
     const int steps = (trans ? NB - i0 : i0 + 16 * MI) / 8;
     const int qs = trans ? -8 : 8;
     T an[MI][4];
@@ -168,8 +171,7 @@ k_diag_mma(plasma_desc_t B, int k, int n0, const T *W, int trans, const plasma_d
         for (int m = 0; m < MI; m++)
 #pragma unroll
             for (int f = 0; f < NF; f++) mma8<3>(acc[m][f], a[m], bf[f]);
-        // FP32: the tensor cores truncate what they add to a sum; the terms
-        // leave them 8 at a time
+        // FP32: the terms leave the tensor cores 8 at a time
         if (sizeof(T) == 4 || i + 1 == steps) {
 #pragma unroll
             for (int m = 0; m < MI; m++)
@@ -189,7 +191,9 @@ k_diag_mma(plasma_desc_t B, int k, int n0, const T *W, int trans, const plasma_d
 #pragma unroll
             for (int e = 0; e < 4; e++) {
                 const int r = i0 + 16 * m + g + 8 * (e >> 1), c = 8 * f + 2 * t + (e & 1);
-                if (r < rows && c < cols) b[(size_t)c * ldb + r] = sum[m][f][e];
+                T x = sum[m][f][e];
+                if (sizeof(T) == 4) x = fma(w[(size_t)r * NB + r], Bs[r * LDS + c], x);
+                if (r < rows && c < cols) b[(size_t)c * ldb + r] = x;
             }
 }
 

@@ -126,8 +126,9 @@ def test_fp32_factor(L, n):
 # FP32 solves with many right-hand sides (tile inverses on the tensor cores,
 # k_diag_mma): A^-1 from identity columns.  Sums that leave the tensor cores
 # every 32 terms, the backward ones begun with the diagonal's, 12.3 and 16.8 u;
-# every 8 terms and towards the diagonal 7.8 and 13.0.
-@pytest.mark.parametrize("n,nb,limit", [(1536, 128, 9.0), (1100, 256, 14.5)])
+# every 8 terms and towards the diagonal, whose own terms are rounded, 6.9 and
+# 12.4.
+@pytest.mark.parametrize("n,nb,limit", [(1536, 128, 7.5), (1100, 256, 14.5)])
 def test_fp32_many_rhs(L, n, nb, limit):
     assert L.plasma_set(pb.PlasmaNb, nb) == 0
     a = gram(n, n).astype(np.float32)
