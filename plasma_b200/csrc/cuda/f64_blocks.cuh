@@ -85,11 +85,16 @@ __device__ __forceinline__ void strip_solve32(double (&y)[4][2], double (&s)[4][
     }
 }
 
-// 1/sqrt(d) for normal d away from the ends of the range: the hardware's
-// approximation (relative error below 2^-20) and one third-order step,
-// r + r e (1/2 + 3/8 e) with e = 1 - d r^2.  Branch-free, so the compiler can
-// run a column's updates between its dependent steps (rsqrt() has a slow
-// path for the ends of the range; blocks that need it take blk_factor_any).
+// 1/sqrt(d) for normal d away from the ends of the range, as mathematics gives
+// it: with r near 1/sqrt(d) and e = 1 - d r^2, 1/sqrt(d) = r (1 - e)^(-1/2),
+// by the binomial series r (1 + e/2 + 3/8 e^2 + ...).  From the hardware's
+// approximation, an instruction with its e below 2^-19, the terms written leave
+// 5/16 e^3 < 2^-58 (a step of Householder's method, of third order); the
+// roundings of d r and of the result remain, so the error is at most one unit
+// in the last place, CUDA's bound for rsqrt().  rsqrt() itself has a slow path
+// for the ends of the range (blocks that need it take blk_factor_any); this
+// has no branch, so the compiler can run a column's updates between its
+// dependent steps.
 __device__ __forceinline__ double blk_rsqrt(double d)
 {
     double r;
@@ -98,7 +103,8 @@ __device__ __forceinline__ double blk_rsqrt(double d)
     return fma(r * e, fma(0.375, e, 0.5), r);
 }
 
-// FP32: one Newton step
+// FP32: the hardware's e is below 2^-21 and the series stops at e/2 (Newton's
+// step), which leaves 3/8 e^2 < 2^-43; the same bound
 __device__ __forceinline__ float blk_rsqrt(float d)
 {
     float r;

@@ -203,3 +203,35 @@ def test_plan_rejects_large_orders(env):
     torch, Batch, L = env
     with pytest.raises(RuntimeError):
         Batch([10, 513])
+
+
+@pytest.mark.parametrize("dtype_name", ["f64", "f32"])
+def test_pivot_reciprocal_roots(env, dtype_name):
+    """The factor of [d 1; 1 x] is [sqrt(d); 1/sqrt(d) ...]: the block factor's
+    own reciprocal square root, over the range that it serves, is within one
+    unit in the last place of the exact one and within two of CUDA's rsqrt
+    (whose bound is one), its square root within one of the exact one."""
+    torch, Batch, _ = env
+    f64 = dtype_name == "f64"
+    lim, bits, npt = (279.0, 53, np.float64) if f64 else (29.0, 24, np.float32)
+    rng = np.random.default_rng(1)
+    d = np.concatenate([10.0 ** rng.uniform(-lim, lim, 4000), 1 + rng.uniform(0, 3, 4000),
+                        2.0 ** np.arange(-90, 91)]).astype(npt)
+    mats = [np.array([[v, 1.0], [1.0, 4.0 / v + 1.0]]) for v in d.astype(np.float64)]
+    b = Batch([2] * len(d), torch.float64 if f64 else torch.float32)
+    A, info = b.pack_matrices(mats), b.info_buffer()
+    b.potrf(A, info)
+    torch.cuda.synchronize()
+    assert not info.any()
+    f = A.cpu().numpy()
+    at = b.off_a[:len(d)]
+    root, recip = f[at], f[at + 1]
+    x = d.astype(np.longdouble)
+
+    def ulps(got, want):
+        _, e = np.frexp(want)
+        return np.abs((got - want) / np.ldexp(np.longdouble(1), e - bits)).max()
+    assert ulps(recip, 1 / np.sqrt(x)) <= 1
+    assert ulps(root, np.sqrt(x)) <= 1
+    cuda = torch.rsqrt(torch.from_numpy(d).cuda()).cpu().numpy().astype(np.longdouble)
+    assert ulps(recip, cuda) <= 2
