@@ -4,7 +4,7 @@
 //     C(m,n) -= A(m,k) A(n,k)^T,   k < n <= m,  C and A in FP64
 //
 // (compute/pzpotrf.c:57-77).  What bounds the DMMA form (update.cu) is the
-// FP64 pipe, 64 multiply-adds a clock and SM; kind::i8 does 16384.  The
+// FP64 pipe, 64 multiply-adds a clock and SM; kind::i8 does 8192.  The
 // product is split after Ozaki et al. (2012) in the integer form of Ootomo,
 // Ozaki and Yokota (2024): every row of the panel is scaled by a power of
 // two 2^e (its largest entry at most 127/128 of it) and written as a 55-bit
@@ -15,12 +15,20 @@
 // and x y is formed from the 28 digit products with p + q <= 6.  Sums of one
 // order t = p + q are exact in 32 bits (at most 7 x 256 x 2^14 < 2^31), the
 // seven sums are joined exactly in 64-bit integers, and C takes one rounding
-// of its own.  Error per entry, relative to |row i| |row j|: 1.0e-16 against
-// 3.3e-16 of an FP64 sum of 256 products (normal entries), 3.6e-17 against
-// 2.4e-16 (uniform); with entries spread over e^(3 N(0,1)) 1.6e-15 against
-// 1.7e-15.  It is scaled by the row, not by the entry, which is the bound
-// that Cholesky's backward error rests on (|L(i,k)| <= sqrt(A(i,i))).  A row
-// holding Inf or NaN makes its products NaN.
+// of its own.
+//
+// Accuracy: the digits are relative to the largest entry of a row in the
+// panel, which is what Cholesky's normwise backward error rests on (|L(i,k)| <=
+// sqrt(A(i,i))).  Largest residual |A - L L^T| of an order of 3329 in units of
+// 2^-53 sqrt(a_ii a_jj), here, with the DMMA update and with LAPACK: likelihood
+// 3.3, 2.3, 2.3; rows scaled by up to 2^200 3.3, 4.1, 3.2; a first panel that
+// holds most of every row 1.7, 7.8, 8.8; its entries falling over 16 decades
+// within the rows 8.7, 10.3, 13.3.  What it does not have is the bound of a sum
+// of rounded products entry by entry, n u |L| |L|^T: entries small against
+// their row's largest lose low bits, and in the last of these matrices the
+// least favourable entry is off by 1.6e14 u |L| |L|^T where the DMMA update is
+// off by 16.  Tiles that are not 128 or 256 wide (PlasmaNb) take that one.  A
+// row holding Inf or NaN makes its products NaN.
 //
 // k_panel_i8: digits of a panel, one CTA per 32 rows; global layout by units
 // of 128 rows: [unit][K / 32][digit][8-row group][16-byte half][8 rows][16
