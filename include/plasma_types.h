@@ -142,7 +142,7 @@ enum {
 
 /* Values of PlasmaMixedPrecisionMode (GPU-build extension). */
 enum {
-    PlasmaFactorFP32 = 0,   /* FP32 factor on CUDA cores                     */
+    PlasmaFactorFP32 = 0,   /* FP32 factor (split products on tensor cores)  */
     PlasmaFactorTF32 = 1,   /* TF32 tensor-core update, FP32 accumulation    */
     PlasmaFactorBF16 = 2,   /* BF16 tensor-core update, FP32 accumulation    */
     PlasmaFactorAuto = 3    /* BF16 first, escalate on failure or stagnation */

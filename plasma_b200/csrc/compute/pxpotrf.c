@@ -38,7 +38,7 @@ typedef struct {
     int sms;
     int mode;          /* PLASMA_TC_* product precision of the tensor-core
                           update, or 0 for the DMMA/SIMT update            */
-    int full;          /* panel copies: every panel (1) or two buffers (0) */
+    int full;          /* panel copies: every panel (1) or three buffers (0) */
     char *panel[3];    /* rounded copies of panel k (buffer k % 3, or all) */
     int i8_steps;      /* FP64: steps k < i8_steps update from the panel's
                           digits on the integer tensor cores               */
@@ -91,9 +91,14 @@ void plasma_pXpotrf_reserve(plasma_context_t *plasma, plasma_enum_t uplo, plasma
 /* FP64: steps whose trailing matrix has at least 3072 rows update on the
  * integer tensor cores (cuda/update_i8.cu); below, the digits' own launch on
  * the critical path and the longer fill of a block cost more than the DMMA
- * update's arithmetic.  Measured with 256-wide tiles, threshold in tile rows:
- * n = 8192 7.5 ms (4 to 16 rows), 8.6 (24), 10.9 (never); n = 16384 33.3 (4),
- * 31.3 (8), 31.2 (16), 32.3 (24), 64 (never). */
+ * update's arithmetic.  dpotrf, ms, thresholds of 1024, 2048, 3072, 4096 rows
+ * and never:
+ *   256-wide tiles  n = 4608  2.79  2.77  2.78  2.90  3.04
+ *                   n = 8192  5.85  5.84  5.84  5.97  9.29
+ *                   n = 16384 27.5  27.3  27.4  27.7  56.8
+ *   128-wide        n = 4608  2.58  2.43  2.51  2.64  2.80
+ *                   n = 8192  6.63  6.56  6.54  6.78  9.94
+ *                   n = 16384 37.7  37.7  37.7  37.8  63.3 */
 static int i8_steps(plasma_desc_t A, plasma_enum_t uplo)
 {
     const int rows = 3072 / imax(A.mb, 1);

@@ -170,7 +170,7 @@ extern "C" int plasma_cuda_trsm_f64(cudaStream_t s, plasma_devstat_t *st, plasma
 {
     const int nk = plasma_tile_mview(A, k);
     if (nk % 32 != 0 || nk == 0 || nk > TF_NBMAX) return 0;
-    if ((long long)(mhi - mlo) * ceil_div(A.mb, 32) <= 148)
+    if ((long long)(mhi - mlo) * ceil_div(A.mb, 32) <= plasma_context_self()->num_sms)
         launch_trsm_f64<4>(s, st, A, k, mlo, mhi, nk);
     else
         launch_trsm_f64<8>(s, st, A, k, mlo, mhi, nk);

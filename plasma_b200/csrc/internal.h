@@ -315,7 +315,7 @@ void plasma_cuda_lacpy(cudaStream_t s, plasma_devstat_t *st,
 #define PLASMA_FACTOR_REFINED 256
 int plasma_cuda_update_tc_ok(plasma_desc_t A, plasma_enum_t uplo);
 /* Operand copies of the panels: full = 0 holds one panel (the caller
- * alternates two buffers), full = 1 every panel of the factor, so that an
+ * alternates three buffers), full = 1 every panel of the factor, so that an
  * update may lag any number of steps behind the panel stream. */
 size_t plasma_cuda_panel_bytes(int tc_mode, plasma_desc_t A, int full);
 int plasma_cuda_update_tc(cudaStream_t s, plasma_devstat_t *st, int tc_mode,

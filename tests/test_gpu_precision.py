@@ -127,7 +127,7 @@ def test_fp32_factor(L, n):
 # k_diag_mma): A^-1 from identity columns.  Sums that leave the tensor cores
 # every 32 terms, the backward ones begun with the diagonal's, 12.3 and 16.8 u;
 # every 8 terms and towards the diagonal, whose own terms are rounded, 6.9 and
-# 12.4.
+# 12.1.
 @pytest.mark.parametrize("n,nb,limit", [(1536, 128, 7.5), (1100, 256, 14.5)])
 def test_fp32_many_rhs(L, n, nb, limit):
     assert L.plasma_set(pb.PlasmaNb, nb) == 0
