@@ -258,6 +258,18 @@ def reference_built():
     return os.path.exists(ref.LIB_PATH)
 
 
+def reference_missing():
+    """Why the reference PLASMA cannot be run here, in one line, or None."""
+    from oracle import ref
+    if not ref.available():
+        return "oracle/_ref is not built and the reference's sources are not here"
+    try:
+        ref.lib()
+    except (OSError, subprocess.CalledProcessError) as e:
+        return f"oracle/_ref does not build or load: {e}".splitlines()[0]
+    return None
+
+
 def reference_sample(routine, n, extra, nb, threads, dt, info, it=None):
     return {"value": dt * 1e3, "unit": "ms", "cores": threads, "kind": "reference",
             "sample": f"reference PLASMA plasma_{routine} (oracle/_ref, OpenBLAS 0.3.15 "
@@ -313,6 +325,10 @@ def run_reference(args):
     to host memory before the timed steps."""
     rank, world, _ = dist_info()
     if rank != 0:
+        return 0
+    missing = reference_missing()
+    if missing:
+        print(json.dumps({"impl": "reference", "unavailable": missing}), flush=True)
         return 0
     import torch
     n, nrhs, nb = args.n, args.nrhs, (args.nb or 256)
@@ -1088,12 +1104,14 @@ def main():
                            "ms_per_step": min(pts), "host_memory": "pageable"}
         del ap, bp, xp
 
-    cpu = None
+    cpu = cpu_missing = None
     if not args.no_cpu and rank == 0:
-        a_h, b_h = host_system(A, B)
-        cpu = cpu_baseline(a_h, b_h, args.nb or 256)
-        cpu.pop("seconds", None)
-        del a_h, b_h
+        cpu_missing = reference_missing()
+        if cpu_missing is None:
+            a_h, b_h = host_system(A, B)
+            cpu = cpu_baseline(a_h, b_h, args.nb or 256)
+            cpu.pop("seconds", None)
+            del a_h, b_h
 
     if rank != 0:
         L.plasma_finalize()
@@ -1151,6 +1169,7 @@ def main():
         "peaks_tflops": peaks,
         "e2e": e2e,
         "cpu_baseline": cpu,
+        **({"cpu_baseline_unavailable": cpu_missing} if cpu_missing else {}),
         "clocks": clk,
         "gpu_launches": int(launches),
     }

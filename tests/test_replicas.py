@@ -77,3 +77,19 @@ def test_reference_arm_prints_the_benchmark_metric():
     assert line["cpu_baseline"]["kind"] == "reference"
     assert line["info"] == 0 and line["iter"] >= 0
     assert line["value"] > 0
+
+
+def test_reference_arm_says_why_it_cannot_run():
+    """Without the reference's library and sources the reference arm prints an
+    "unavailable" line and exits 0, and the GPU arm's baseline is absent with
+    the same reason instead of an exception that loses its figures."""
+    code = ("import sys, oracle.ref as r; r.LIB_PATH = r.REFERENCE_DIR = '/nonexistent'; "
+            "import bench; assert bench.reference_missing(); "
+            "sys.argv = ['bench.py', '--impl', 'reference', '--steps', '1']; "
+            "sys.exit(bench.main())")
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr
+    line = json.loads(r.stdout.strip().splitlines()[-1])
+    assert line["impl"] == "reference" and "not here" in line["unavailable"]
+    assert set(line) == {"impl", "unavailable"}
