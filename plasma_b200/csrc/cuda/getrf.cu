@@ -684,12 +684,13 @@ k_colmax(plasma_desc_t D, double *out, const plasma_devstat_t *st)
 // them with the unit-lower sub-block diagonal (U12 = L11^-1 A12, written to
 // the panel by the CTAs in turn) and updates its rows (A22 -= L21 U12).
 // A zero pivot records info (the first one, as k_lu_pivot) and the
-// factorization goes on without scaling that column.  A 64-column FP32
-// panel of 4096 rows took 168 us with the candidates read across the cluster
-// between barriers and the rows interchanged in shared memory; it takes 96 us
-// (four rows a thread), 79 (two) and 74 (one): about 1.1 us a column is the
-// exchange and the chain around it.  One record per CTA behind a CTA barrier
-// instead of one per warp: 119 us.
+// factorization goes on without scaling that column.  Mean times of the
+// 64-column FP32 panels of n = 4096: 96 us with 2049 to 4096 rows (four a
+// thread), 79 with 1025 to 2048 (two), 74 with up to 1024 (one): about 1.1 us a
+// column is the exchange and the chain around it.  All panels together were
+// 168 us in the mean with the candidates read across the cluster between
+// barriers and the rows interchanged in shared memory; one record per CTA behind
+// a CTA barrier, instead of one per warp, takes 119 us with four rows a thread.
 // ---------------------------------------------------------------------------
 constexpr int CL_CTAS = 8;
 constexpr int CL_THREADS = 128;
