@@ -22,7 +22,7 @@
 //     queue behind it (5700 clocks a block alone, 9200 with one DMMA warp on
 //     the same scheduler).
 // Measured beside the one-CTA left-looking kernel before it (16-column
-// sub-panels, shuffles): order 128 61 -> 25 us, order 256 217 -> 75 us.
+// sub-panels, shuffles): order 128 61 -> 27 us, order 256 217 -> 78 us.
 // Pivot test and info as LAPACK dpotrf: the first pivot that is not > 0, NaN
 // included.
 #include "common.cuh"
